@@ -133,27 +133,33 @@ struct WorkItem {
 // Device-side control block of one enumeration launch.
 //
 // The donation queue is a ring of `qcap` (a power of two, at least 32) slots addressed by
-// monotone 32-bit positions: position p lives in slot p & (qcap - 1).  Each slot carries a
-// 64-bit sequence word (epoch << 32 | position): the producer of position p may write the slot
-// once its word reads (epoch, p) — or, in the first lap, any older epoch — and publishes with
-// (epoch, p + 1); the consumer that takes p releases the slot with (epoch, p + qcap).  Slots are
-// reused for the whole launch, no position is ever skipped, and nobody waits on a slot.
-struct EnumControl {
+// monotone 32-bit positions: position p lives in slot p & (qcap - 1).  Producers and consumers
+// each take positions in order: a warp out of work takes the next one as its own (q_tail) and
+// waits for that position's item, so q_tail - q_head (as a signed number) is the number of
+// waiting warps.  Each slot carries a 64-bit sequence word (epoch << 32 | position): the producer
+// of position p may write the slot once its word reads (epoch, p) — or, in the first lap, any
+// older epoch — and publishes with (epoch, p + 1); the consumer of p releases the slot with
+// (epoch, p + qcap).  (epoch, CSM_QUEUE_OVER) tells the waiting warps that nothing is left.
+// Slots are reused for the whole launch and no position is ever skipped.
+//
+// The counters that many warps touch at once lie in 128-byte lines of their own, so that traffic
+// on one does not queue behind the others.
+struct alignas(128) EnumControl {
     unsigned long long ticket;        // next seed / frontier ticket
     unsigned long long nticket;       // total tickets
-    unsigned int q_head;              // donation positions reserved
-    unsigned int q_tail;              // donation positions claimed
-    unsigned int hungry;              // outstanding work requests of idle warps
-    unsigned int active;              // warps holding work
     unsigned int error;               // CSM_ERRBIT_* of this launch
     unsigned int epoch;               // launch epoch, stamps the queue's sequence words
+    unsigned long long t_start;       // device clock (ns) when the launch's control block was reset
+    alignas(128) unsigned int q_head; // donation positions reserved (8-byte aligned pair with q_tail)
+    unsigned int q_tail;              // donation positions taken by warps out of work
+    alignas(128) unsigned int active; // warps holding work, and items in the ring
+    alignas(128)
     unsigned long long out_rows;      // rows written (materialize / expand)
     unsigned long long scan_entries;  // statistics
     unsigned long long probes;
     unsigned long long tail_lists;
     unsigned long long donations;
     unsigned long long expand_bound;  // upper bound of the next BFS level
-    unsigned long long t_start;       // device clock (ns) when the launch's control block was reset
     unsigned long long queue_full;    // donations refused because the ring was full
     unsigned long long shared_last;   // last levels counted once for a prefix (DevPlan.shared_last)
     // First failed consistency check of the launch (CSM_ERRBIT_CORRUPT): where (CSM_BAD_*) and
@@ -170,8 +176,10 @@ struct EnumControl {
 // Positions past this are never reserved (a launch would need 2^31 donations to reach it).
 #define CSM_QUEUE_POS_LIMIT 0x7FFFFFFFu
 #define CSM_QUEUE_MIN_SLOTS 32u
+#define CSM_QUEUE_OVER 0xFFFFFFFFu
 
 #define CSM_ERRBIT_TIMEOUT 1u  // the launch ran past its time limit and stopped early
 #define CSM_ERRBIT_OUTPUT 2u
 #define CSM_ERRBIT_POOL 8u
+#define CSM_ERRBIT_IDLE 4u     // a warp out of work waited past its bound (with CSM_ERRBIT_TIMEOUT)
 #define CSM_ERRBIT_CORRUPT 16u  // a consistency check failed (see EnumControl.bad_*)

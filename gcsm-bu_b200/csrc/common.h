@@ -147,9 +147,16 @@ struct WorkItem {
 struct alignas(128) EnumControl {
     unsigned long long ticket;        // next seed / frontier ticket
     unsigned long long nticket;       // total tickets
-    unsigned int error;               // CSM_ERRBIT_* of this launch
-    unsigned int epoch;               // launch epoch, stamps the queue's sequence words
-    unsigned long long t_start;       // device clock (ns) when the launch's control block was reset
+    unsigned int error;               // CSM_ERRBIT_* of this phase
+    unsigned int epoch;               // phase epoch, stamps the queue's sequence words
+    unsigned long long t_start;       // device clock (ns) when the next launch's state was set up
+    // Semi-BFS: what the next launch of the phase reads, decided on the device between launches.
+    unsigned int src;                 // 0 = seed tickets, 1 + b = frontier buffer b
+    unsigned int go;                  // the next expansion launch runs (0: it returns at once)
+    unsigned int halt;                // an expansion failed: the counting launch returns at once
+    unsigned int levels;              // expansion launches that ran
+    unsigned int blocks_done;         // blocks of the deciding launch that have finished
+    unsigned long long max_front;     // largest frontier of the phase
     alignas(128) unsigned int q_head; // donation positions reserved (8-byte aligned pair with q_tail)
     unsigned int q_tail;              // donation positions taken by warps out of work
     alignas(128) unsigned int active; // warps holding work, and items in the ring
@@ -182,4 +189,5 @@ struct alignas(128) EnumControl {
 #define CSM_ERRBIT_OUTPUT 2u
 #define CSM_ERRBIT_POOL 8u
 #define CSM_ERRBIT_IDLE 4u     // a warp out of work waited past its bound (with CSM_ERRBIT_TIMEOUT)
+#define CSM_ERRBIT_FRONTIER 32u  // a semi-BFS level outgrew its frontier buffer
 #define CSM_ERRBIT_CORRUPT 16u  // a consistency check failed (see EnumControl.bad_*)

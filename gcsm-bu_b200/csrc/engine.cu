@@ -162,7 +162,6 @@ csm_status Engine::init() {
     }
     CSM_CUDA(dev_alloc(&d_ctrl_, 1));
     CSM_CUDA(cudaMemset(d_ctrl_, 0, sizeof(EnumControl)));
-    CSM_CUDA(dev_alloc(&d_misc_, 8));
     CSM_CUDA(cudaMallocHost(&h_counts_, sizeof(unsigned long long) * 64));
     CSM_CUDA(cudaMallocHost(&h_ctrl_, sizeof(EnumControl) * 2));
     return CSM_OK;
@@ -175,7 +174,7 @@ Engine::~Engine() {
                    g_.vlab, d_plans_, d_terms_, d_upd_src_, d_upd_dst_, d_upd_lab_, d_upd_del_, d_keys_raw_, d_keys_,
                    d_sort_temp_, bs_.eff, bs_.heads, bs_.nheads, bs_.seg_nins, bs_.seg_ndel, bs_.seg_end, bs_.scr_y,
                    bs_.scr_lb, bs_.counters, bs_.error, d_ctrl_, d_queue_, d_seq_, d_seed_lo_, d_ticket_prefix_,
-                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_misc_, d_rel_delta_, d_touched_, d_memo_};
+                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (h_pin_) cudaFreeHost(h_pin_);
@@ -587,6 +586,9 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
     last_loop_ = false;
     for (const auto &hp : plans_)
         if (hp.dev.tail_start == hp.dev.n && hp.dev.n >= 3) last_loop_ = true;
+    // Breadth-first launches a phase can need: from the seeds to the deepest expandable level.
+    expand_levels_ = 0;
+    for (const auto &hp : plans_) expand_levels_ = std::max(expand_levels_, (int)hp.dev.expand_stop - 1);
     return CSM_OK;
 }
 
@@ -926,7 +928,9 @@ csm_status Engine::enqueue_batch(uint64_t n, const uint32_t *src, const uint32_t
         CSM_CUDA(store_sort_keys(d_sort_temp_, tb, d_keys_raw_, d_keys_, m, kl_, s));
         store_classify(m, d_keys_, kl_, g_, bs_, s);
         store_touched(m, d_keys_, kl_, d_touched_, words_, s);
-        stats_.kernel_launches += 4;
+        // Both phases start from the same seeds: the batch's keys by relation.
+        launch_seed_tickets(d_plans_, np, d_keys_, m, kl_, sc_.seed_lo, sc_.ticket_prefix, s);
+        stats_.kernel_launches += 6;
         if (d_rel_delta_) {
             CSM_CUDA(cudaMemsetAsync(d_rel_delta_, 0, sizeof(long long) * g_.R, s));
             store_rel_delta(m, d_keys_, kl_, bs_, d_rel_delta_, s);
@@ -1119,6 +1123,8 @@ csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *ds
         stats_.donations += c.donations;
         stats_.donations_refused += c.queue_full;
         stats_.enum_shared_last += c.shared_last;
+        stats_.enum_launches += c.levels;
+        last_frontier_rows_ = std::max(last_frontier_rows_, c.max_front);
         if (c.error & CSM_ERRBIT_CORRUPT) {
             poisoned_ = true;
             return fail(CSM_ERR_STATE, describe_bad(c));
@@ -1131,6 +1137,8 @@ csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *ds
                                                     "batch's counts are incomplete; the graph holds the whole batch"
                                                   : "the enumeration ran past its time limit (time_limit_us): this batch's "
                                                     "counts are incomplete; the graph holds the whole batch");
+        if ((c.error & CSM_ERRBIT_FRONTIER) && deferred_ == CSM_OK)
+            deferred_ = fail(CSM_ERR_OVERFLOW, "semi-BFS frontier overflow");
         if ((c.error & CSM_ERRBIT_OUTPUT) && deferred_ == CSM_OK)
             deferred_ = fail(CSM_ERR_OVERFLOW, "embedding row buffer too small");
     }
@@ -1205,73 +1213,26 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
     phase_ran_[ph] = true;
     CSM_CUDA(record_event(ev_[2 + 2 * ph], s));
 
-    launch_ctrl_reset(sc_.ctrl, 0, 0, s);
-    launch_seed_tickets(d_plans_, np, d_keys_, m, kl_, sc_.seed_lo, sc_.ticket_prefix, sc_.ctrl, s);
-    stats_.kernel_launches += 3;
-    const WorkItem *frontier = nullptr;
-    unsigned long long nfront = 0;
-    if (strategy >= 2 && !rows) {
-        // Semi-BFS (Matching / BfsMatching, match_gpu.cu:1916-2294): expand levels while the
-        // frontier is small (strategy 2) or while it fits the budget (strategy 3); the size of
-        // the next level is bounded from list sizes before it is written, so a level that would
-        // not fit is never started and the search continues depth first from the current one.
-        CSM_CUDA(cudaMemcpyAsync(h_counts_ + 2 * np + 4, &sc_.ctrl->nticket, sizeof(unsigned long long),
-                                 cudaMemcpyDeviceToHost, s));
-        CSM_CUDA(cudaStreamSynchronize(s));
-        unsigned long long cur = h_counts_[2 * np + 4] * 32;  // seed candidates (upper bound)
-        const unsigned long long target = (unsigned long long)lc_.frontier_mult * total_warps;
-        int buf = 0;
-        for (int level = 0; level < CSM_MAXQV; level++) {
-            if (strategy == 2 && cur >= target) break;
-            if (cur == 0) break;
-            unsigned long long bound = cur;
-            if (frontier) {
-                h_counts_[2 * np + 4] = nfront;
-                CSM_CUDA(cudaMemcpyAsync(d_misc_, h_counts_ + 2 * np + 4, 8, cudaMemcpyHostToDevice, s));
-                CSM_CUDA(cudaMemsetAsync(&sc_.ctrl->expand_bound, 0, 8, s));
-                launch_expand_bound(P, frontier, d_misc_, s);
-                CSM_CUDA(cudaMemcpyAsync(h_counts_ + 2 * np + 5, &sc_.ctrl->expand_bound, 8, cudaMemcpyDeviceToHost, s));
-                CSM_CUDA(cudaStreamSynchronize(s));
-                bound = h_counts_[2 * np + 5];
-            }
-            if (bound > frontier_cap_) break;
-            EnumParams X = P;
-            X.mode = CSM_ENUM_MODE_EXPAND;
-            X.donate = 0;
-            X.frontier = frontier;
-            X.expand_out = d_frontier_[buf];
-            X.expand_cap = frontier_cap_;
-            if (frontier) launch_ctrl_reset(sc_.ctrl, 0, nfront, s);
+    // Semi-BFS (Matching / BfsMatching, match_gpu.cu:1916-2294): expand levels while the frontier is
+    // small (strategy 2) or while it fits the budget (strategy 3).  The size of the next level is
+    // bounded from list sizes before it is written, so a level that would not fit is never started
+    // and the search continues depth first from the current one.  All launches of the phase are
+    // issued at once; the decisions are taken on the device.
+    const bool expand = strategy >= 2 && !rows && frontier_cap_ > 0;
+    const unsigned long long target =
+        strategy == 2 ? (unsigned long long)lc_.frontier_mult * total_warps : ~0ull;
+    launch_phase_begin(sc_.ctrl, sc_.ticket_prefix, np, expand, target, frontier_cap_, s);
+    stats_.kernel_launches++;
+    for (int b = 0; b < 2; b++) P.frontier[b] = expand ? d_frontier_[b] : nullptr;
+    P.frontier_cap = expand ? frontier_cap_ : 0;
+    if (expand) {
+        EnumParams X = P;
+        X.mode = CSM_ENUM_MODE_EXPAND;
+        X.donate = 0;
+        for (int level = 1; level <= expand_levels_; level++) {
             launch_enumerate(X, blocks_, warps_per_block_, occupancy_, s);
-            stats_.enum_launches++;
-            stats_.kernel_launches++;
-            CSM_CUDA(cudaMemcpyAsync(&h_ctrl_[ph], sc_.ctrl, sizeof(EnumControl), cudaMemcpyDeviceToHost, s));
-            CSM_CUDA(cudaStreamSynchronize(s));
-            const unsigned long long rows_out = h_ctrl_[ph].out_rows;
-            const unsigned int errb = h_ctrl_[ph].error;
-            if (errb & (CSM_ERRBIT_OUTPUT | CSM_ERRBIT_TIMEOUT | CSM_ERRBIT_CORRUPT)) {
-                // Out of time (or, never expected, of frontier room): the phase stops here and
-                // the batch reports it; the update kernels after it still run.
-                if ((errb & CSM_ERRBIT_OUTPUT) && deferred_ == CSM_OK)
-                    deferred_ = fail(CSM_ERR_OVERFLOW, "semi-BFS frontier overflow");
-                CSM_CUDA(record_event(ev_[3 + 2 * ph], s));
-                return CSM_OK;
-            }
-            // This expansion launch's work counters, before the next launch's control block
-            // replaces them (the batch's final launch is added when the batch completes).
-            stats_.enum_scan_entries += h_ctrl_[ph].scan_entries;
-            stats_.enum_probes += h_ctrl_[ph].probes;
-            stats_.enum_tail_lists += h_ctrl_[ph].tail_lists;
-            stats_.donations += h_ctrl_[ph].donations;
-            stats_.donations_refused += h_ctrl_[ph].queue_full;
-            stats_.enum_shared_last += h_ctrl_[ph].shared_last;
-            const bool grew = rows_out != nfront || frontier == nullptr;
-            frontier = d_frontier_[buf];
-            nfront = rows_out;
-            last_frontier_rows_ = std::max(last_frontier_rows_, nfront);
-            buf ^= 1;
-            cur = nfront;
-            if (!grew) break;
+            launch_expand_decide(X, level == expand_levels_, target, s);
+            stats_.kernel_launches += 2;
         }
     }
     EnumParams D = P;
@@ -1279,11 +1240,6 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
     // Work donation in the depth-first launch for every strategy but 1 ("DFS w/o work
     // stealing"); after a BFS phase (strategy 3) it evens out the frontier items' subtrees.
     D.donate = strategy == 1 ? 0u : 1u;
-    if (frontier) {
-        D.frontier = frontier;
-        launch_ctrl_reset(sc_.ctrl, 0, nfront, s);
-        stats_.kernel_launches++;
-    }
     if (!rows && !memo_plan_.empty()) {
         // Tables of the pendant plans for this phase's graph and flags.
         for (size_t t = 0; t < memo_plan_.size(); t++)

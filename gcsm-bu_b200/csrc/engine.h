@@ -274,7 +274,6 @@ class Engine {
     unsigned long long row_cap_ = 0;
     unsigned long long *h_counts_ = nullptr;  // pinned readback
     EnumControl *h_ctrl_ = nullptr;           // pinned: control block of the DEL and INS launches
-    unsigned long long *d_misc_ = nullptr;    // small device scratch
     bool phase_ran_[2] = {false, false};
     EnumScratch sc_;                          // scratch used by enumerate_phase
     bool no_alloc_ = false;                   // inside apply_device_noalloc
@@ -282,6 +281,7 @@ class Engine {
     int warps_per_block_ = 8;
     int occupancy_ = 4;                       // enumeration kernel variant (blocks per SM)
     int blocks_ = 0;
+    int expand_levels_ = 0;                   // most breadth-first levels any plan expands
     LaunchConfig lc_{};                       // configuration in use
     std::vector<LaunchConfig> tune_cands_;    // autotuner candidates
     std::vector<double> tune_ms_;             // accumulated enumeration time per candidate

@@ -628,15 +628,15 @@ __device__ int await_item(WarpState &S, const EnumParams &P, unsigned int &err, 
 
 // Takes the next seed chunk or frontier item into S: 1 = taken, 0 = none left, -1 = a frontier
 // item that failed its check (skipped).
-__device__ int take_ticket(WarpState &S, const EnumParams &P) {
+__device__ int take_ticket(WarpState &S, const EnumParams &P, const WorkItem *frontier) {
     const uint32_t lane = lane_id();
     unsigned long long t = 0;
     if (lane == 0) t = atomicAdd(&P.ctrl->ticket, 1ull);
     t = __shfl_sync(0xffffffffu, t, 0);
     const unsigned long long nt = *(volatile unsigned long long *)&P.ctrl->nticket;
     if (t >= nt) return 0;
-    if (P.frontier != nullptr) {
-        const WorkItem *it = P.frontier + t;
+    if (frontier != nullptr) {
+        const WorkItem *it = frontier + t;
         if (lane == 0) {
             S.item_plan = it->plan;
             S.item_depth = it->depth;
@@ -982,7 +982,7 @@ __device__ unsigned long long settle_pendant(WarpState &S, const EnumParams &P, 
 template <bool LASTLOOP, int MODE>
 __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32_t &scans,
                                        uint32_t &probes, uint32_t &tails, uint32_t &shared, unsigned int &err,
-                                       unsigned long long deadline) {
+                                       unsigned long long deadline, WorkItem *expand_out) {
     const uint32_t lane = lane_id();
     const DevPlan *pl = P.plans + S.item_plan;
     const uint32_t n = pl->n;
@@ -995,8 +995,8 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
         unsigned long long r = 0;
         if (lane == 0) r = atomicAdd(&P.ctrl->out_rows, 1ull);
         r = __shfl_sync(0xffffffffu, r, 0);
-        if (r < P.expand_cap) {
-            WorkItem *o = P.expand_out + r;
+        if (r < P.frontier_cap) {
+            WorkItem *o = expand_out + r;
             if (lane == 0) {
                 o->plan = S.item_plan;
                 o->depth = S.item_depth;
@@ -1005,7 +1005,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             }
             if (lane < CSM_MAXQV) o->f[lane] = S.f[lane];
         } else if (lane == 0) {
-            err |= CSM_ERRBIT_OUTPUT;
+            err |= CSM_ERRBIT_FRONTIER;
         }
         __syncwarp();
         return 0;
@@ -1211,10 +1211,10 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             unsigned long long r = 0;
             if (lane == 0 && c) r = atomicAdd(&P.ctrl->out_rows, (unsigned long long)c);
             r = __shfl_sync(0xffffffffu, r, 0);
-            if (c && r + c > P.expand_cap) {
-                if (lane == 0) err |= CSM_ERRBIT_OUTPUT;
+            if (c && r + c > P.frontier_cap) {
+                if (lane == 0) err |= CSM_ERRBIT_FRONTIER;
             } else if (ok) {
-                WorkItem *o = P.expand_out + r + rank;
+                WorkItem *o = expand_out + r + rank;
                 o->plan = S.item_plan;
                 o->depth = d + 1;
                 o->lo = 0;
@@ -1325,6 +1325,10 @@ __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
     WarpState &S = reinterpret_cast<WarpState *>(smem)[threadIdx.x >> 5];
     const uint32_t lane = lane_id();
     if (P.abort_flag != nullptr && *(volatile const unsigned int *)P.abort_flag) return;
+    if (MODE == CSM_ENUM_MODE_EXPAND ? !P.ctrl->go : P.ctrl->halt) return;
+    const uint32_t src = P.ctrl->src;
+    const WorkItem *frontier = src == 0 ? nullptr : P.frontier[src - 1];
+    WorkItem *expand_out = MODE == CSM_ENUM_MODE_EXPAND ? P.frontier[src == 1 ? 1 : 0] : nullptr;
     // Per-lane work counters (statistics only), 32-bit to keep registers for the search; a
     // lane flushes them to the launch totals before they could wrap.
     uint32_t scans = 0, probes = 0, tails = 0, shared = 0;
@@ -1349,7 +1353,7 @@ __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
         }
         int got = 0;
         if (have_source) {
-            got = take_ticket(S, P);
+            got = take_ticket(S, P, frontier);
             if (got < 0) continue;  // a frontier item that failed its check
             if (!got) have_source = false;
         }
@@ -1359,7 +1363,7 @@ __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
             if (got < 0) continue;
             if (!got) break;
         }
-        const unsigned long long c = run_item<LASTLOOP, MODE>(S, P, scans, probes, tails, shared, err, deadline);
+        const unsigned long long c = run_item<LASTLOOP, MODE>(S, P, scans, probes, tails, shared, err, deadline, expand_out);
         if (lane == 0 && c) atomicAdd(P.counts + S.item_plan, c);
         if ((scans | probes | tails | shared) >= (1u << 30)) {
             atomicAdd(&P.ctrl->scan_entries, (unsigned long long)scans);
@@ -1385,75 +1389,88 @@ __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
     }
 }
 
-// Per plan: the key range of its seed relation, and the number of 32-key seed chunks.
+// Per plan: the key range of its seed relation, and the number of 32-key seed chunks.  One warp per
+// plan and a 32-ary search: about log32(m) dependent reads for each end.
 __global__ void k_seed_ranges(const DevPlan *plans, uint32_t nplans, const unsigned long long *keys, uint32_t m,
                               KeyLayout kl, uint32_t *seed_lo, uint32_t *chunks) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = lane_id();
+    const uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (p >= nplans) return;
     const uint32_t rel = plans[p].seed_rel;
-    // [lo, hi) = keys whose relation field equals rel.
-    uint32_t lo = 0, hi = m;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (kl.rel(keys[mid]) < rel) lo = mid + 1;
-        else hi = mid;
+    uint32_t end[2];
+#pragma unroll
+    for (uint32_t e = 0; e < 2; e++) {
+        // First key whose relation is at least rel + e.
+        uint32_t lo = e ? end[0] : 0u, hi = m;
+        while (hi > lo) {
+            const uint32_t step = (hi - lo + 31u) / 32u;
+            const uint32_t i = lo + (lane + 1) * step - 1;
+            const bool below = i < hi && kl.rel(__ldg(keys + i)) < rel + e;
+            const uint32_t c = __popc(__ballot_sync(0xffffffffu, below));
+            const uint32_t nhi = lo + (c + 1) * step - 1;
+            lo += c * step;
+            hi = nhi < hi ? nhi : hi;
+            if (lo > hi) lo = hi;
+        }
+        end[e] = lo;
     }
-    uint32_t a = lo;
-    lo = a;
-    hi = m;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (kl.rel(keys[mid]) <= rel) lo = mid + 1;
-        else hi = mid;
+    if (lane == 0) {
+        seed_lo[p] = end[0];
+        seed_lo[nplans + p] = end[1];
+        chunks[p] = (end[1] - end[0] + 31u) / 32u;
     }
-    seed_lo[p] = a;
-    seed_lo[nplans + p] = lo;
-    chunks[p] = (lo - a + 31u) / 32u;
 }
 
 // Exclusive prefix of chunk counts (one block; plans are few).
-__global__ void k_ticket_prefix(const uint32_t *chunks, uint32_t nplans, uint32_t *prefix, EnumControl *ctrl) {
-    __shared__ uint32_t part[1024];
-    const uint32_t t = threadIdx.x;
+__global__ void __launch_bounds__(1024) k_ticket_prefix(const uint32_t *chunks, uint32_t nplans, uint32_t *prefix) {
+    __shared__ uint32_t part[32];
+    const uint32_t t = threadIdx.x, lane = lane_id();
     const uint32_t per = (nplans + blockDim.x - 1) / blockDim.x;
     uint32_t s = 0;
     for (uint32_t i = t * per; i < (t + 1) * per && i < nplans; i++) s += chunks[i];
-    part[t] = s;
+    uint32_t incl = s;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+    }
+    if (lane == 31) part[t >> 5] = incl;
     __syncthreads();
-    if (t == 0) {
-        uint32_t acc = 0;
-        for (uint32_t i = 0; i < blockDim.x; i++) {
-            uint32_t v = part[i];
-            part[i] = acc;
-            acc += v;
+    if (t < 32) {
+        uint32_t w = part[t];
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= (uint32_t)o) w += v;
         }
-        ctrl->nticket = acc;
-        prefix[nplans] = acc;
+        part[t] = w;
     }
     __syncthreads();
-    uint32_t acc = part[t];
+    uint32_t acc = incl - s + (t >= 32 ? part[(t >> 5) - 1] : 0u);
     for (uint32_t i = t * per; i < (t + 1) * per && i < nplans; i++) {
         prefix[i] = acc;
         acc += chunks[i];
     }
+    if (t == blockDim.x - 1) prefix[nplans] = acc;
 }
 
-// Resets the control block for one launch.  The launch epoch (which marks queue slots ready)
-// is the previous one plus one, kept on the device so that every launch on this scratch gets a
-// fresh epoch whichever engine, stream or replayed graph issues it.
-__global__ void k_ctrl_reset(EnumControl *ctrl, uint32_t active, unsigned long long nticket) {
+// Resets the control block for one phase.  The phase epoch (which marks queue slots ready) is the
+// previous one plus one, kept on the device so that every phase on this scratch gets a fresh epoch
+// whichever engine, stream or replayed graph issues it.
+__global__ void k_phase_begin(EnumControl *ctrl, const uint32_t *nticket, uint32_t expand, unsigned long long target,
+                              unsigned long long frontier_cap) {
+    uint32_t *w = reinterpret_cast<uint32_t *>(ctrl);
     uint32_t epoch = ctrl->epoch + 1u;
     if (epoch == 0) epoch = 1;
-    EnumControl c;
-    memset(&c, 0, sizeof(c));
-    c.active = active;
-    c.epoch = epoch;
-    c.nticket = nticket;
-    c.t_start = device_ns();
-    *ctrl = c;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < sizeof(EnumControl) / 4; i += blockDim.x) w[i] = 0u;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const unsigned long long seeds = 32ull * *nticket;  // upper bound
+    ctrl->epoch = epoch;
+    ctrl->nticket = *nticket;
+    ctrl->go = expand && seeds > 0 && seeds < target && seeds <= frontier_cap;
+    ctrl->t_start = device_ns();
 }
 
-// Upper bound of the next BFS level: sum over items of their smallest candidate list.
 // Table of a pendant plan (DevPlan.memo_slot): for every data vertex v, the count of its
 // counting level c for a prefix whose vertex at memo_depth is v — the candidates w of v's list
 // under the flag rule and c's NLF filter, each with its Cartesian tail, exactly as the
@@ -1505,28 +1522,57 @@ __global__ void k_pendant_counts(EnumParams P, uint32_t plan, unsigned long long
     }
 }
 
-__global__ void k_expand_bound(EnumParams P, const WorkItem *items, const unsigned long long *nitems) {
+// Between two expansion launches.  The level just written becomes the source of the next launch,
+// and the last block to finish decides whether that launch expands it further: only when an upper
+// bound of what it would write (the sum of every item's smallest candidate list) fits the frontier,
+// so no level overflows.  Deciding here instead of on the host takes two host synchronisations out
+// of every level; launches after the last level find go == 0 and return.
+__global__ void k_expand_decide(EnumParams P, uint32_t last, unsigned long long target) {
+    EnumControl *ctrl = P.ctrl;
+    if (!ctrl->go) return;  // no expansion ran: the state is already the counting launch's
     const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    const unsigned long long n = *nitems;
-    unsigned long long acc = 0;
-    for (unsigned long long i = (blockIdx.x * (blockDim.x >> 5)) + (threadIdx.x >> 5); i < n; i += nw) {
-        const WorkItem *it = items + i;
-        const DevPlan *pl = P.plans + it->plan;
-        const uint32_t d = it->depth;
-        if (d >= pl->expand_stop) {
-            if (lane == 0) acc += 1;  // passes through unchanged
-            continue;
+    const uint32_t out = ctrl->src == 1 ? 1u : 0u;  // the buffer the expansion wrote
+    const unsigned long long n = ctrl->out_rows;
+    const bool failed = (ctrl->error & (CSM_ERRBIT_FRONTIER | CSM_ERRBIT_TIMEOUT | CSM_ERRBIT_CORRUPT)) != 0;
+    const bool stop = failed || last || n == 0 || n >= target;
+    if (!stop) {
+        const unsigned long long nw = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+        unsigned long long acc = 0;
+        for (unsigned long long i = (blockIdx.x * (blockDim.x >> 5)) + (threadIdx.x >> 5); i < n; i += nw) {
+            const WorkItem *it = P.frontier[out] + i;
+            const DevPlan *pl = P.plans + it->plan;
+            const uint32_t d = it->depth;
+            if (d >= pl->expand_stop) {
+                if (lane == 0) acc += 1;  // passes through unchanged
+                continue;
+            }
+            const DevLevel *lv = &pl->lv[d];
+            uint32_t sz = 0xFFFFFFFFu;
+            if (lane < lv->nbn) sz = list_of(P, lv->bn_rel[lane], it->f[lv->bn_depth[lane]], 800 + d).y;
+            for (int o = 16; o > 0; o >>= 1) sz = min(sz, __shfl_xor_sync(0xffffffffu, sz, o));
+            if (lane == 0) acc += sz;
         }
-        const DevLevel *lv = &pl->lv[d];
-        uint32_t sz = 0xFFFFFFFFu;
-        if (lane < lv->nbn) {
-            sz = list_of(P, lv->bn_rel[lane], it->f[lv->bn_depth[lane]], 800 + d).y;
-        }
-        for (int o = 16; o > 0; o >>= 1) sz = min(sz, __shfl_xor_sync(0xffffffffu, sz, o));
-        if (lane == 0) acc += sz;
+        if (lane == 0 && acc) atomicAdd(&ctrl->expand_bound, acc);
     }
-    if (lane == 0 && acc) atomicAdd(&P.ctrl->expand_bound, acc);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(&ctrl->blocks_done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    ctrl->blocks_done = 0;
+    ctrl->levels++;
+    if (failed) {
+        ctrl->halt = 1;
+        ctrl->go = 0;
+        return;
+    }
+    ctrl->src = 1 + out;
+    ctrl->ticket = 0;
+    ctrl->nticket = n;
+    ctrl->out_rows = 0;
+    if (n > ctrl->max_front) ctrl->max_front = n;
+    ctrl->go = !stop && *(volatile unsigned long long *)&ctrl->expand_bound <= P.frontier_cap;
+    ctrl->expand_bound = 0;
+    ctrl->t_start = device_ns();
 }
 
 }  // namespace
@@ -1573,25 +1619,24 @@ void launch_enumerate(const EnumParams &p, int blocks, int warps_per_block, int 
 }
 
 void launch_seed_tickets(const DevPlan *plans, uint32_t nplans, const unsigned long long *keys, uint32_t m,
-                         KeyLayout kl, uint32_t *seed_lo, uint32_t *ticket_prefix, EnumControl *ctrl,
-                         cudaStream_t s) {
+                         KeyLayout kl, uint32_t *seed_lo, uint32_t *ticket_prefix, cudaStream_t s) {
     // seed_lo holds three arrays of nplans: first key, end key, chunk count.
     uint32_t *chunks = seed_lo + 2 * nplans;
-    k_seed_ranges<<<(nplans + 127) / 128, 128, 0, s>>>(plans, nplans, keys, m, kl, seed_lo, chunks);
-    k_ticket_prefix<<<1, 1024, 0, s>>>(chunks, nplans, ticket_prefix, ctrl);
+    k_seed_ranges<<<(nplans + 3) / 4, 128, 0, s>>>(plans, nplans, keys, m, kl, seed_lo, chunks);
+    k_ticket_prefix<<<1, 1024, 0, s>>>(chunks, nplans, ticket_prefix);
 }
 
-void launch_ctrl_reset(EnumControl *ctrl, uint32_t active, unsigned long long nticket, cudaStream_t s) {
-    k_ctrl_reset<<<1, 1, 0, s>>>(ctrl, active, nticket);
+void launch_phase_begin(EnumControl *ctrl, const uint32_t *ticket_prefix, uint32_t nplans, bool expand,
+                        unsigned long long target, unsigned long long frontier_cap, cudaStream_t s) {
+    k_phase_begin<<<1, 128, 0, s>>>(ctrl, ticket_prefix + nplans, expand ? 1u : 0u, target, frontier_cap);
+}
+
+void launch_expand_decide(const EnumParams &p, bool last, unsigned long long target, cudaStream_t s) {
+    k_expand_decide<<<296, 256, 0, s>>>(p, last ? 1u : 0u, target);
 }
 
 void launch_pendant_counts(const EnumParams &p, uint32_t plan, unsigned long long *out, cudaStream_t s) {
     k_pendant_counts<<<148 * 8, 256, 0, s>>>(p, plan, out);
-}
-
-void launch_expand_bound(const EnumParams &p, const WorkItem *items, const unsigned long long *nitems,
-                         cudaStream_t s) {
-    k_expand_bound<<<296, 256, 0, s>>>(p, items, nitems);
 }
 
 }  // namespace csm

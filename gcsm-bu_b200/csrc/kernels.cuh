@@ -91,8 +91,10 @@ struct EnumParams {
     uint32_t phase;
     const uint32_t *seed_lo;         // per plan: first key of its seed relation
     const uint32_t *ticket_prefix;   // per plan: prefix of seed chunks (nplans + 1)
-    const WorkItem *frontier;        // alternative work source (semi-BFS frontier)
-    uint32_t nfrontier;
+    // Semi-BFS frontier buffers.  EnumControl.src names the one the launch reads (or the seed
+    // tickets); an expansion writes the other.
+    WorkItem *frontier[2];
+    unsigned long long frontier_cap; // items each of them holds
     WorkItem *queue;                 // donation ring (qmask + 1 slots)
     unsigned long long *seq;         // per slot: epoch << 32 | position (see EnumControl)
     uint32_t qmask;
@@ -101,8 +103,6 @@ struct EnumParams {
     uint32_t mode;                   // 0 count, 1 materialize, 2 expand one level
     uint32_t *rows;                  // materialize: rows of 1 + CSM_MAXQV words
     unsigned long long row_cap;
-    WorkItem *expand_out;
-    unsigned long long expand_cap;
     uint32_t donate;
     uint32_t steal_min;
     uint32_t idle_limit;             // polls of an idle warp waiting for donated work
@@ -128,13 +128,18 @@ size_t enum_smem_bytes(int warps_per_block);
 // resident 256-thread blocks per SM.
 int enum_blocks_per_sm(int warps_per_block, int occupancy);
 void launch_enumerate(const EnumParams &p, int blocks, int warps_per_block, int occupancy, cudaStream_t s);
+// Seed ranges and tickets of a batch (both phases read the same ones).
 void launch_seed_tickets(const DevPlan *plans, uint32_t nplans, const unsigned long long *keys, uint32_t m,
-                         KeyLayout kl, uint32_t *seed_lo, uint32_t *ticket_prefix, EnumControl *ctrl,
-                         cudaStream_t s);
-void launch_ctrl_reset(EnumControl *ctrl, uint32_t active, unsigned long long nticket, cudaStream_t s);
+                         KeyLayout kl, uint32_t *seed_lo, uint32_t *ticket_prefix, cudaStream_t s);
+// Starts a phase: control block reset, its tickets those of launch_seed_tickets.  With `expand`, an
+// expansion launch follows if the seeds are at least one, fewer than `target` and fit the frontier.
+void launch_phase_begin(EnumControl *ctrl, const uint32_t *ticket_prefix, uint32_t nplans, bool expand,
+                        unsigned long long target, unsigned long long frontier_cap, cudaStream_t s);
+// Between expansion launches: makes the level just written the next launch's source and decides
+// whether that launch expands it further (not when `last`, empty, of `target` items or more, or when
+// the bound of the next level exceeds the frontier buffers).
+void launch_expand_decide(const EnumParams &p, bool last, unsigned long long target, cudaStream_t s);
 // Fills table `out` (one entry per data vertex) for the pendant plan `plan` in this phase.
 void launch_pendant_counts(const EnumParams &p, uint32_t plan, unsigned long long *out, cudaStream_t s);
-void launch_expand_bound(const EnumParams &p, const WorkItem *items, const unsigned long long *nitems,
-                         cudaStream_t s);
 
 }  // namespace csm

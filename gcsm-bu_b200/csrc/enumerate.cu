@@ -514,7 +514,10 @@ __device__ bool try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl,
     const uint32_t top = pl->shared_last ? pl->n - 3u : d;
     // Above a pendant counting level, buffered candidates are settled from the table, never
     // entered: they are not handed out as items of the counting level either.
-    const uint32_t sib_end = pl->memo_slot != CSM_NO_MEMO ? E - 1u : E;
+    // The candidates above a tail that is counted one prefix at a time are handed out as items of
+    // depth E, a tail count each: those counts are long (20-100 us over hub lists).
+    const bool long_tail = E >= 3 && E < pl->n && !pl->tail.lane_par;
+    const uint32_t sib_end = pl->memo_slot != CSM_NO_MEMO ? E - 1u : long_tail ? E + 1u : E;
     for (uint32_t l = L0; l <= d && l <= top; l++) {
         const uint32_t lo = S.lo[l], hi = S.hi[l];
         const uint32_t minr = (l == 1) ? 64u : P.steal_min;
@@ -532,8 +535,9 @@ __device__ bool try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl,
             __syncwarp();
             return true;
         }
-        const uint32_t nb = S.nbuf[l], ps = S.pos[l];
-        if (l < d && l + 1 < sib_end && nb > ps) {
+        // Buffered siblings; of the current level's own buffer the next one stays.
+        const uint32_t nb = S.nbuf[l], ps = S.pos[l] + (l == d ? 1u : 0u);
+        if (l + 1 < sib_end && nb > ps) {
             const uint32_t cnt = nb - ps;
             const uint32_t slot = reserve_slots(P, cnt);
             if (slot == 0xFFFFFFFFu) return false;
@@ -987,7 +991,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
     const DevPlan *pl = P.plans + S.item_plan;
     const uint32_t n = pl->n;
     const uint32_t E = pl->tail_start;
-    const uint32_t L0 = S.item_depth == 0 ? 1u : S.item_depth;
+    uint32_t L0 = S.item_depth == 0 ? 1u : S.item_depth;
     unsigned long long cnt = 0;
 
     if (MODE == CSM_ENUM_MODE_EXPAND && L0 >= pl->expand_stop) {
@@ -1011,7 +1015,17 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
         return 0;
     }
 
-    if (L0 == 1) {
+    if (MODE == CSM_ENUM_MODE_COUNT && L0 == E && E < n) {
+        // A single prefix above a tail (see try_donate): the only buffered candidate of its level.
+        L0 = E - 1;
+        if (lane == 0) {
+            S.buf[L0][0] = S.f[L0];
+            S.nbuf[L0] = 1;
+            S.pos[L0] = 0;
+            S.lo[L0] = S.hi[L0] = 0;
+        }
+        __syncwarp();
+    } else if (L0 == 1) {
         if (lane == 0) {
             S.lo[1] = S.item_lo;
             S.hi[1] = S.item_hi;
@@ -1091,6 +1105,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             if (d + 1 == E) {
                 cnt += tail_count(S, P, pl, probes);
                 tails++;
+                iter |= 7u;  // look for waiting warps after every long step
             } else {
                 d++;
                 if (lane == 0 && d + 2 == n) S.sl_state = 0;  // a new prefix f[0..n-3]

@@ -32,6 +32,12 @@
 #define CSM_PHASE_INS 1
 #define CSM_PHASE_DEL 2
 
+// Entries of a tail key's list that its vertices may use: all of them, those that are no batch
+// edges, or batch edges only (the seed edge's leaf, see DevPlan.seed_group).
+#define CSM_KEY_ANY 0
+#define CSM_KEY_OLD 1
+#define CSM_KEY_BATCH 2
+
 // Maximum tail-leaf bookkeeping of one plan (Cartesian flattening, kernels/cartesian_product.cu).
 #define CSM_TAIL_MAXKEYS 8
 #define CSM_TAIL_MAXMASKS 32
@@ -70,7 +76,7 @@ struct DevTailTerm {
 struct DevTail {
     uint8_t nkeys;                              // distinct (parent depth, relation, old) lists
     uint8_t key_parent[CSM_TAIL_MAXKEYS];
-    uint8_t key_old[CSM_TAIL_MAXKEYS];
+    uint8_t key_old[CSM_TAIL_MAXKEYS];          // CSM_KEY_ANY, _OLD or _BATCH: entries that count
     uint16_t key_rel[CSM_TAIL_MAXKEYS];
     // Per key, bit j set when the query vertex at depth j has the key's leaf label: only the
     // data vertices matched at those depths can sit in the key's list (labels partition the
@@ -114,7 +120,20 @@ struct DevPlan {
     // not pendant; CSM_MEMO_PENDING: pendant, no table assigned yet).
     uint8_t memo_slot;
     uint8_t memo_depth;
+    // CSM_SEED_*: where the updated query edge ends in a leaf (a query vertex of degree one), all
+    // batch edges at one data vertex share everything but the leaf, so the search starts once per
+    // data vertex f[0] of the inner endpoint that owns batch edges, and the leaf is counted.  Depth
+    // 1 then holds no query vertex: f[1] is the number of f[0]'s batch edges in the seed relation.
+    // WEIGHT: no other query vertex can be matched to such an edge's end, so every match counts
+    // f[1] times.  TAIL: the leaf is a tail vertex (last in the order, one position past the query's
+    // vertices) with a CSM_KEY_BATCH key.
+    uint8_t seed_group;
 };
+
+#define CSM_SEED_EDGE 0
+#define CSM_SEED_WEIGHT 1
+#define CSM_SEED_TAIL 2
+#define CSM_NO_QV 0xFFu  // an order position without a query vertex
 
 #define CSM_NO_MEMO 0xFFu
 #define CSM_MEMO_PENDING 0xFEu

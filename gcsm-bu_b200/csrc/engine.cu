@@ -506,6 +506,8 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
             return rel_table_[((size_t)vl(q.vlabel[u]) * nel + el(q.edge_label(u, uu))) * nvl + vl(q.vlabel[uu])];
         };
         auto ps = build_plans(q, (uint16_t)qi, nlf_base_[qi], stats[qi], po, rel_of);
+        if (po.cartesian)
+            for (HostPlan &hp : ps) group_leaf_seeds(q, nlf_base_[qi], rel_of, hp);
         begin.push_back((uint32_t)plans.size());
         plans.insert(plans.end(), ps.begin(), ps.end());
     }

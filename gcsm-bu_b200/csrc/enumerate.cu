@@ -152,6 +152,19 @@ __device__ __forceinline__ uint32_t flagged_in_list(const EnumParams &P, uint32_
     return (h < P.m && P.kl.list_of(__ldg(P.keys + h)) == lk) ? __ldg(P.seg_flagged + h) : 0u;
 }
 
+// Whether entry e of a tail key's list counts under the key's rule (CSM_KEY_*).
+__device__ __forceinline__ bool key_counts(uint32_t rule, uint32_t e) {
+    return rule == CSM_KEY_ANY || (e & 1u) == (rule >> 1);
+}
+
+// Entries of list (rel, x), of `size` entries, that count under a tail key's rule.
+__device__ __forceinline__ uint32_t key_entries(const EnumParams &P, uint32_t rel, uint32_t x, uint32_t size,
+                                                uint32_t rule) {
+    if (rule == CSM_KEY_ANY) return size;
+    const uint32_t batch = flagged_in_list(P, rel, x);
+    return rule == CSM_KEY_OLD ? size - batch : batch;
+}
+
 // Lane-parallel tail, shared part: for the counting level d = tail_start - 1 and the current
 // prefix f[0..d-1], every tail key whose parent is matched before depth d gets its list and
 // the number of its entries the leaves may still use given that prefix.
@@ -163,15 +176,15 @@ __device__ void prep_tail_shared(WarpState &S, const EnumParams &P, const DevPla
         const uint32_t pd = __ldg(&T->key_parent[lane]);
         if (pd < d) {
             const uint32_t rel = __ldg(&T->key_rel[lane]);
-            const bool old = __ldg(&T->key_old[lane]) != 0;
+            const uint32_t rule = __ldg(&T->key_old[lane]);
             const uint32_t x = S.f[pd];
             const uint2 ms = list_of(P, rel, x, 100 + d);
-            uint32_t left = ms.y - (old ? flagged_in_list(P, rel, x) : 0u);
+            uint32_t left = key_entries(P, rel, x, ms.y, rule);
             const uint32_t excl = __ldg(&T->key_excl[lane]);
             for (uint32_t j = 0; j < d; j++) {
                 if (j == pd || !((excl >> j) & 1u)) continue;
                 const uint32_t e = find_entry(P.g.pool + ms.x, ms.y, S.f[j]);
-                if (e != 0xFFFFFFFFu && !(old && (e & 1u))) left--;
+                if (e != 0xFFFFFFFFu && key_counts(rule, e)) left--;
             }
             S.ts_off[lane] = ms.x;
             S.ts_size[lane] = ms.y;
@@ -197,24 +210,23 @@ __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uin
         if (k >= nkeys) break;
         const uint32_t pd = __ldg(&T->key_parent[k]);
         const uint32_t rel = __ldg(&T->key_rel[k]);
-        const bool old = __ldg(&T->key_old[k]) != 0;
+        const uint32_t rule = __ldg(&T->key_old[k]);
         uint32_t left;
         if (pd < d && d >= 2) {
             // Shared list: only this lane's candidate may still sit in it (looked up by the
             // warp beforehand, bit k of shared_hit).
             left = ts_base[k] - ((shared_hit >> k) & 1u);
-            (void)old;
         } else {
             const uint32_t x = (pd == d) ? v : x0;  // d >= 2: pd == d; d == 1: parent 0 or 1
             const uint2 ms = list_of(P, rel, x, 200 + d);
-            left = ms.y - (old ? flagged_in_list(P, rel, x) : 0u);
+            left = key_entries(P, rel, x, ms.y, rule);
             const uint32_t excl = __ldg(&T->key_excl[k]);
             for (uint32_t j = 0; j <= d; j++) {
                 if (j == pd || !((excl >> j) & 1u)) continue;
                 const uint32_t z = (j == d) ? v : (d == 1 ? x0 : f[j]);
                 const uint32_t e = find_entry(P.g.pool + ms.x, ms.y, z);
                 probes++;
-                if (e != 0xFFFFFFFFu && !(old && (e & 1u))) left--;
+                if (e != 0xFFFFFFFFu && key_counts(rule, e)) left--;
             }
         }
         ksize[k] = left;
@@ -299,7 +311,8 @@ __device__ uint32_t tail_intersection(WarpState &S, const EnumParams &P, const D
         }
     if (lane < nkeys) S.t_cur[lane] = 0;
     __syncwarp();
-    const bool old0 = __ldg(&T->key_old[k0]) != 0;
+    const uint32_t rule0 = __ldg(&T->key_old[k0]);
+    const uint32_t excl = __ldg(&T->key_excl[k0]) & ((1u << E) - 1u);  // the keys of a mask share their label
     uint32_t cnt = 0;
     for (uint32_t base = 0; base < best; base += 32) {
         const uint32_t idx = base + lane;
@@ -308,13 +321,13 @@ __device__ uint32_t tail_intersection(WarpState &S, const EnumParams &P, const D
         if (ok) {
             const uint32_t e = __ldg(P.g.pool + S.t_off[k0] + idx);
             w = e >> 1;
-            ok = !(old0 && (e & 1u));
+            ok = key_counts(rule0, e);
             if (w >= P.g.V) {
                 record_bad(P, CSM_BAD_ENTRY, e, S.t_off[k0] + idx, 700 + E);
                 ok = false;
             }
         }
-        for (uint32_t z = 0; ok && z < E; z++) ok = S.f[z] != w;
+        for (uint32_t em = excl; ok && em; em &= em - 1) ok = S.f[__ffs(em) - 1] != w;
         const uint32_t vmask = __ballot_sync(0xffffffffu, idx < best);
         const uint32_t target = __shfl_sync(0xffffffffu, w, 31 - __clz(vmask));
         const uint32_t key_hi = (target + 1) << 1;
@@ -337,7 +350,7 @@ __device__ uint32_t tail_intersection(WarpState &S, const EnumParams &P, const D
             }
             if (ok) {
                 probes++;
-                ok = e != 0xFFFFFFFFu && !(__ldg(&T->key_old[k]) && (e & 1u));
+                ok = e != 0xFFFFFFFFu && key_counts(__ldg(&T->key_old[k]), e);
             }
             __syncwarp();
             if (lane == 0) S.t_cur[k] = hi;
@@ -369,8 +382,8 @@ __device__ unsigned long long tail_count(WarpState &S, const EnumParams &P, cons
         const uint2 ms = list_of(P, rel, x, 300 + E);
         S.t_off[lane] = ms.x;
         S.t_size[lane] = ms.y;
-        // Flagged entries of this list = batch edges of (rel, x) in this phase.
-        S.t_flag[lane] = (__ldg(&T->key_old[lane]) && ((single >> lane) & 1u)) ? flagged_in_list(P, rel, x) : 0u;
+        // Entries of this list that do not count under its rule.
+        S.t_flag[lane] = ((single >> lane) & 1u) ? ms.y - key_entries(P, rel, x, ms.y, __ldg(&T->key_old[lane])) : 0u;
         S.t_excl[lane] = 0;
     }
     __syncwarp();
@@ -383,7 +396,7 @@ __device__ unsigned long long tail_count(WarpState &S, const EnumParams &P, cons
         const uint32_t z = S.f[pi % E];
         const uint32_t e = find_entry(P.g.pool + S.t_off[k], S.t_size[k], z);
         nprobe++;
-        if (e != 0xFFFFFFFFu && !(__ldg(&T->key_old[k]) && (e & 1u))) atomicAdd(&S.t_excl[k], 1u);
+        if (e != 0xFFFFFFFFu && key_counts(__ldg(&T->key_old[k]), e)) atomicAdd(&S.t_excl[k], 1u);
     }
     probes += nprobe;
     __syncwarp();
@@ -485,6 +498,14 @@ __device__ uint32_t reserve_slots(const EnumParams &P, uint32_t cnt) {
     return __shfl_sync(0xffffffffu, won, 0) ? pos : 0xFFFFFFFFu;
 }
 
+// f[0] and f[1] of the seed at sorted batch key c: the edge's endpoints, or, where the plan's seeds
+// are the inner endpoint's data vertices, that vertex and its number of batch edges (c is then the
+// first key of the vertex's list).
+__device__ __forceinline__ uint2 seed_pair(const EnumParams &P, const DevPlan *pl, uint32_t c) {
+    const unsigned long long key = __ldg(P.keys + c);
+    return make_uint2(P.kl.src(key), pl->seed_group == CSM_SEED_EDGE ? P.kl.dst(key) : __ldg(P.seg_flagged + c));
+}
+
 // Writes the item of ring position `pos` and publishes it with stamp (epoch, pos + 1).
 __device__ void publish_item(const EnumParams &P, uint32_t pos, uint32_t plan, uint32_t depth, uint32_t lo,
                              uint32_t hi, const uint32_t *prefix, uint32_t nprefix, bool extra, uint32_t extra_v,
@@ -544,8 +565,8 @@ __device__ bool try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl,
             for (uint32_t j = 0; j < cnt; j++) {
                 const uint32_t c = S.buf[l][ps + j];
                 if (l == 1) {
-                    const unsigned long long key = __ldg(P.keys + c);
-                    uint32_t pre[2] = {P.kl.src(key), P.kl.dst(key)};
+                    const uint2 seed = seed_pair(P, pl, c);
+                    uint32_t pre[2] = {seed.x, seed.y};
                     publish_item(P, slot + j, S.item_plan, 2, 0, 0xFFFFFFFFu, pre, 2, false, 0, 0);
                 } else {
                     publish_item(P, slot + j, S.item_plan, l + 1, 0, 0xFFFFFFFFu, S.f, l, true, c, l);
@@ -1039,6 +1060,9 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
     uint32_t d = L0;
     uint32_t iter = 0;
     unsigned long long sl_before = 0;
+    // Matches of the seeds already done, and what each match of the current seed counts.
+    unsigned long long total = 0;
+    uint32_t weight = S.item_depth >= 2 && pl->seed_group == CSM_SEED_WEIGHT ? S.f[1] : 1u;
     if (lane == 0) S.sl_state = 0;
     const uint32_t *nlf0 = bitmap(P, pl->nlf0);
     const uint32_t *nlf1 = bitmap(P, pl->nlf1);
@@ -1090,18 +1114,23 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 continue;
             // Descend into the next buffered candidate.
             const uint32_t c = S.buf[d][S.pos[d]];
+            if (d == 1) {
+                total += cnt * weight;  // the seed before this one is done
+                cnt = 0;
+            }
             __syncwarp();
             if (lane == 0) {
                 S.pos[d]++;
                 if (d == 1) {
-                    const unsigned long long key = __ldg(P.keys + c);
-                    S.f[0] = P.kl.src(key);
-                    S.f[1] = P.kl.dst(key);
+                    const uint2 seed = seed_pair(P, pl, c);
+                    S.f[0] = seed.x;
+                    S.f[1] = seed.y;
                 } else {
                     S.f[d] = c;
                 }
             }
             __syncwarp();
+            if (d == 1 && pl->seed_group == CSM_SEED_WEIGHT) weight = S.f[1];
             if (d + 1 == E) {
                 cnt += tail_count(S, P, pl, probes);
                 tails++;
@@ -1140,7 +1169,11 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             if (ok) {
                 const unsigned long long key = __ldg(P.keys + idx);
                 const uint32_t x = P.kl.src(key), y = P.kl.dst(key);
-                ok = __ldg(P.eff + idx) == P.phase && x != y && test_bit(nlf0, x) && test_bit(nlf1, y);
+                if (pl->seed_group == CSM_SEED_EDGE)
+                    ok = __ldg(P.eff + idx) == P.phase && x != y && test_bit(nlf0, x) && test_bit(nlf1, y);
+                else  // the first key of a list with batch edges (the leaf's NLF rule is implied)
+                    ok = (idx == 0 || P.kl.list_of(__ldg(P.keys + idx - 1)) != P.kl.list_of(key)) &&
+                         __ldg(P.seg_flagged + idx) > 0 && test_bit(nlf0, x);
                 cand = idx;
             }
         } else {
@@ -1235,9 +1268,9 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 o->lo = 0;
                 o->hi = 0xFFFFFFFFu;
                 if (d == 1) {
-                    const unsigned long long key = __ldg(P.keys + cand);
-                    o->f[0] = P.kl.src(key);
-                    o->f[1] = P.kl.dst(key);
+                    const uint2 seed = seed_pair(P, pl, cand);
+                    o->f[0] = seed.x;
+                    o->f[1] = seed.y;
                 } else {
                     for (uint32_t k = 0; k < d; k++) o->f[k] = S.f[k];
                     o->f[d] = cand;
@@ -1278,8 +1311,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                     if (lane == 0) S.ts_cur[k] = hi;
                     if (ok) {
                         probes++;
-                        const bool old_k = __ldg(&T->key_old[k]) != 0;
-                        if (e != 0xFFFFFFFFu && !(old_k && (e & 1u))) shared_hit |= 1u << k;
+                        if (e != 0xFFFFFFFFu && key_counts(__ldg(&T->key_old[k]), e)) shared_hit |= 1u << k;
                     }
                 }
                 __syncwarp();
@@ -1287,8 +1319,9 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             unsigned long long t = 0;
             if (ok) {
                 if (d == 1) {
-                    const unsigned long long key = __ldg(P.keys + cand);
-                    t = tail_count_lane(S.ts_base, S.f, P, pl, 1, P.kl.src(key), P.kl.dst(key), 0, probes);
+                    const uint2 seed = seed_pair(P, pl, cand);
+                    t = tail_count_lane(S.ts_base, S.f, P, pl, 1, seed.x, seed.y, 0, probes);
+                    if (pl->seed_group == CSM_SEED_WEIGHT) t *= seed.y;
                 } else {
                     t = tail_count_lane(S.ts_base, S.f, P, pl, d, 0, cand, shared_hit, probes);
                 }
@@ -1328,7 +1361,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             __syncwarp();
         }
     }
-    return cnt;
+    return total + cnt * weight;
 }
 
 // MINB resident blocks of 256 threads per SM: the register budget per thread follows from it.

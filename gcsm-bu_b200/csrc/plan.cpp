@@ -342,7 +342,9 @@ bool build_tail(const Query &q, const HostPlan &hp, int qe, const RelOf &rel_of,
             if ((int)p >= hp.tail_start) return false;  // not a tail: a neighbour in the tail
             uint32_t pu = hp.order[p];
             int rel = rel_of(pu, u);
-            int old = q.qe_index[pu * q.nv + u] > qe ? 1 : 0;
+            // The seed edge itself is a tail key only where its leaf is counted in the tail.
+            const int idx = q.qe_index[pu * q.nv + u];
+            int old = idx == qe ? CSM_KEY_BATCH : idx > qe ? CSM_KEY_OLD : CSM_KEY_ANY;
             auto k = std::make_tuple((int)p, rel, old);
             int ki = (int)(std::find(keys.begin(), keys.end(), k) - keys.begin());
             if (ki == (int)keys.size()) keys.push_back(k);
@@ -363,7 +365,7 @@ bool build_tail(const Query &q, const HostPlan &hp, int qe, const RelOf &rel_of,
             if ((l.keys >> k) & 1u) leaf_label = l.label;
         uint16_t excl = 0;
         for (int d = 0; d < n; d++)
-            if (q.vlabel[hp.order[d]] == leaf_label) excl |= (uint16_t)(1u << d);
+            if (hp.order[d] != CSM_NO_QV && q.vlabel[hp.order[d]] == leaf_label) excl |= (uint16_t)(1u << d);
         tail.key_excl[k] = excl;
     }
     std::map<uint32_t, std::vector<uint16_t>> classes;  // label -> the key sets of its vertices
@@ -427,6 +429,78 @@ bool build_tail(const Query &q, const HostPlan &hp, int qe, const RelOf &rel_of,
         if (__builtin_popcount(masks[k]) != 1) tail.lane_par = 0;
     }
     return true;
+}
+
+// Device form of a plan whose order and backward neighbours are set, with its tail from depth
+// `tail_start` or, where that tail exceeds the device tables, a later one.
+void pack_plan(const Query &q, uint32_t i, uint16_t query_id, uint32_t nlf_base, const RelOf &rel_of, bool materialize,
+               int tail_start, HostPlan &hp) {
+    const std::vector<uint8_t> &order = hp.order;
+    const uint32_t n = (uint32_t)order.size();
+    // Shorten the tail until its bookkeeping fits the device tables.
+    DevTail tail{};
+    std::vector<DevTailTerm> terms;
+    hp.tail_start = tail_start;
+    while (hp.tail_start < (int)n && !build_tail(q, hp, (int)i, rel_of, tail, terms)) hp.tail_start++;
+    if (hp.tail_start >= (int)n) {
+        hp.tail_start = (int)n;
+        std::memset(&tail, 0, sizeof(tail));
+        terms.clear();
+    }
+    hp.terms = terms;
+    DevPlan &dp = hp.dev;
+    std::memset(&dp, 0, sizeof(dp));
+    dp.query = query_id;
+    dp.n = (uint8_t)n;
+    dp.qe = (uint8_t)i;
+    dp.tail_start = (uint8_t)hp.tail_start;
+    dp.materialize = materialize ? 1 : 0;
+    for (uint32_t d = 0; d < n; d++) dp.order[d] = order[d];
+    dp.nlf0 = nlf_base + order[0];
+    if (order[1] != CSM_NO_QV) {
+        dp.seed_rel = rel_of(order[0], order[1]);
+        dp.nlf1 = nlf_base + order[1];
+    }
+    uint32_t bn_base = 0;
+    for (uint32_t d = 0; d < n; d++) {
+        DevLevel &lv = dp.lv[d];
+        lv.bn_base = (uint8_t)bn_base;
+        bn_base += (uint32_t)hp.bn[d].size();
+        lv.qv = order[d];
+        lv.nlf_bitmap = CSM_NO_BITMAP;
+        if (order[d] == CSM_NO_QV) continue;
+        lv.nbn = (uint8_t)hp.bn[d].size();
+        // All query neighbours matched before this level: the NLF filter is implied.
+        if (hp.bn[d].size() != q.nbrs[order[d]].size()) lv.nlf_bitmap = nlf_base + order[d];
+        for (uint32_t j = 0; j < d; j++)
+            if (order[j] != CSM_NO_QV && q.vlabel[order[j]] == q.vlabel[order[d]]) lv.excl_mask |= (uint16_t)(1u << j);
+        for (size_t k = 0; k < hp.bn[d].size(); k++) {
+            uint32_t bu = order[hp.bn[d][k]];
+            lv.bn_depth[k] = hp.bn[d][k];
+            lv.bn_rel[k] = rel_of(bu, order[d]);
+            if (q.qe_index[bu * q.nv + order[d]] > (int)i) lv.old_mask |= (uint16_t)(1u << k);
+        }
+    }
+    dp.tail = tail;
+    dp.nterms = (uint32_t)terms.size();
+    if (hp.tail_start == (int)n && n >= 4) {
+        dp.shared_last = 1;
+        for (uint8_t b : hp.bn[n - 1])
+            if (b == n - 2) dp.shared_last = 0;
+    }
+    dp.expand_stop = (uint8_t)(dp.shared_last ? n - 2 : hp.tail_start - 1);
+    dp.memo_slot = CSM_NO_MEMO;
+    const int c = hp.tail_start - 1;
+    if (hp.tail_start < (int)n && tail.lane_par && c >= 3 && hp.bn[c].size() == 1 && dp.lv[c].excl_mask == 0) {
+        bool pendant = true;
+        for (int k = 0; k < tail.nkeys; k++)
+            if (tail.key_parent[k] != c || (tail.key_excl[k] & ((1u << c) - 1u)) != 0) pendant = false;
+        if (pendant) {
+            dp.memo_slot = CSM_MEMO_PENDING;
+            dp.memo_depth = hp.bn[c][0];
+            dp.expand_stop = (uint8_t)(c - 1);
+        }
+    }
 }
 
 }  // namespace
@@ -513,69 +587,62 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
                 return st.avg[order[a] * n + u] < st.avg[order[b] * n + u];
             });
         }
-        // Shorten the tail until its bookkeeping fits the device tables.
-        DevTail tail{};
-        std::vector<DevTailTerm> terms;
-        hp.tail_start = tail_start;
-        while (hp.tail_start < (int)n && !build_tail(q, hp, (int)i, rel_of, tail, terms)) hp.tail_start++;
-        if (hp.tail_start >= (int)n) {
-            hp.tail_start = (int)n;
-            std::memset(&tail, 0, sizeof(tail));
-            terms.clear();
-        }
-        hp.terms = terms;
-        DevPlan &dp = hp.dev;
-        std::memset(&dp, 0, sizeof(dp));
-        dp.query = query_id;
-        dp.n = (uint8_t)n;
-        dp.qe = (uint8_t)i;
-        dp.tail_start = (uint8_t)hp.tail_start;
-        dp.materialize = opt.materialize ? 1 : 0;
-        dp.seed_rel = rel_of(order[0], order[1]);
-        for (uint32_t d = 0; d < n; d++) dp.order[d] = order[d];
-        dp.nlf0 = nlf_base + order[0];
-        dp.nlf1 = nlf_base + order[1];
-        uint32_t bn_base = 0;
-        for (uint32_t d = 0; d < n; d++) {
-            DevLevel &lv = dp.lv[d];
-            lv.bn_base = (uint8_t)bn_base;
-            bn_base += (uint32_t)hp.bn[d].size();
-            lv.qv = order[d];
-            lv.nbn = (uint8_t)hp.bn[d].size();
-            // All query neighbours matched before this level: the NLF filter is implied.
-            lv.nlf_bitmap = hp.bn[d].size() == q.nbrs[order[d]].size() ? CSM_NO_BITMAP : nlf_base + order[d];
-            for (uint32_t j = 0; j < d; j++)
-                if (q.vlabel[order[j]] == q.vlabel[order[d]]) lv.excl_mask |= (uint16_t)(1u << j);
-            for (size_t k = 0; k < hp.bn[d].size(); k++) {
-                uint32_t bu = order[hp.bn[d][k]];
-                lv.bn_depth[k] = hp.bn[d][k];
-                lv.bn_rel[k] = rel_of(bu, order[d]);
-                if (q.qe_index[bu * n + order[d]] > (int)i) lv.old_mask |= (uint16_t)(1u << k);
-            }
-        }
-        dp.tail = tail;
-        dp.nterms = (uint32_t)terms.size();
-        if (hp.tail_start == (int)n && n >= 4) {
-            dp.shared_last = 1;
-            for (uint8_t b : hp.bn[n - 1])
-                if (b == n - 2) dp.shared_last = 0;
-        }
-        dp.expand_stop = (uint8_t)(dp.shared_last ? n - 2 : hp.tail_start - 1);
-        dp.memo_slot = CSM_NO_MEMO;
-        const int c = hp.tail_start - 1;
-        if (hp.tail_start < (int)n && tail.lane_par && c >= 3 && hp.bn[c].size() == 1 && dp.lv[c].excl_mask == 0) {
-            bool pendant = true;
-            for (int k = 0; k < tail.nkeys; k++)
-                if (tail.key_parent[k] != c || (tail.key_excl[k] & ((1u << c) - 1u)) != 0) pendant = false;
-            if (pendant) {
-                dp.memo_slot = CSM_MEMO_PENDING;
-                dp.memo_depth = hp.bn[c][0];
-                dp.expand_stop = (uint8_t)(c - 1);
-            }
-        }
+        pack_plan(q, i, query_id, nlf_base, rel_of, opt.materialize, tail_start, hp);
         plans.push_back(hp);
     }
     return plans;
+}
+
+// The leaf of the seed edge is the only query vertex that tells its batch edges at one data vertex
+// apart.  Another query vertex x of the leaf's label can be matched to the far end of one of those
+// edges unless x hangs off the inner endpoint by an edge of the same relation that must be no batch
+// edge; where some x can, the leaf is counted in the tail, whose polynomial handles the overlap.
+bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp) {
+    const int i = hp.dev.qe;
+    const uint32_t n = (uint32_t)hp.order.size();
+    if (n < 3 || hp.dev.materialize) return false;
+    const bool first = q.degree(hp.order[0]) == 1, second = q.degree(hp.order[1]) == 1;
+    if (!first && !second) return false;
+    const uint8_t leaf = hp.order[first ? 0 : 1], inner = hp.order[first ? 1 : 0];
+    bool overlap = false;
+    for (uint32_t x = 0; x < q.nv; x++) {
+        if (x == leaf || x == inner || q.vlabel[x] != q.vlabel[leaf]) continue;
+        const int e = q.qe_index[inner * q.nv + x];
+        if (!(e > i && q.qe_elabel[e] == q.qe_elabel[i])) overlap = true;
+    }
+    if (overlap && n + 1 > CSM_MAXQV) return false;
+    HostPlan g;
+    g.order = {inner, CSM_NO_QV};
+    g.order.insert(g.order.end(), hp.order.begin() + 2, hp.order.end());
+    if (overlap) g.order.push_back(leaf);
+    const int m = (int)g.order.size();
+    std::vector<int> at(q.nv, -1);
+    for (int d = 0; d < m; d++)
+        if (g.order[d] != CSM_NO_QV) at[g.order[d]] = d;
+    // Every vertex keeps the backward neighbours (and their order) that it has in the plan.
+    g.bn.assign(m, {});
+    for (int d = 2; d < (int)n; d++)
+        for (uint8_t b : hp.bn[d]) g.bn[d].push_back((uint8_t)at[hp.order[b]]);
+    int tail_start = hp.tail_start;
+    if (overlap) {
+        g.bn[m - 1] = {0};
+        // The tail grows over the last head vertices adjacent to no tail vertex, as in build_plans.
+        while (tail_start > 2) {
+            bool free_vertex = true;
+            for (int t = tail_start; t < m; t++)
+                if (q.adjacent(g.order[tail_start - 1], g.order[t])) free_vertex = false;
+            if (!free_vertex) break;
+            tail_start--;
+        }
+    }
+    pack_plan(q, (uint32_t)i, hp.dev.query, nlf_base, rel_of, false, tail_start, g);
+    if (overlap && g.tail_start >= m) return false;
+    g.dev.seed_group = overlap ? CSM_SEED_TAIL : CSM_SEED_WEIGHT;
+    g.dev.seed_rel = rel_of(inner, leaf);
+    g.dev.nlf1 = nlf_base + leaf;
+    hp.dev = g.dev;
+    hp.terms = g.terms;
+    return true;
 }
 
 std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans) {
@@ -593,9 +660,11 @@ std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans) {
             }
             os << ") ";
         }
-        os << "\n    tail: " << (hp.tail_start < (int)hp.order.size() ? "from depth " + std::to_string(hp.tail_start) : std::string("none"))
+        os << "\n    tail: " << (hp.dev.tail_start < hp.dev.n ? "from depth " + std::to_string(hp.dev.tail_start) : std::string("none"))
            << ", " << hp.terms.size() << " terms" << (hp.dev.shared_last ? ", last level shared by the level above" : "")
            << (hp.dev.memo_slot != CSM_NO_MEMO ? ", pendant counting level" : "")
+           << (hp.dev.seed_group == CSM_SEED_WEIGHT ? ", leaf of the updated edge counted per inner vertex"
+               : hp.dev.seed_group == CSM_SEED_TAIL ? ", leaf of the updated edge counted in the tail" : "")
            << "\n";
     }
     return os.str();

@@ -47,6 +47,13 @@ using RelOf = std::function<uint16_t(uint32_t u, uint32_t uu)>;  // relation of 
 std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nlf_base,
                                   const EdgeStats &st, const PlanOptions &opt, const RelOf &rel_of);
 
+// Rewrites the device form of the plan of a query edge with a leaf endpoint so that its seeds are
+// the data vertices of the inner endpoint instead of the batch edges (DevPlan.seed_group); order,
+// bn and tail_start keep describing the plan it stands for.  Returns whether it did: not for edges
+// without a leaf, queries of two vertices or of CSM_MAXQV, or row-materialising plans, nor when the
+// leaf would need a tail that exceeds the device tables.
+bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp);
+
 // Text description, one block per query edge, in the spirit of PlanManager::PrintOrders.
 std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans);
 

@@ -1,0 +1,183 @@
+// Host-only check of group_leaf_seeds (gcsm-bu_b200/csrc/plan.cpp): on random labelled queries and
+// random data graphs with some edges marked as batch edges, the plan that starts once per data vertex
+// of the inner endpoint counts what the plan that starts at every batch edge counts.  Both device
+// forms are evaluated by the same small interpreter (levels, flag rules, exclusions, tail polynomial).
+#include <algorithm>
+#include <cstdio>
+#include <map>
+#include <random>
+#include <set>
+#include <tuple>
+#include <vector>
+
+#include "plan.h"
+#include "query.h"
+
+using namespace csm;
+
+namespace {
+
+struct Entry {
+    uint32_t v;
+    bool batch;
+};
+
+struct Graph {
+    uint32_t n = 0;
+    std::map<std::pair<int, uint32_t>, std::vector<Entry>> lists;  // (relation, vertex)
+    const std::vector<Entry> &list(int rel, uint32_t v) const {
+        static const std::vector<Entry> none;
+        auto it = lists.find({rel, v});
+        return it == lists.end() ? none : it->second;
+    }
+    // 0 = absent, 1 = present, 2 = present and a batch edge
+    int entry(int rel, uint32_t v, uint32_t w) const {
+        for (const Entry &e : list(rel, v))
+            if (e.v == w) return e.batch ? 2 : 1;
+        return 0;
+    }
+};
+
+bool counts(int rule, bool batch) { return rule == CSM_KEY_ANY || batch == (rule == CSM_KEY_BATCH); }
+
+long long tail(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, const uint32_t *f) {
+    const DevTail &t = p.tail;
+    std::vector<long long> size(t.nmasks, 0);
+    for (int mi = 0; mi < t.nmasks; mi++)
+        for (uint32_t w = 0; w < g.n; w++) {
+            bool ok = true;
+            for (int k = 0; ok && k < t.nkeys; k++) {
+                if (!((t.mask[mi] >> k) & 1u)) continue;
+                const int e = g.entry(t.key_rel[k], f[t.key_parent[k]], w);
+                ok = e && counts(t.key_old[k], e == 2);
+                for (int j = 0; ok && j < p.tail_start; j++)
+                    if (((t.key_excl[k] >> j) & 1u) && f[j] == w) ok = false;
+            }
+            size[mi] += ok;
+        }
+    long long total = 1;
+    for (int c = 0; c < t.nclasses; c++) {
+        long long s = 0;
+        for (int i = t.class_term_begin[c]; i < t.class_term_begin[c + 1]; i++) {
+            long long prod = terms[i].coef;
+            for (int j = 0; j < terms[i].nf; j++) prod *= size[terms[i].f[j]];
+            s += prod;
+        }
+        total *= s;
+    }
+    return total;
+}
+
+long long walk(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, uint32_t *f, int d) {
+    if (d == p.n) return 1;
+    if (d == p.tail_start) return tail(g, p, terms, f);
+    const DevLevel &lv = p.lv[d];
+    long long total = 0;
+    for (const Entry &e : g.list(lv.bn_rel[0], f[lv.bn_depth[0]])) {
+        bool ok = true;
+        for (int k = 0; ok && k < lv.nbn; k++) {
+            const int x = g.entry(lv.bn_rel[k], f[lv.bn_depth[k]], e.v);
+            ok = x && !(((lv.old_mask >> k) & 1u) && x == 2);
+        }
+        for (int j = 0; ok && j < d; j++)
+            if (((lv.excl_mask >> j) & 1u) && f[j] == e.v) ok = false;
+        if (!ok) continue;
+        f[d] = e.v;
+        total += walk(g, p, terms, f, d + 1);
+    }
+    return total;
+}
+
+long long count(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms) {
+    long long total = 0;
+    for (uint32_t v = 0; v < g.n; v++) {
+        uint32_t batch = 0;
+        for (const Entry &e : g.list(p.seed_rel, v)) batch += e.batch;
+        // The position without a query vertex holds a number: it must never be read as a vertex.
+        uint32_t f[CSM_MAXQV] = {v, batch};
+        if (p.seed_group != CSM_SEED_EDGE) {
+            if (batch) total += (p.seed_group == CSM_SEED_WEIGHT ? batch : 1) * walk(g, p, terms, f, 2);
+            continue;
+        }
+        for (const Entry &e : g.list(p.seed_rel, v)) {
+            if (!e.batch) continue;
+            f[1] = e.v;
+            total += walk(g, p, terms, f, 2);
+        }
+    }
+    return total;
+}
+
+}  // namespace
+
+int main() {
+    std::mt19937 rng(77);
+    int grouped[3] = {0, 0, 0}, nonzero = 0;
+    for (int qn = 0; qn < 300; qn++) {
+        const uint32_t nv = 2 + rng() % 5, nlab = 1 + rng() % 3;
+        std::vector<uint32_t> vl(nv), src, dst, el;
+        for (auto &x : vl) x = rng() % nlab;
+        std::set<std::pair<uint32_t, uint32_t>> seen;
+        for (uint32_t v = 1; v < nv; v++) {
+            const uint32_t p = rng() % v;
+            src.push_back(p), dst.push_back(v), el.push_back(rng() % 2);
+            seen.insert({p, v});
+        }
+        for (int e = (int)(rng() % 3); e > 0; e--) {
+            uint32_t a = rng() % nv, b = rng() % nv;
+            if (a > b) std::swap(a, b);
+            if (a == b || !seen.insert({a, b}).second) continue;
+            src.push_back(a), dst.push_back(b), el.push_back(rng() % 2);
+        }
+        Query q;
+        if (!build_query(nv, vl.data(), (uint32_t)src.size(), src.data(), dst.data(), el.data(), q).empty()) return 1;
+        std::map<std::tuple<uint32_t, uint32_t, uint32_t>, uint16_t> rels;
+        RelOf rel_of = [&](uint32_t u, uint32_t uu) -> uint16_t {
+            auto k = std::make_tuple(q.vlabel[u], q.edge_label(u, uu), q.vlabel[uu]);
+            return rels.emplace(k, (uint16_t)rels.size()).first->second;
+        };
+        EdgeStats st;
+        st.card.assign(nv * nv, 1);
+        st.avg.assign(nv * nv, 1.f);
+        for (auto &x : st.avg) x = 1.f + (float)(rng() % 100);
+        PlanOptions po;
+        po.order = (Order)(qn % 4);
+        std::vector<HostPlan> plans = build_plans(q, 0, 0, st, po, rel_of);
+        // A data graph of the query's labels; two labelled edges of one pair are two edges.
+        Graph g;
+        g.n = 9;
+        std::vector<uint32_t> gl(g.n);
+        for (auto &x : gl) x = rng() % nlab;
+        for (uint32_t a = 0; a < g.n; a++)
+            for (uint32_t b = a + 1; b < g.n; b++)
+                for (uint32_t l = 0; l < 2; l++) {
+                    if (rng() % 5 > 2) continue;
+                    const bool batch = rng() % 3 == 0;
+                    for (auto e : {std::make_pair(a, b), std::make_pair(b, a)}) {
+                        auto it = rels.find(std::make_tuple(gl[e.first], l, gl[e.second]));
+                        if (it != rels.end()) g.lists[{it->second, e.first}].push_back({e.second, batch});
+                    }
+                }
+        for (size_t i = 0; i < plans.size(); i++) {
+            HostPlan hp = plans[i];
+            const long long want = count(g, plans[i].dev, plans[i].terms);
+            const bool did = group_leaf_seeds(q, 0, rel_of, hp);
+            grouped[hp.dev.seed_group]++;
+            const auto &e = q.qe_list[i];
+            if (did != (nv > 2 && (q.degree(e.first) == 1 || q.degree(e.second) == 1))) {
+                std::printf("FAIL grouping of query %d plan %zu\n", qn, i);
+                return 1;
+            }
+            const long long got = count(g, hp.dev, hp.terms);
+            nonzero += did && want > 0;
+            if (got != want) {
+                std::printf("FAIL query %d plan %zu: %lld per inner vertex, %lld per batch edge\n", qn, i, got, want);
+                return 1;
+            }
+        }
+    }
+    if (grouped[CSM_SEED_WEIGHT] < 50 || grouped[CSM_SEED_TAIL] < 50 || nonzero < 100)
+        return std::printf("too few grouped plans: %d %d, %d with matches\n", grouped[1], grouped[2], nonzero), 1;
+    std::printf("ok %d weighted, %d in the tail, %d with matches\n", grouped[1], grouped[2], nonzero);
+    return 0;
+}

@@ -43,6 +43,12 @@
 #define CSM_TAIL_MAXMASKS 32
 #define CSM_TAIL_MAXCLASSES 8
 
+#define CSM_NO_PAIR 0xFFFFu
+#define CSM_PAIR_SWAP 0x8000u
+#define CSM_PAIR_SIGS 4095        // signatures fit 12 bits of a table entry's tag, the phase 20
+#define CSM_PAIR_PHASES 0xFFFFFu
+#define CSM_PAIR_MAXMASKS 8       // most masks of a pair_par tail
+
 // One matching-order level (one query vertex) of a plan.
 struct DevLevel {
     uint16_t bn_rel[CSM_MAXBN];   // relation of (backward neighbour -> this vertex)
@@ -85,7 +91,13 @@ struct DevTail {
     uint8_t nmasks;                             // key subsets whose intersection size is used
     uint8_t nclasses;
     uint8_t lane_par;                           // every mask is one key: count 32 prefixes per warp step
+    uint8_t pair_par;                           // every mask is one key or a pair with a memo signature: same
+    uint8_t single;                             // keys that are a mask by themselves
     uint16_t mask[CSM_TAIL_MAXMASKS];
+    // Signature of a mask of two keys, CSM_NO_PAIR for every other: the two (relation, rule) pairs.
+    // The size of the intersection is a function of it and the two data vertices, kept per phase in a
+    // table that all warps share.  Bit 15: the keys stand the other way round in the signature.
+    uint16_t mask_pair[CSM_TAIL_MAXMASKS];
     uint16_t class_term_begin[CSM_TAIL_MAXCLASSES + 1];  // into the plan's term list
 };
 
@@ -175,6 +187,7 @@ struct alignas(128) EnumControl {
     unsigned int halt;                // an expansion failed: the counting launch returns at once
     unsigned int levels;              // expansion launches that ran
     unsigned int blocks_done;         // blocks of the deciding launch that have finished
+    unsigned int pair_phase;          // phase number of the engine's pair table (1 .. CSM_PAIR_PHASES)
     unsigned long long max_front;     // largest frontier of the phase
     alignas(128) unsigned int q_head; // donation positions reserved (8-byte aligned pair with q_tail)
     unsigned int q_tail;              // donation positions taken by warps out of work

@@ -174,7 +174,7 @@ Engine::~Engine() {
                    g_.vlab, d_plans_, d_terms_, d_upd_src_, d_upd_dst_, d_upd_lab_, d_upd_del_, d_keys_raw_, d_keys_,
                    d_sort_temp_, bs_.eff, bs_.heads, bs_.nheads, bs_.seg_nins, bs_.seg_ndel, bs_.seg_end, bs_.scr_y,
                    bs_.scr_lb, bs_.counters, bs_.error, d_ctrl_, d_queue_, d_seq_, d_seed_lo_, d_ticket_prefix_,
-                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_};
+                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_, d_pairs_, d_pair_phase_};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (h_pin_) cudaFreeHost(h_pin_);
@@ -562,6 +562,8 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
         memo_plan.clear();
     }
     memo_plan_ = std::move(memo_plan);
+    const csm_status pst = install_pairs(plans);
+    if (pst != CSM_OK) return pst;
     std::vector<DevPlan> dplans;
     std::vector<DevTailTerm> terms;
     for (auto &hp : plans) {
@@ -591,6 +593,54 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
     // Breadth-first launches a phase can need: from the seeds to the deepest expandable level.
     expand_levels_ = 0;
     for (const auto &hp : plans_) expand_levels_ = std::max(expand_levels_, (int)hp.dev.expand_stop - 1);
+    return CSM_OK;
+}
+
+// Signatures of the tails' pair masks, shared by all plans, and the table of their counts.
+csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
+    // 4M entries (64 MB) stay in the L2 cache; like the pendant tables they take a quarter of the
+    // free memory at most.
+    constexpr uint32_t kPairSlots = 1u << 22;
+    std::vector<std::pair<uint32_t, uint32_t>> sigs;
+    bool used = false;
+    for (HostPlan &hp : plans) {
+        DevTail &t = hp.dev.tail;
+        bool all = hp.dev.tail_start < hp.dev.n && hp.dev.tail_start >= 3 && t.nmasks <= CSM_PAIR_MAXMASKS && !t.lane_par;
+        for (int m = 0; m < t.nmasks; m++) {
+            const int bits = __builtin_popcount(t.mask[m]);
+            if (bits != 2) {
+                all = all && bits == 1;
+                continue;
+            }
+            const int ka = __builtin_ctz(t.mask[m]), kb = 31 - __builtin_clz(t.mask[m]);
+            uint32_t a = (uint32_t)t.key_rel[ka] << 2 | t.key_old[ka], b = (uint32_t)t.key_rel[kb] << 2 | t.key_old[kb];
+            const bool swap = b < a;
+            if (swap) std::swap(a, b);
+            const size_t id = std::find(sigs.begin(), sigs.end(), std::make_pair(a, b)) - sigs.begin();
+            if (id >= CSM_PAIR_SIGS) {
+                all = false;
+                continue;
+            }
+            if (id == sigs.size()) sigs.push_back({a, b});
+            t.mask_pair[m] = (uint16_t)(id | (swap ? CSM_PAIR_SWAP : 0u));
+        }
+        t.pair_par = all ? 1 : 0;
+        used = used || all;
+    }
+    if (used && !d_pairs_) {
+        size_t free_b = 0, total_b = 0;
+        const size_t want = sizeof(uint4) * (size_t)kPairSlots;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 4 &&
+            dev_alloc(&d_pair_phase_, 1) == cudaSuccess && dev_alloc(&d_pairs_, kPairSlots) == cudaSuccess) {
+            pair_slots_ = kPairSlots;
+            pair_phases_ = CSM_PAIR_PHASES;  // cleared before the first batch
+        } else {
+            (void)cudaGetLastError();
+            d_pairs_ = nullptr;
+        }
+    }
+    if (!d_pairs_)
+        for (HostPlan &hp : plans) hp.dev.tail.pair_par = 0;
     return CSM_OK;
 }
 
@@ -1049,6 +1099,13 @@ csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *ds
     last_frontier_rows_ = 0;
     deferred_ = CSM_OK;
     NlfTables nt{d_spec_begin_, d_specs_, d_bits_, words_};
+    if (d_pairs_ && pair_phases_ + 64 > CSM_PAIR_PHASES) {
+        // Entries carry the number of their phase; before the numbers run out the table starts over.
+        CSM_CUDA(cudaMemsetAsync(d_pairs_, 0, sizeof(uint4) * (size_t)pair_slots_, s));
+        CSM_CUDA(cudaMemsetAsync(d_pair_phase_, 0, sizeof(unsigned int), s));
+        pair_phases_ = 0;
+    }
+    pair_phases_ += 2 * (tune_left_ > 0 ? tune_cands_.size() + 1 : 2);  // the batch's phases, a rerun's too
     const bool tuning = tune_left_ > 0 && !no_alloc_ && cfg_.materialize_rows == 0;
     csm_status est;
     if (graphs_on() && !tuning && src == d_upd_src_)
@@ -1223,7 +1280,10 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
     const bool expand = strategy >= 2 && !rows && frontier_cap_ > 0;
     const unsigned long long target =
         strategy == 2 ? (unsigned long long)lc_.frontier_mult * total_warps : ~0ull;
-    launch_phase_begin(sc_.ctrl, sc_.ticket_prefix, np, expand, target, frontier_cap_, s);
+    launch_phase_begin(sc_.ctrl, sc_.ticket_prefix, np, expand, target, frontier_cap_, d_pairs_ ? d_pair_phase_ : nullptr,
+                       s);
+    P.pairs = d_pairs_;
+    P.pair_slots = pair_slots_;
     stats_.kernel_launches++;
     for (int b = 0; b < 2; b++) P.frontier[b] = expand ? d_frontier_[b] : nullptr;
     P.frontier_cap = expand ? frontier_cap_ : 0;

@@ -255,6 +255,7 @@ class Engine {
     bool tables_ready_ = false;
     csm_status compute_edge_stats(std::vector<EdgeStats> &stats);
     csm_status install_plans(const std::vector<EdgeStats> &stats);
+    csm_status install_pairs(std::vector<HostPlan> &plans);
     csm_status maybe_replan();
     size_t terms_cap_ = 0;
     long long *d_rel_delta_ = nullptr;      // [R] net entry change of the current batch
@@ -281,6 +282,10 @@ class Engine {
     int warps_per_block_ = 8;
     int occupancy_ = 4;                       // enumeration kernel variant (blocks per SM)
     int blocks_ = 0;
+    uint4 *d_pairs_ = nullptr;                // pair table, null when no plan uses it
+    unsigned int *d_pair_phase_ = nullptr;    // phases it has seen, counted on the device
+    uint32_t pair_slots_ = 0;
+    uint64_t pair_phases_ = 0;                // the same, an upper bound kept by the host
     int expand_levels_ = 0;                   // most breadth-first levels any plan expands
     LaunchConfig lc_{};                       // configuration in use
     std::vector<LaunchConfig> tune_cands_;    // autotuner candidates

@@ -172,7 +172,7 @@ __device__ void prep_tail_shared(WarpState &S, const EnumParams &P, const DevPla
     const uint32_t lane = lane_id();
     const DevTail *T = &pl->tail;
     const uint32_t nkeys = __ldg(&T->nkeys);
-    if (lane < nkeys) {
+    if (lane < nkeys && ((__ldg(&T->single) >> lane) & 1u)) {
         const uint32_t pd = __ldg(&T->key_parent[lane]);
         if (pd < d) {
             const uint32_t rel = __ldg(&T->key_rel[lane]);
@@ -195,9 +195,33 @@ __device__ void prep_tail_shared(WarpState &S, const EnumParams &P, const DevPla
     __syncwarp();
 }
 
-// Lane-parallel tail, per lane: the tail count of the prefix f[0..d-1] + v, where v is this
-// lane's candidate at depth d (for d == 1 the prefix is the seed edge (x0, v)).  Only for
-// plans whose masks are single keys (no list intersections).
+// Lane-parallel tail, per lane: what is left of tail key k's list for the prefix f[0..d-1] + v, where
+// v is this lane's candidate at depth d (for d == 1 the prefix is the seed (x0, v)).
+__device__ __forceinline__ uint32_t tail_key_left(const uint32_t *ts_base, const uint32_t *f, const EnumParams &P,
+                                                  const DevTail *T, uint32_t k, uint32_t d, uint32_t x0, uint32_t v,
+                                                  uint32_t shared_hit, uint32_t &probes) {
+    const uint32_t pd = __ldg(&T->key_parent[k]);
+    // Shared list: only this lane's candidate may still sit in it (looked up by the warp beforehand,
+    // bit k of shared_hit).
+    if (pd < d && d >= 2) return ts_base[k] - ((shared_hit >> k) & 1u);
+    const uint32_t rel = __ldg(&T->key_rel[k]);
+    const uint32_t rule = __ldg(&T->key_old[k]);
+    const uint32_t x = (pd == d) ? v : x0;  // d >= 2: pd == d; d == 1: parent 0 or 1
+    const uint2 ms = list_of(P, rel, x, 200 + d);
+    uint32_t left = key_entries(P, rel, x, ms.y, rule);
+    const uint32_t excl = __ldg(&T->key_excl[k]);
+    for (uint32_t j = 0; j <= d; j++) {
+        if (j == pd || !((excl >> j) & 1u)) continue;
+        const uint32_t z = (j == d) ? v : (d == 1 ? x0 : f[j]);
+        const uint32_t e = find_entry(P.g.pool + ms.x, ms.y, z);
+        probes++;
+        if (e != 0xFFFFFFFFu && key_counts(rule, e)) left--;
+    }
+    return left;
+}
+
+// Lane-parallel tail, per lane: the tail count of the prefix f[0..d-1] + v.  Only for plans whose
+// masks are single keys (no list intersections).
 __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uint32_t *f, const EnumParams &P,
                                               const DevPlan *pl,
                                               uint32_t d, uint32_t x0, uint32_t v, uint32_t shared_hit,
@@ -208,28 +232,7 @@ __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uin
 #pragma unroll
     for (uint32_t k = 0; k < CSM_TAIL_MAXKEYS; k++) {
         if (k >= nkeys) break;
-        const uint32_t pd = __ldg(&T->key_parent[k]);
-        const uint32_t rel = __ldg(&T->key_rel[k]);
-        const uint32_t rule = __ldg(&T->key_old[k]);
-        uint32_t left;
-        if (pd < d && d >= 2) {
-            // Shared list: only this lane's candidate may still sit in it (looked up by the
-            // warp beforehand, bit k of shared_hit).
-            left = ts_base[k] - ((shared_hit >> k) & 1u);
-        } else {
-            const uint32_t x = (pd == d) ? v : x0;  // d >= 2: pd == d; d == 1: parent 0 or 1
-            const uint2 ms = list_of(P, rel, x, 200 + d);
-            left = key_entries(P, rel, x, ms.y, rule);
-            const uint32_t excl = __ldg(&T->key_excl[k]);
-            for (uint32_t j = 0; j <= d; j++) {
-                if (j == pd || !((excl >> j) & 1u)) continue;
-                const uint32_t z = (j == d) ? v : (d == 1 ? x0 : f[j]);
-                const uint32_t e = find_entry(P.g.pool + ms.x, ms.y, z);
-                probes++;
-                if (e != 0xFFFFFFFFu && key_counts(rule, e)) left--;
-            }
-        }
-        ksize[k] = left;
+        ksize[k] = tail_key_left(ts_base, f, P, T, k, d, x0, v, shared_hit, probes);
     }
     // Masks are single keys here: mask mi stands for key ffs(mask) - 1.
     unsigned long long total = 1;
@@ -247,6 +250,172 @@ __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uin
 #pragma unroll
                 for (uint32_t k = 0; k < CSM_TAIL_MAXKEYS; k++)
                     if (mk == (1u << k)) sz = ksize[k];
+                prod *= sz;
+            }
+            s += prod;
+        }
+        total *= s;
+    }
+    return total;
+}
+
+// Entries that two sorted lists share, each under its rule (CSM_KEY_*).  The warp scans the shorter
+// list 32 entries at a time; every lane searches its entry in the window of the longer list that the
+// chunk spans, which starts where the last chunk ended and is doubled until it holds the chunk's
+// largest entry.  The window is a power of two and reads past the end count as large, so the search
+// has no data-dependent branch: log2(window) dependent reads, most of them from a few cache lines.
+__device__ uint32_t intersect_lists(const EnumParams &P, uint2 a, uint32_t rule_a, uint2 b, uint32_t rule_b) {
+    const uint32_t lane = lane_id();
+    if (b.y < a.y) {
+        const uint2 t = a;
+        a = b;
+        b = t;
+        const uint32_t r = rule_a;
+        rule_a = rule_b;
+        rule_b = r;
+    }
+    const uint32_t *A = P.g.pool + a.x, *B = P.g.pool + b.x;
+    // First window: twice what a chunk spans on average.
+    const uint32_t per = a.y ? b.y / a.y : 0u;
+    const uint32_t w0 = 64u << (per ? 31 - __clz(per) : 0);
+    uint32_t cnt = 0, c0 = 0;
+    for (uint32_t base = 0; base < a.y && c0 < b.y; base += 32) {
+        const uint32_t i = base + lane;
+        const uint32_t e = i < a.y ? __ldg(A + i) : 0xFFFFFFFFu;
+        const uint32_t key = e & ~1u;
+        const uint32_t last = a.y - base < 32u ? a.y - base - 1u : 31u;
+        const uint32_t top = __shfl_sync(0xffffffffu, key, last);
+        uint32_t w = w0;
+        while (w < b.y - c0 && __ldg(B + c0 + w - 1u) < top) w <<= 1;
+        uint32_t pos = c0;
+        for (uint32_t s = w >> 1; s; s >>= 1) {
+            const uint32_t p = pos + s - 1u;
+            const uint32_t v = p < b.y ? __ldg(B + p) : 0xFFFFFFFFu;
+            if (v < key) pos += s;
+        }
+        const uint32_t g = pos < b.y ? __ldg(B + pos) : 0xFFFFFFFFu;
+        const bool hit = i < a.y && (g & ~1u) == key && g != 0xFFFFFFFFu && key_counts(rule_a, e) && key_counts(rule_b, g);
+        cnt += __popc(__ballot_sync(0xffffffffu, hit));
+        c0 = __shfl_sync(0xffffffffu, pos, last);
+    }
+    return cnt;
+}
+
+// Slot of the pair table for (a, b) under `tag`.
+__device__ __forceinline__ uint4 *pair_slot(const EnumParams &P, uint32_t a, uint32_t b, uint32_t tag) {
+    uint32_t h = a * 0x9E3779B1u ^ (b * 0x85EBCA77u + tag * 0xC2B2AE3Du);
+    h ^= h >> 15;
+    h *= 0x2C1B3C6Du;
+    h ^= h >> 13;
+    return P.pairs + (h & (P.pair_slots - 1u));
+}
+
+// A table entry is read and written as one 128-bit access, so a reader sees an entry of one writer.
+__device__ __forceinline__ uint4 load_pair(const uint4 *slot) {
+    unsigned long long lo, hi;
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(slot)
+                 : "memory");
+    return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+
+__device__ __forceinline__ void store_pair(uint4 *slot, uint32_t a, uint32_t b, uint32_t tag, uint32_t count) {
+    const unsigned long long lo = (unsigned long long)b << 32 | a, hi = (unsigned long long)count << 32 | tag;
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%0, %1}; st.relaxed.gpu.global.b128 [%2], t; }" ::"l"(lo), "l"(hi), "l"(slot)
+                 : "memory");
+}
+
+// Size of the pair mask mi for this lane's prefix f[0..d-1] + cand (where ok): from the pair table, or
+// counted by the whole warp, one missing pair after the other, and put there.  The table holds the
+// intersection of the two lists under their rules; the prefix vertices of the mask's label that sit in
+// both are taken off here.
+__device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const DevTail *T, uint32_t mi, uint32_t d, bool ok,
+                              uint32_t cand) {
+    const uint32_t lane = lane_id();
+    const uint32_t mask = __ldg(&T->mask[mi]), sig = __ldg(&T->mask_pair[mi]);
+    uint32_t ka = __ffs(mask) - 1, kb = 31 - __clz(mask);
+    if (sig & CSM_PAIR_SWAP) {
+        const uint32_t t = ka;
+        ka = kb;
+        kb = t;
+    }
+    const uint32_t pa = __ldg(&T->key_parent[ka]), pb = __ldg(&T->key_parent[kb]);
+    const uint32_t ra = __ldg(&T->key_rel[ka]), rb = __ldg(&T->key_rel[kb]);
+    const uint32_t rule_a = __ldg(&T->key_old[ka]), rule_b = __ldg(&T->key_old[kb]);
+    const uint32_t tag = P.ctrl->pair_phase << 12 | (sig & 0xFFFu);
+    const uint32_t a = pa == d ? cand : S.f[pa], b = pb == d ? cand : S.f[pb];
+    uint32_t ta = a, tb = b;  // lists of one relation and rule: either order is the same pair
+    if (ra == rb && rule_a == rule_b && b < a) {
+        ta = b;
+        tb = a;
+    }
+    uint4 *slot = pair_slot(P, ta, tb, tag);
+    uint32_t count = 0;
+    bool miss = false;
+    if (ok) {
+        const uint4 e = load_pair(slot);
+        miss = e.x != ta || e.y != tb || e.z != tag;
+        count = e.w;
+    }
+    for (uint32_t need = __ballot_sync(0xffffffffu, miss); need;) {
+        const uint32_t l = __ffs(need) - 1;
+        const uint32_t va = __shfl_sync(0xffffffffu, a, l), vb = __shfl_sync(0xffffffffu, b, l);
+        const uint32_t c = intersect_lists(P, list_of(P, ra, va, 1000 + d), rule_a, list_of(P, rb, vb, 1000 + d), rule_b);
+        const bool same = miss && a == va && b == vb;
+        if (same) count = c;
+        if (lane == l) store_pair(slot, ta, tb, tag, c);
+        need &= ~__ballot_sync(0xffffffffu, same);
+    }
+    uint32_t excl = __ldg(&T->key_excl[ka]) & ((2u << d) - 1u) & ~(1u << pa) & ~(1u << pb);
+    if (excl && ok) {
+        const uint2 la = list_of(P, ra, a, 1100 + d), lb = list_of(P, rb, b, 1100 + d);
+        for (; excl; excl &= excl - 1) {
+            const uint32_t j = __ffs(excl) - 1, z = j == d ? cand : S.f[j];
+            const uint32_t ea = find_entry(P.g.pool + la.x, la.y, z);
+            if (ea == 0xFFFFFFFFu || !key_counts(rule_a, ea)) continue;
+            const uint32_t eb = find_entry(P.g.pool + lb.x, lb.y, z);
+            if (eb != 0xFFFFFFFFu && key_counts(rule_b, eb)) count--;
+        }
+    }
+    return count;
+}
+
+// Lane-parallel tail with pair masks (DevTail.pair_par), counting level d >= 2: the tail count of the
+// prefix f[0..d-1] + cand for every lane with ok set (0 for the others).  A pair of data vertices
+// recurs under many prefixes — the lists of two vertices intersect the same whatever was matched
+// between them — so most sizes are one table read instead of a scan of two lists.
+__device__ unsigned long long tail_count_pairs(const WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t d,
+                                               bool ok, uint32_t cand, uint32_t shared_hit, uint32_t &probes) {
+    const DevTail *T = &pl->tail;
+    const uint32_t nmasks = __ldg(&T->nmasks);
+    uint32_t msize[CSM_PAIR_MAXMASKS];
+#pragma unroll
+    for (uint32_t mi = 0; mi < CSM_PAIR_MAXMASKS; mi++) {
+        if (mi >= nmasks) break;
+        if (__ldg(&T->mask_pair[mi]) != CSM_NO_PAIR) {
+            msize[mi] = pair_size(S, P, T, mi, d, ok, cand);
+        } else {
+            msize[mi] = 0;
+            if (ok)
+                msize[mi] = tail_key_left(S.ts_base, S.f, P, T, __ffs(__ldg(&T->mask[mi])) - 1, d, 0, cand, shared_hit, probes);
+        }
+    }
+    unsigned long long total = ok ? 1 : 0;
+    const DevTailTerm *terms = P.terms + pl->term_begin;
+    const uint32_t nclasses = __ldg(&T->nclasses);
+    for (uint32_t c = 0; c < nclasses; c++) {
+        unsigned long long s = 0;
+        const uint32_t tb = __ldg(&T->class_term_begin[c]), te = __ldg(&T->class_term_begin[c + 1]);
+        for (uint32_t t = tb; t < te; t++) {
+            unsigned long long prod = (unsigned long long)__ldg(&terms[t].coef);
+            const uint32_t nf = __ldg(&terms[t].nf);
+            for (uint32_t j = 0; j < nf; j++) {
+                const uint32_t mi = __ldg(&terms[t].f[j]);
+                uint32_t sz = 0;
+#pragma unroll
+                for (uint32_t k = 0; k < CSM_PAIR_MAXMASKS; k++)
+                    if (mi == k) sz = msize[k];
                 prod *= sz;
             }
             s += prod;
@@ -292,7 +461,8 @@ __device__ void enter_level(WarpState &S, const EnumParams &P, const DevPlan *pl
         S.exm[d] = __ldg(&lv->excl_mask);
     }
     __syncwarp();
-    if (d + 1 == pl->tail_start && pl->tail_start < pl->n && pl->tail.lane_par) prep_tail_shared(S, P, pl, d);
+    if (d + 1 == pl->tail_start && pl->tail_start < pl->n && (pl->tail.lane_par || pl->tail.pair_par))
+        prep_tail_shared(S, P, pl, d);
 }
 
 // Size of the intersection of the tail lists in `mask` (at least two), each under its flag rule,
@@ -537,7 +707,7 @@ __device__ bool try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl,
     // entered: they are not handed out as items of the counting level either.
     // The candidates above a tail that is counted one prefix at a time are handed out as items of
     // depth E, a tail count each: those counts are long (20-100 us over hub lists).
-    const bool long_tail = E >= 3 && E < pl->n && !pl->tail.lane_par;
+    const bool long_tail = E >= 3 && E < pl->n && !pl->tail.lane_par && !pl->tail.pair_par;
     const uint32_t sib_end = pl->memo_slot != CSM_NO_MEMO ? E - 1u : long_tail ? E + 1u : E;
     for (uint32_t l = L0; l <= d && l <= top; l++) {
         const uint32_t lo = S.lo[l], hi = S.hi[l];
@@ -1004,7 +1174,7 @@ __device__ unsigned long long settle_pendant(WarpState &S, const EnumParams &P, 
 // Runs one work item to completion (or until the device clock passes `deadline`, when that is
 // nonzero: the rest of the item is then dropped and CSM_ERRBIT_TIMEOUT set).  Returns the number
 // of matches counted.
-template <bool LASTLOOP, int MODE>
+template <bool LASTLOOP, bool PAIRS, int MODE>
 __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32_t &scans,
                                        uint32_t &probes, uint32_t &tails, uint32_t &shared, unsigned int &err,
                                        unsigned long long deadline, WorkItem *expand_out) {
@@ -1277,7 +1447,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 }
             }
             __syncwarp();
-        } else if (d + 1 == E && E < n && pl->tail.lane_par) {
+        } else if (d + 1 == E && E < n && (pl->tail.lane_par || (PAIRS && pl->tail.pair_par))) {
             // Counting level before the tail: every surviving lane sizes its own tail.  Lists
             // shared by the chunk (parent matched above this level) are searched by the warp
             // with a cursor, as the probe lists are: the chunk's candidates ascend.
@@ -1289,7 +1459,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 const uint32_t tgt = __shfl_sync(0xffffffffu, cand, 31 - __clz(vm));
                 const uint32_t key_hi = (tgt + 1) << 1;
                 for (uint32_t k = 0; k < nkeys; k++) {
-                    if (__ldg(&T->key_parent[k]) >= d) continue;
+                    if (__ldg(&T->key_parent[k]) >= d || !((__ldg(&T->single) >> k) & 1u)) continue;
                     if (!((__ldg(&T->key_excl[k]) >> d) & 1u)) continue;  // candidates never in this list
                     if (!__any_sync(0xffffffffu, ok)) break;
                     const uint32_t *L = P.g.pool + S.ts_off[k];
@@ -1317,7 +1487,10 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 __syncwarp();
             }
             unsigned long long t = 0;
-            if (ok) {
+            if (PAIRS && pl->tail.pair_par) {
+                t = tail_count_pairs(S, P, pl, d, ok, cand, shared_hit, probes);
+                iter |= 7u;
+            } else if (ok) {
                 if (d == 1) {
                     const uint2 seed = seed_pair(P, pl, cand);
                     t = tail_count_lane(S.ts_base, S.f, P, pl, 1, seed.x, seed.y, 0, probes);
@@ -1367,7 +1540,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
 // MINB resident blocks of 256 threads per SM: the register budget per thread follows from it.
 // MODE: CSM_ENUM_MODE_* of the launch (each variant holds only its mode's code, which keeps the
 // hot loop's instruction footprint small).
-template <int MINB, bool LASTLOOP, int MODE>
+template <int MINB, bool LASTLOOP, bool PAIRS, int MODE>
 __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     WarpState &S = reinterpret_cast<WarpState *>(smem)[threadIdx.x >> 5];
@@ -1411,7 +1584,7 @@ __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
             if (got < 0) continue;
             if (!got) break;
         }
-        const unsigned long long c = run_item<LASTLOOP, MODE>(S, P, scans, probes, tails, shared, err, deadline, expand_out);
+        const unsigned long long c = run_item<LASTLOOP, PAIRS, MODE>(S, P, scans, probes, tails, shared, err, deadline, expand_out);
         if (lane == 0 && c) atomicAdd(P.counts + S.item_plan, c);
         if ((scans | probes | tails | shared) >= (1u << 30)) {
             atomicAdd(&P.ctrl->scan_entries, (unsigned long long)scans);
@@ -1504,7 +1677,7 @@ __global__ void __launch_bounds__(1024) k_ticket_prefix(const uint32_t *chunks, 
 // previous one plus one, kept on the device so that every phase on this scratch gets a fresh epoch
 // whichever engine, stream or replayed graph issues it.
 __global__ void k_phase_begin(EnumControl *ctrl, const uint32_t *nticket, uint32_t expand, unsigned long long target,
-                              unsigned long long frontier_cap) {
+                              unsigned long long frontier_cap, unsigned int *pair_phase) {
     uint32_t *w = reinterpret_cast<uint32_t *>(ctrl);
     uint32_t epoch = ctrl->epoch + 1u;
     if (epoch == 0) epoch = 1;
@@ -1517,6 +1690,7 @@ __global__ void k_phase_begin(EnumControl *ctrl, const uint32_t *nticket, uint32
     ctrl->nticket = *nticket;
     ctrl->go = expand && seeds > 0 && seeds < target && seeds <= frontier_cap;
     ctrl->t_start = device_ns();
+    if (pair_phase) ctrl->pair_phase = *pair_phase = *pair_phase + 1u;
 }
 
 // Table of a pendant plan (DevPlan.memo_slot): for every data vertex v, the count of its
@@ -1630,17 +1804,19 @@ size_t enum_smem_bytes(int warps_per_block) { return sizeof(WarpState) * (size_t
 namespace {
 using EnumKernel = void (*)(EnumParams);
 template <int MINB>
-EnumKernel enum_kernel_mode(bool last_loop, uint32_t mode) {
-    if (mode == CSM_ENUM_MODE_EXPAND) return k_enumerate<MINB, false, CSM_ENUM_MODE_EXPAND>;
-    if (mode == CSM_ENUM_MODE_ROWS) return k_enumerate<MINB, false, CSM_ENUM_MODE_ROWS>;
-    return last_loop ? k_enumerate<MINB, true, CSM_ENUM_MODE_COUNT> : k_enumerate<MINB, false, CSM_ENUM_MODE_COUNT>;
+EnumKernel enum_kernel_mode(bool last_loop, bool pairs, uint32_t mode) {
+    if (mode == CSM_ENUM_MODE_EXPAND) return k_enumerate<MINB, false, false, CSM_ENUM_MODE_EXPAND>;
+    if (mode == CSM_ENUM_MODE_ROWS) return k_enumerate<MINB, false, false, CSM_ENUM_MODE_ROWS>;
+    if (pairs)
+        return last_loop ? k_enumerate<MINB, true, true, CSM_ENUM_MODE_COUNT> : k_enumerate<MINB, false, true, CSM_ENUM_MODE_COUNT>;
+    return last_loop ? k_enumerate<MINB, true, false, CSM_ENUM_MODE_COUNT> : k_enumerate<MINB, false, false, CSM_ENUM_MODE_COUNT>;
 }
 
-EnumKernel enum_kernel(int occupancy, bool last_loop, uint32_t mode) {
+EnumKernel enum_kernel(int occupancy, bool last_loop, bool pairs, uint32_t mode) {
     switch (occupancy) {
-        case 6: return enum_kernel_mode<6>(last_loop, mode);
-        case 5: return enum_kernel_mode<5>(last_loop, mode);
-        default: return enum_kernel_mode<4>(last_loop, mode);
+        case 6: return enum_kernel_mode<6>(last_loop, pairs, mode);
+        case 5: return enum_kernel_mode<5>(last_loop, pairs, mode);
+        default: return enum_kernel_mode<4>(last_loop, pairs, mode);
     }
 }
 }  // namespace
@@ -1649,8 +1825,8 @@ int enum_blocks_per_sm(int warps_per_block, int occupancy) {
     // The smallest residency of the variants: a persistent grid must fit each of them.
     const size_t smem = enum_smem_bytes(warps_per_block);
     int best = 1 << 30;
-    for (int v = 0; v < 4; v++) {
-        EnumKernel k = enum_kernel(occupancy, v == 1, v < 2 ? CSM_ENUM_MODE_COUNT : (uint32_t)(v - 1));
+    for (int v = 0; v < 6; v++) {
+        EnumKernel k = enum_kernel(occupancy, v & 1, v & 2, v < 4 ? CSM_ENUM_MODE_COUNT : (uint32_t)(v - 3));
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int nb = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, warps_per_block * 32, smem) != cudaSuccess) return 1;
@@ -1661,7 +1837,7 @@ int enum_blocks_per_sm(int warps_per_block, int occupancy) {
 
 void launch_enumerate(const EnumParams &p, int blocks, int warps_per_block, int occupancy, cudaStream_t s) {
     const size_t smem = enum_smem_bytes(warps_per_block);
-    EnumKernel k = enum_kernel(occupancy, p.last_loop != 0, p.mode);
+    EnumKernel k = enum_kernel(occupancy, p.last_loop != 0, p.pairs != nullptr, p.mode);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k<<<blocks, warps_per_block * 32, smem, s>>>(p);
 }
@@ -1675,8 +1851,9 @@ void launch_seed_tickets(const DevPlan *plans, uint32_t nplans, const unsigned l
 }
 
 void launch_phase_begin(EnumControl *ctrl, const uint32_t *ticket_prefix, uint32_t nplans, bool expand,
-                        unsigned long long target, unsigned long long frontier_cap, cudaStream_t s) {
-    k_phase_begin<<<1, 128, 0, s>>>(ctrl, ticket_prefix + nplans, expand ? 1u : 0u, target, frontier_cap);
+                        unsigned long long target, unsigned long long frontier_cap, unsigned int *pair_phase,
+                        cudaStream_t s) {
+    k_phase_begin<<<1, 128, 0, s>>>(ctrl, ticket_prefix + nplans, expand ? 1u : 0u, target, frontier_cap, pair_phase);
 }
 
 void launch_expand_decide(const EnumParams &p, bool last, unsigned long long target, cudaStream_t s) {

@@ -116,6 +116,10 @@ struct EnumParams {
     // Pendant counting levels (DevPlan.memo_slot): per table, the count below a prefix for every
     // data vertex at the plan's memo_depth; nullptr counts those levels like any other.
     const unsigned long long *memo;
+    // Pair table (DevTail.mask_pair): pair_slots entries of 16 bytes {vertex, vertex, phase << 12 |
+    // signature, count}, a power of two of them, or nullptr.
+    uint4 *pairs;
+    uint32_t pair_slots;
 };
 
 #define CSM_ROW_WORDS (1 + CSM_MAXQV)
@@ -133,8 +137,10 @@ void launch_seed_tickets(const DevPlan *plans, uint32_t nplans, const unsigned l
                          KeyLayout kl, uint32_t *seed_lo, uint32_t *ticket_prefix, cudaStream_t s);
 // Starts a phase: control block reset, its tickets those of launch_seed_tickets.  With `expand`, an
 // expansion launch follows if the seeds are at least one, fewer than `target` and fit the frontier.
+// `pair_phase` counts the phases that the engine's pair table has seen (nullptr without a table).
 void launch_phase_begin(EnumControl *ctrl, const uint32_t *ticket_prefix, uint32_t nplans, bool expand,
-                        unsigned long long target, unsigned long long frontier_cap, cudaStream_t s);
+                        unsigned long long target, unsigned long long frontier_cap, unsigned int *pair_phase,
+                        cudaStream_t s);
 // Between expansion launches: makes the level just written the next launch's source and decides
 // whether that launch expands it further (not when `last`, empty, of `target` items or more, or when
 // the bound of the next level exceeds the frontier buffers).

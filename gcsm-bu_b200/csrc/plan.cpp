@@ -427,7 +427,9 @@ bool build_tail(const Query &q, const HostPlan &hp, int qe, const RelOf &rel_of,
     for (size_t k = 0; k < masks.size(); k++) {
         tail.mask[k] = masks[k];
         if (__builtin_popcount(masks[k]) != 1) tail.lane_par = 0;
+        else tail.single |= (uint8_t)masks[k];
     }
+    for (size_t k = 0; k < CSM_TAIL_MAXMASKS; k++) tail.mask_pair[k] = CSM_NO_PAIR;
     return true;
 }
 
@@ -574,8 +576,13 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
                 tail_start--;
             }
             // Without leaves, one or two such vertices are counted faster by the last-level
-            // loops (the shared last level covers two).
-            if (leaf_start == (int)n && (int)n - tail_start < 3) tail_start = (int)n;
+            // loops (the shared last level covers two) — but two of different labels with two lists
+            // each are a product of two pair intersections, which the pair table mostly holds.
+            if (leaf_start == (int)n && (int)n - tail_start < 3) {
+                const uint32_t a = order[n - 2], b = order[n - 1];
+                if ((int)n - tail_start != 2 || q.vlabel[a] == q.vlabel[b] || q.degree(a) != 2 || q.degree(b) != 2)
+                    tail_start = (int)n;
+            }
         }
         hp.order = order;
         hp.bn.assign(n, {});

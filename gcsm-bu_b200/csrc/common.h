@@ -93,6 +93,7 @@ struct DevTail {
     uint8_t lane_par;                           // every mask is one key: count 32 prefixes per warp step
     uint8_t pair_par;                           // every mask is one key or a pair with a memo signature: same
     uint8_t single;                             // keys that are a mask by themselves
+    uint8_t deep;                               // pendant plans: classes whose keys hang off depth c
     uint16_t mask[CSM_TAIL_MAXMASKS];
     // Signature of a mask of two keys, CSM_NO_PAIR for every other: the two (relation, rule) pairs.
     // The size of the intersection is a function of it and the two data vertices, kept per phase in a
@@ -130,8 +131,13 @@ struct DevPlan {
     // with c or a tail vertex.  The count below a prefix is then a function of the one data vertex
     // at memo_depth, precomputed for every vertex per phase into table memo_slot (CSM_NO_MEMO:
     // not pendant; CSM_MEMO_PENDING: pendant, no table assigned yet).
+    // Also where, beside that, some tail classes hang off vertices matched before c and do not share
+    // c's label (they are a factor of the prefix), and where prefix vertices share c's label (depths of
+    // lv[c].excl_mask): each such vertex that is a candidate of c takes its own tail value off the
+    // sum.  Table memo_tail holds those values, the tail count below c for every data vertex at c.
     uint8_t memo_slot;
     uint8_t memo_depth;
+    uint8_t memo_tail;
     // CSM_SEED_*: where the updated query edge ends in a leaf (a query vertex of degree one), all
     // batch edges at one data vertex share everything but the leaf, so the search starts once per
     // data vertex f[0] of the inner endpoint that owns batch edges, and the leaf is counted.  Depth

@@ -174,7 +174,7 @@ Engine::~Engine() {
                    g_.vlab, d_plans_, d_terms_, d_upd_src_, d_upd_dst_, d_upd_lab_, d_upd_del_, d_keys_raw_, d_keys_,
                    d_sort_temp_, bs_.eff, bs_.heads, bs_.nheads, bs_.seg_nins, bs_.seg_ndel, bs_.seg_end, bs_.scr_y,
                    bs_.scr_lb, bs_.counters, bs_.error, d_ctrl_, d_queue_, d_seq_, d_seed_lo_, d_ticket_prefix_,
-                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_, d_pairs_, d_pair_phase_};
+                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_, d_memo_desc_, d_pairs_, d_pair_phase_};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (h_pin_) cudaFreeHost(h_pin_);
@@ -507,61 +507,85 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
         };
         auto ps = build_plans(q, (uint16_t)qi, nlf_base_[qi], stats[qi], po, rel_of);
         if (po.cartesian)
-            for (HostPlan &hp : ps) group_leaf_seeds(q, nlf_base_[qi], rel_of, hp);
+            for (HostPlan &hp : ps) {
+                group_leaf_seeds(q, nlf_base_[qi], rel_of, hp);
+                extend_pendant(hp);
+            }
         begin.push_back((uint32_t)plans.size());
         plans.insert(plans.end(), ps.begin(), ps.end());
     }
     begin.push_back((uint32_t)plans.size());
     if (!plans_.empty() && plans.size() != plans_.size()) return fail(CSM_ERR_STATE, "re-planning changed the plan count");
-    // Pendant plans with the same counting level and tail read one table: its entries do not
-    // depend on the depths or on the query.  At most kMaxPendantTables tables (V entries each);
+    // Pendant plans with the same counting level and deep tail classes read one table: its entries do
+    // not depend on the depths or on the query.  The tail values it sums are a table too, shared by
+    // what hangs off the counting vertex alone.  At most kMaxPendantTables of each (V entries);
     // further pendant plans, or all of them when the tables do not fit, count normally.
     constexpr size_t kMaxPendantTables = 16;
-    std::vector<std::vector<int64_t>> sigs;
-    std::vector<uint32_t> memo_plan;
+    std::vector<std::vector<int64_t>> sigs, tail_sigs;
+    std::vector<uint32_t> tables;  // per table: representative plan, slot, tail values' slot
     for (uint32_t i = 0; i < plans.size(); i++) {
         DevPlan &dp = plans[i].dev;
         if (dp.memo_slot != CSM_MEMO_PENDING) continue;
         const DevLevel &lv = dp.lv[dp.tail_start - 1];
         const DevTail &t = dp.tail;
-        std::vector<int64_t> sig{lv.bn_rel[0], lv.old_mask & 1, lv.nlf_bitmap, t.nkeys, t.nmasks, t.nclasses};
-        for (int k = 0; k < t.nkeys; k++) sig.insert(sig.end(), {t.key_rel[k], t.key_old[k]});
-        for (int k = 0; k < t.nmasks; k++) sig.push_back(t.mask[k]);
-        for (int c = 0; c <= t.nclasses; c++) sig.push_back(t.class_term_begin[c]);
-        for (const DevTailTerm &term : plans[i].terms) {
-            sig.insert(sig.end(), {term.coef, term.nf});
-            for (int j = 0; j < term.nf; j++) sig.push_back(term.f[j]);
+        std::vector<int64_t> tail_sig;
+        for (int c = 0; c < t.nclasses; c++) {
+            if (!((t.deep >> c) & 1u)) continue;
+            tail_sig.push_back(-1);
+            for (int x = t.class_term_begin[c]; x < t.class_term_begin[c + 1]; x++) {
+                const DevTailTerm &term = plans[i].terms[x];
+                tail_sig.insert(tail_sig.end(), {term.coef, term.nf});
+                for (int j = 0; j < term.nf; j++) {
+                    const int k = __builtin_ctz(t.mask[term.f[j]]);
+                    tail_sig.insert(tail_sig.end(), {t.key_rel[k], t.key_old[k]});
+                }
+            }
         }
+        std::vector<int64_t> sig{lv.bn_rel[0], lv.old_mask & 1, lv.nlf_bitmap};
+        sig.insert(sig.end(), tail_sig.begin(), tail_sig.end());
         size_t slot = std::find(sigs.begin(), sigs.end(), sig) - sigs.begin();
+        const size_t ts = std::find(tail_sigs.begin(), tail_sigs.end(), tail_sig) - tail_sigs.begin();
         if (slot == sigs.size()) {
             if (sigs.size() == kMaxPendantTables) continue;
             sigs.push_back(sig);
-            memo_plan.push_back(i);
+            if (ts == tail_sigs.size()) tail_sigs.push_back(tail_sig);
+            tables.insert(tables.end(), {i, (uint32_t)slot, (uint32_t)ts});
         }
         dp.memo_slot = (uint8_t)slot;
+        dp.memo_tail = (uint8_t)ts;
     }
-    if (memo_plan.size() > memo_cap_) {
+    // Tail value tables come first.
+    const uint32_t ntail = (uint32_t)tail_sigs.size();
+    for (size_t t = 0; t < tables.size(); t += 3) tables[t + 1] += ntail;
+    for (auto &hp : plans)
+        if (hp.dev.memo_slot < CSM_MEMO_PENDING) hp.dev.memo_slot = (uint8_t)(hp.dev.memo_slot + ntail);
+    const size_t ntables = ntail + sigs.size();
+    if (ntables > memo_cap_) {
         if (d_memo_) cudaFree(d_memo_);
         d_memo_ = nullptr;
         memo_cap_ = 0;
         // The tables are an optimisation: they only take memory the adjacency pool is unlikely
         // to need (at most a quarter of what is free now).
         size_t free_b = 0, total_b = 0;
-        const size_t want = memo_plan.size() * (size_t)g_.V * sizeof(unsigned long long);
+        const size_t want = ntables * (size_t)g_.V * sizeof(unsigned long long);
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 4 &&
-            dev_alloc(&d_memo_, memo_plan.size() * (size_t)g_.V) == cudaSuccess) {
-            memo_cap_ = memo_plan.size();
+            (d_memo_desc_ || dev_alloc(&d_memo_desc_, 3 * kMaxPendantTables) == cudaSuccess) &&
+            dev_alloc(&d_memo_, ntables * (size_t)g_.V) == cudaSuccess) {
+            memo_cap_ = ntables;
         } else {
             (void)cudaGetLastError();
             d_memo_ = nullptr;
         }
     }
-    if (memo_plan.size() > memo_cap_) {
+    if (ntables > memo_cap_) {
         for (auto &hp : plans)
             if (hp.dev.memo_slot != CSM_NO_MEMO) hp.dev.memo_slot = CSM_MEMO_PENDING;
-        memo_plan.clear();
+        tables.clear();
     }
-    memo_plan_ = std::move(memo_plan);
+    memo_tables_ = (uint32_t)(tables.size() / 3);
+    if (memo_tables_)
+        CSM_CUDA(cudaMemcpyAsync(d_memo_desc_, tables.data(), sizeof(uint32_t) * tables.size(), cudaMemcpyHostToDevice,
+                                 stream_));
     const csm_status pst = install_pairs(plans);
     if (pst != CSM_OK) return pst;
     std::vector<DevPlan> dplans;
@@ -1302,11 +1326,10 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
     // Work donation in the depth-first launch for every strategy but 1 ("DFS w/o work
     // stealing"); after a BFS phase (strategy 3) it evens out the frontier items' subtrees.
     D.donate = strategy == 1 ? 0u : 1u;
-    if (!rows && !memo_plan_.empty()) {
+    if (!rows && memo_tables_) {
         // Tables of the pendant plans for this phase's graph and flags.
-        for (size_t t = 0; t < memo_plan_.size(); t++)
-            launch_pendant_counts(D, memo_plan_[t], d_memo_ + t * (size_t)g_.V, s);
-        stats_.kernel_launches += memo_plan_.size();
+        launch_pendant_tables(D, d_memo_desc_, memo_tables_, d_memo_, s);
+        stats_.kernel_launches += 2;
         D.memo = d_memo_;
     }
     launch_enumerate(D, blocks_, warps_per_block_, occupancy_, s);

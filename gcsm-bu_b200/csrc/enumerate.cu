@@ -220,25 +220,16 @@ __device__ __forceinline__ uint32_t tail_key_left(const uint32_t *ts_base, const
     return left;
 }
 
-// Lane-parallel tail, per lane: the tail count of the prefix f[0..d-1] + v.  Only for plans whose
-// masks are single keys (no list intersections).
-__device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uint32_t *f, const EnumParams &P,
-                                              const DevPlan *pl,
-                                              uint32_t d, uint32_t x0, uint32_t v, uint32_t shared_hit,
-                                              uint32_t &probes) {
+// Value of a tail polynomial whose masks are single keys (mask mi stands for key ffs(mask) - 1), over
+// the tail classes in `classes`.
+__device__ __forceinline__ unsigned long long tail_product(const EnumParams &P, const DevPlan *pl,
+                                                           const uint32_t (&ksize)[CSM_TAIL_MAXKEYS], uint32_t classes) {
     const DevTail *T = &pl->tail;
-    const uint32_t nkeys = __ldg(&T->nkeys);
-    uint32_t ksize[CSM_TAIL_MAXKEYS];
-#pragma unroll
-    for (uint32_t k = 0; k < CSM_TAIL_MAXKEYS; k++) {
-        if (k >= nkeys) break;
-        ksize[k] = tail_key_left(ts_base, f, P, T, k, d, x0, v, shared_hit, probes);
-    }
-    // Masks are single keys here: mask mi stands for key ffs(mask) - 1.
     unsigned long long total = 1;
     const DevTailTerm *terms = P.terms + pl->term_begin;
     const uint32_t nclasses = __ldg(&T->nclasses);
     for (uint32_t c = 0; c < nclasses; c++) {
+        if (!((classes >> c) & 1u)) continue;
         unsigned long long s = 0;
         const uint32_t tb = __ldg(&T->class_term_begin[c]), te = __ldg(&T->class_term_begin[c + 1]);
         for (uint32_t t = tb; t < te; t++) {
@@ -257,6 +248,23 @@ __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uin
         total *= s;
     }
     return total;
+}
+
+// Lane-parallel tail, per lane: the tail count of the prefix f[0..d-1] + v.  Only for plans whose
+// masks are single keys (no list intersections).
+__device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uint32_t *f, const EnumParams &P,
+                                              const DevPlan *pl,
+                                              uint32_t d, uint32_t x0, uint32_t v, uint32_t shared_hit,
+                                              uint32_t &probes) {
+    const DevTail *T = &pl->tail;
+    const uint32_t nkeys = __ldg(&T->nkeys);
+    uint32_t ksize[CSM_TAIL_MAXKEYS];
+#pragma unroll
+    for (uint32_t k = 0; k < CSM_TAIL_MAXKEYS; k++) {
+        if (k >= nkeys) break;
+        ksize[k] = tail_key_left(ts_base, f, P, T, k, d, x0, v, shared_hit, probes);
+    }
+    return tail_product(P, pl, ksize, 0xFFu);
 }
 
 // Entries that two sorted lists share, each under its rule (CSM_KEY_*).  The warp scans the shorter
@@ -1150,18 +1158,58 @@ __device__ unsigned long long count_shared_last(WarpState &S, const EnumParams &
 }
 
 // Pendant counting level c = d + 1 (DevPlan.memo_slot): every buffered candidate of level d
-// contributes the table entry of the data vertex at memo_depth (the candidate itself when that
-// depth is d).  Consumes the buffer.
+// contributes the table entry of the data vertex y at memo_depth (the candidate itself when that
+// depth is d), less the tail values of the prefix vertices of c's label that are candidates of c below
+// y, times the tail classes that hang off the prefix.  Consumes the buffer.
 __device__ unsigned long long settle_pendant(WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t d,
                                              uint32_t &tails) {
     const uint32_t lane = lane_id();
     const uint32_t ps = S.pos[d], k = S.nbuf[d] - ps;
     const uint32_t md = pl->memo_depth;
-    const unsigned long long *table = P.memo + (size_t)pl->memo_slot * P.g.V;
+    const DevTail *T = &pl->tail;
+    const DevLevel *lv = &pl->lv[d + 1];
     unsigned long long v = 0;
     if (lane < k) {
-        const uint32_t x = md == d ? S.buf[d][ps + lane] : S.f[md];
-        v = __ldg(table + x);
+        const uint32_t x = S.buf[d][ps + lane];
+        const uint32_t y = md == d ? x : S.f[md];
+        v = __ldg(P.memo + (size_t)pl->memo_slot * P.g.V + y);
+        uint32_t excl = __ldg(&lv->excl_mask) & ~(1u << md);
+        if (excl && v) {
+            const uint2 ms = list_of(P, __ldg(&lv->bn_rel[0]), y, 950 + d);
+            const bool old = (__ldg(&lv->old_mask) & 1u) != 0;
+            const uint32_t nlf_id = __ldg(&lv->nlf_bitmap);
+            for (; excl; excl &= excl - 1) {
+                const uint32_t j = __ffs(excl) - 1, z = j == d ? x : S.f[j];
+                const uint32_t e = find_entry(P.g.pool + ms.x, ms.y, z);
+                if (e == 0xFFFFFFFFu || (old && (e & 1u))) continue;
+                if (nlf_id != CSM_NO_BITMAP && !test_bit(bitmap(P, nlf_id), z)) continue;
+                v -= __ldg(P.memo + (size_t)pl->memo_tail * P.g.V + z);
+            }
+        }
+        const uint32_t rest = ((1u << __ldg(&T->nclasses)) - 1u) & ~__ldg(&T->deep);
+        if (rest && v) {
+            const uint32_t nkeys = __ldg(&T->nkeys);
+            uint32_t ksize[CSM_TAIL_MAXKEYS];
+#pragma unroll
+            for (uint32_t q = 0; q < CSM_TAIL_MAXKEYS; q++) {
+                if (q >= nkeys) break;
+                const uint32_t pd = __ldg(&T->key_parent[q]);
+                ksize[q] = 0;
+                if (pd > d) continue;
+                const uint32_t rel = __ldg(&T->key_rel[q]), rule = __ldg(&T->key_old[q]);
+                const uint32_t p = pd == d ? x : S.f[pd];
+                const uint2 ms = list_of(P, rel, p, 960 + d);
+                uint32_t left = key_entries(P, rel, p, ms.y, rule);
+                uint32_t em = __ldg(&T->key_excl[q]) & ((2u << d) - 1u) & ~(1u << pd);
+                for (; em; em &= em - 1) {
+                    const uint32_t j = __ffs(em) - 1;
+                    const uint32_t e = find_entry(P.g.pool + ms.x, ms.y, j == d ? x : S.f[j]);
+                    if (e != 0xFFFFFFFFu && key_counts(rule, e)) left--;
+                }
+                ksize[q] = left;
+            }
+            v *= tail_product(P, pl, ksize, rest);
+        }
     }
     tails += k;  // warp-uniform, like every other use of the tail counter
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1693,55 +1741,75 @@ __global__ void k_phase_begin(EnumControl *ctrl, const uint32_t *nticket, uint32
     if (pair_phase) ctrl->pair_phase = *pair_phase = *pair_phase + 1u;
 }
 
-// Table of a pendant plan (DevPlan.memo_slot): for every data vertex v, the count of its
-// counting level c for a prefix whose vertex at memo_depth is v — the candidates w of v's list
-// under the flag rule and c's NLF filter, each with its Cartesian tail, exactly as the
-// lane-parallel counting level sums them (no prefix exclusion can apply).  One warp per vertex.
-__global__ void k_pendant_counts(EnumParams P, uint32_t plan, unsigned long long *out) {
+// Tail values of the pendant plans (DevPlan.memo_tail): for every data vertex w at the counting level,
+// the deep tail classes' count below it (no prefix vertex can sit in their lists).  blockIdx.y names
+// the table; the first of those that share tail values fills them.
+__global__ void k_tail_values(EnumParams P, const uint32_t *desc, unsigned long long *memo) {
+    const DevPlan *pl = P.plans + desc[3 * blockIdx.y];
+    const uint32_t slot = desc[3 * blockIdx.y + 2];
+    for (uint32_t t = 0; t < blockIdx.y; t++)
+        if (desc[3 * t + 2] == slot) return;
+    unsigned long long *out = memo + (size_t)slot * P.g.V;
+    const DevTail *T = &pl->tail;
+    const uint32_t c = pl->tail_start - 1u, nkeys = __ldg(&T->nkeys), deep = __ldg(&T->deep);
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < P.g.V; w += gridDim.x * blockDim.x) {
+        uint32_t ksize[CSM_TAIL_MAXKEYS];
+#pragma unroll
+        for (uint32_t k = 0; k < CSM_TAIL_MAXKEYS; k++) {
+            if (k >= nkeys) break;
+            ksize[k] = 0;
+            if (__ldg(&T->key_parent[k]) != c) continue;
+            const uint32_t rel = __ldg(&T->key_rel[k]);
+            const uint2 ms = list_of(P, rel, w, 900 + c);
+            if (ms.y) ksize[k] = key_entries(P, rel, w, ms.y, __ldg(&T->key_old[k]));
+        }
+        out[w] = tail_product(P, pl, ksize, deep);
+    }
+}
+
+// Table of a pendant plan (DevPlan.memo_slot): for every data vertex v, the count of its counting
+// level c for a prefix whose vertex at memo_depth is v — the sum of the tail values of v's list
+// under the flag rule and c's NLF filter.  A lane looks at one vertex (most have no list in the
+// relation); the warp then scans the lists found, 32 entries at a time.
+__global__ void k_pendant_counts(EnumParams P, const uint32_t *desc, unsigned long long *memo) {
     const uint32_t lane = threadIdx.x & 31u;
-    const DevPlan *pl = P.plans + plan;
+    const DevPlan *pl = P.plans + desc[3 * blockIdx.y];
+    unsigned long long *out = memo + (size_t)desc[3 * blockIdx.y + 1] * P.g.V;
+    const unsigned long long *value = memo + (size_t)desc[3 * blockIdx.y + 2] * P.g.V;
     const uint32_t c = pl->tail_start - 1u;
     const DevLevel *lv = &pl->lv[c];
     const uint32_t rel = __ldg(&lv->bn_rel[0]);
     const bool old = (__ldg(&lv->old_mask) & 1u) != 0;
     const uint32_t nlf_id = __ldg(&lv->nlf_bitmap);
     const uint32_t *nlf = nlf_id == CSM_NO_BITMAP ? nullptr : bitmap(P, nlf_id);
-    uint32_t scans = 0, probes = 0, tails = 0;
+    uint32_t scans = 0;
     const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < P.g.V; v += nw) {
-        const uint2 ms = list_of(P, rel, v, 900 + c);
-        unsigned long long acc = 0;
-        for (uint32_t base = 0; base < ms.y; base += 32) {
-            const uint32_t idx = base + lane;
-            if (idx >= ms.y) continue;
-            const uint32_t e = __ldg(P.g.pool + ms.x + idx);
-            const uint32_t w = e >> 1;
-            scans++;
-            bool ok = !(old && (e & 1u));
-            if (w >= P.g.V) {
-                record_bad(P, CSM_BAD_ENTRY, e, ms.x + idx, 900 + c);
-                ok = false;
+    for (uint32_t base = 32u * (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); base < P.g.V; base += 32u * nw) {
+        const uint32_t v = base + lane;
+        const uint2 ms = v < P.g.V ? list_of(P, rel, v, 900 + c) : make_uint2(0u, 0u);
+        unsigned long long mine = 0;
+        for (uint32_t todo = __ballot_sync(0xffffffffu, ms.y != 0); todo; todo &= todo - 1) {
+            const uint32_t l = __ffs(todo) - 1;
+            const uint32_t off = __shfl_sync(0xffffffffu, ms.x, l), size = __shfl_sync(0xffffffffu, ms.y, l);
+            unsigned long long acc = 0;
+            for (uint32_t i = lane; i < size; i += 32) {
+                const uint32_t e = __ldg(P.g.pool + off + i), w = e >> 1;
+                scans++;
+                bool ok = !(old && (e & 1u));
+                if (w >= P.g.V) {
+                    record_bad(P, CSM_BAD_ENTRY, e, off + i, 900 + c);
+                    ok = false;
+                }
+                if (ok && (!nlf || test_bit(nlf, w))) acc += value[w];
             }
-            if (ok && nlf) ok = test_bit(nlf, w);
-            if (ok) {
-                acc += tail_count_lane(nullptr, nullptr, P, pl, c, 0, w, 0, probes);
-                tails++;
-            }
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == l) mine = acc;
         }
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) out[v] = acc;
+        if (v < P.g.V) out[v] = mine;
     }
-    unsigned long long s64 = scans, p64 = probes, t64 = tails;
-    for (int o = 16; o > 0; o >>= 1) {
-        s64 += __shfl_xor_sync(0xffffffffu, s64, o);
-        p64 += __shfl_xor_sync(0xffffffffu, p64, o);
-        t64 += __shfl_xor_sync(0xffffffffu, t64, o);
-    }
-    if (lane == 0) {
-        if (s64) atomicAdd(&P.ctrl->scan_entries, s64);
-        if (p64) atomicAdd(&P.ctrl->probes, p64);
-        if (t64) atomicAdd(&P.ctrl->tail_lists, t64);
-    }
+    unsigned long long s64 = scans;
+    for (int o = 16; o > 0; o >>= 1) s64 += __shfl_xor_sync(0xffffffffu, s64, o);
+    if (lane == 0 && s64) atomicAdd(&P.ctrl->scan_entries, s64);
 }
 
 // Between two expansion launches.  The level just written becomes the source of the next launch,
@@ -1860,8 +1928,12 @@ void launch_expand_decide(const EnumParams &p, bool last, unsigned long long tar
     k_expand_decide<<<296, 256, 0, s>>>(p, last ? 1u : 0u, target);
 }
 
-void launch_pendant_counts(const EnumParams &p, uint32_t plan, unsigned long long *out, cudaStream_t s) {
-    k_pendant_counts<<<148 * 8, 256, 0, s>>>(p, plan, out);
+void launch_pendant_tables(const EnumParams &p, const uint32_t *desc, uint32_t ntables, unsigned long long *memo,
+                           cudaStream_t s) {
+    // Enough blocks for one pass over the vertices, at most eight per SM and table.
+    const uint32_t blocks = p.g.V / 256u + 1u < 148u * 8u ? p.g.V / 256u + 1u : 148u * 8u;
+    k_tail_values<<<dim3(blocks, ntables), 256, 0, s>>>(p, desc, memo);
+    k_pendant_counts<<<dim3(blocks, ntables), 256, 0, s>>>(p, desc, memo);
 }
 
 }  // namespace csm

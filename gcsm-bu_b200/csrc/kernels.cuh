@@ -145,7 +145,9 @@ void launch_phase_begin(EnumControl *ctrl, const uint32_t *ticket_prefix, uint32
 // whether that launch expands it further (not when `last`, empty, of `target` items or more, or when
 // the bound of the next level exceeds the frontier buffers).
 void launch_expand_decide(const EnumParams &p, bool last, unsigned long long target, cudaStream_t s);
-// Fills table `out` (one entry per data vertex) for the pendant plan `plan` in this phase.
-void launch_pendant_counts(const EnumParams &p, uint32_t plan, unsigned long long *out, cudaStream_t s);
+// Fills the pendant tables (one entry per data vertex) for this phase: `desc` names, for each of
+// `ntables`, a plan that reads it, its slot in `memo` and the slot of the tail values it sums.
+void launch_pendant_tables(const EnumParams &p, const uint32_t *desc, uint32_t ntables, unsigned long long *memo,
+                           cudaStream_t s);
 
 }  // namespace csm

@@ -500,6 +500,7 @@ void pack_plan(const Query &q, uint32_t i, uint16_t query_id, uint32_t nlf_base,
         if (pendant) {
             dp.memo_slot = CSM_MEMO_PENDING;
             dp.memo_depth = hp.bn[c][0];
+            dp.tail.deep = (uint8_t)((1u << tail.nclasses) - 1u);
             dp.expand_stop = (uint8_t)(c - 1);
         }
     }
@@ -649,6 +650,36 @@ bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, Ho
     g.dev.nlf1 = nlf_base + leaf;
     hp.dev = g.dev;
     hp.terms = g.terms;
+    return true;
+}
+
+bool extend_pendant(HostPlan &hp) {
+    DevPlan &dp = hp.dev;
+    const DevTail &t = dp.tail;
+    const int c = dp.tail_start - 1;
+    if (dp.memo_slot != CSM_NO_MEMO || dp.tail_start >= dp.n || !t.lane_par || c < 3 || dp.lv[c].nbn != 1) return false;
+    uint8_t deep = 0;
+    for (int cl = 0; cl < t.nclasses; cl++) {
+        bool below = false, above = false;
+        for (int i = t.class_term_begin[cl]; i < t.class_term_begin[cl + 1]; i++)
+            for (int j = 0; j < hp.terms[i].nf; j++) {
+                const int k = __builtin_ctz(t.mask[hp.terms[i].f[j]]);
+                if (t.key_parent[k] == c) {
+                    below = true;
+                    if (t.key_excl[k] & ((1u << c) - 1u)) return false;  // a prefix vertex could sit in the list
+                } else {
+                    above = true;
+                    if ((t.key_excl[k] >> c) & 1u) return false;  // c's vertex could sit in the list
+                }
+            }
+        if (below && above) return false;
+        if (below) deep |= (uint8_t)(1u << cl);
+    }
+    if (!deep) return false;
+    dp.tail.deep = deep;
+    dp.memo_slot = CSM_MEMO_PENDING;
+    dp.memo_depth = dp.lv[c].bn_depth[0];
+    dp.expand_stop = (uint8_t)(c - 1);
     return true;
 }
 

@@ -1,7 +1,8 @@
-// Host-only check of group_leaf_seeds (gcsm-bu_b200/csrc/plan.cpp): on random labelled queries and
-// random data graphs with some edges marked as batch edges, the plan that starts once per data vertex
-// of the inner endpoint counts what the plan that starts at every batch edge counts.  Both device
-// forms are evaluated by the same small interpreter (levels, flag rules, exclusions, tail polynomial).
+// Host-only check of group_leaf_seeds and extend_pendant (gcsm-bu_b200/csrc/plan.cpp): on random
+// labelled queries and random data graphs with some edges marked as batch edges, the plan that starts
+// once per data vertex of the inner endpoint, and the plan whose counting level is settled from
+// per-vertex sums, count what the plan that starts at every batch edge counts.  All device forms are
+// evaluated by the same small interpreter (levels, flag rules, exclusions, tail polynomial, tables).
 #include <algorithm>
 #include <cstdio>
 #include <map>
@@ -40,23 +41,27 @@ struct Graph {
 
 bool counts(int rule, bool batch) { return rule == CSM_KEY_ANY || batch == (rule == CSM_KEY_BATCH); }
 
-long long tail(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, const uint32_t *f) {
+// The tail classes in `classes` for the prefix f; `depths` of it are set.
+long long tail(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, const uint32_t *f,
+               unsigned classes, int depths) {
     const DevTail &t = p.tail;
     std::vector<long long> size(t.nmasks, 0);
     for (int mi = 0; mi < t.nmasks; mi++)
         for (uint32_t w = 0; w < g.n; w++) {
+            if (t.key_parent[__builtin_ctz(t.mask[mi])] >= depths) continue;  // of a class not asked for
             bool ok = true;
             for (int k = 0; ok && k < t.nkeys; k++) {
                 if (!((t.mask[mi] >> k) & 1u)) continue;
                 const int e = g.entry(t.key_rel[k], f[t.key_parent[k]], w);
                 ok = e && counts(t.key_old[k], e == 2);
-                for (int j = 0; ok && j < p.tail_start; j++)
+                for (int j = 0; ok && j < depths; j++)
                     if (((t.key_excl[k] >> j) & 1u) && f[j] == w) ok = false;
             }
             size[mi] += ok;
         }
     long long total = 1;
     for (int c = 0; c < t.nclasses; c++) {
+        if (!((classes >> c) & 1u)) continue;
         long long s = 0;
         for (int i = t.class_term_begin[c]; i < t.class_term_begin[c + 1]; i++) {
             long long prod = terms[i].coef;
@@ -68,9 +73,35 @@ long long tail(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> 
     return total;
 }
 
+// What hangs off vertex w at the counting level alone: a table entry of its own.
+long long tail_value(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, uint32_t w) {
+    uint32_t f[CSM_MAXQV];
+    std::fill(f, f + CSM_MAXQV, 0xFFFFFFFFu);  // no prefix
+    f[p.tail_start - 1] = w;
+    return tail(g, p, terms, f, p.tail.deep, p.tail_start);
+}
+
+// A pendant counting level below the prefix f[0..c-1]: the sum over its list, without exclusions, less
+// the prefix vertices that the sum should not hold, times what hangs off the prefix.
+long long settle(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, const uint32_t *f) {
+    const int c = p.tail_start - 1, md = p.memo_depth;
+    const DevLevel &lv = p.lv[c];
+    const bool old = lv.old_mask & 1u;
+    long long sum = 0;
+    for (const Entry &e : g.list(lv.bn_rel[0], f[md]))
+        if (!(old && e.batch)) sum += tail_value(g, p, terms, e.v);
+    for (int j = 0; j < c; j++) {
+        if (!((lv.excl_mask >> j) & 1u) || j == md) continue;
+        const int x = g.entry(lv.bn_rel[0], f[md], f[j]);
+        if (x && !(old && x == 2)) sum -= tail_value(g, p, terms, f[j]);
+    }
+    return sum * tail(g, p, terms, f, ~(unsigned)p.tail.deep, c);
+}
+
 long long walk(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, uint32_t *f, int d) {
     if (d == p.n) return 1;
-    if (d == p.tail_start) return tail(g, p, terms, f);
+    if (p.memo_slot == CSM_MEMO_PENDING && d + 1 == p.tail_start) return settle(g, p, terms, f);
+    if (d == p.tail_start) return tail(g, p, terms, f, ~0u, d);
     const DevLevel &lv = p.lv[d];
     long long total = 0;
     for (const Entry &e : g.list(lv.bn_rel[0], f[lv.bn_depth[0]])) {
@@ -112,9 +143,9 @@ long long count(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm>
 
 int main() {
     std::mt19937 rng(77);
-    int grouped[3] = {0, 0, 0}, nonzero = 0;
-    for (int qn = 0; qn < 300; qn++) {
-        const uint32_t nv = 2 + rng() % 5, nlab = 1 + rng() % 3;
+    int grouped[3] = {0, 0, 0}, nonzero = 0, pendant = 0;
+    for (int qn = 0; qn < 600; qn++) {
+        const uint32_t nv = 2 + rng() % 6, nlab = 1 + rng() % 4;
         std::vector<uint32_t> vl(nv), src, dst, el;
         for (auto &x : vl) x = rng() % nlab;
         std::set<std::pair<uint32_t, uint32_t>> seen;
@@ -145,7 +176,7 @@ int main() {
         std::vector<HostPlan> plans = build_plans(q, 0, 0, st, po, rel_of);
         // A data graph of the query's labels; two labelled edges of one pair are two edges.
         Graph g;
-        g.n = 9;
+        g.n = 14;
         std::vector<uint32_t> gl(g.n);
         for (auto &x : gl) x = rng() % nlab;
         for (uint32_t a = 0; a < g.n; a++)
@@ -170,14 +201,26 @@ int main() {
             }
             const long long got = count(g, hp.dev, hp.terms);
             nonzero += did && want > 0;
+            for (HostPlan ep : {plans[i], hp}) {
+                if (!extend_pendant(ep)) continue;
+                const long long settled = count(g, ep.dev, ep.terms);
+                pendant += want > 0;
+                if (settled != want) {
+                    std::printf("FAIL query %d plan %zu: %lld settled, %lld counted\n", qn, i, settled, want);
+                    return 1;
+                }
+            }
             if (got != want) {
                 std::printf("FAIL query %d plan %zu: %lld per inner vertex, %lld per batch edge\n", qn, i, got, want);
                 return 1;
             }
         }
     }
-    if (grouped[CSM_SEED_WEIGHT] < 50 || grouped[CSM_SEED_TAIL] < 50 || nonzero < 100)
-        return std::printf("too few grouped plans: %d %d, %d with matches\n", grouped[1], grouped[2], nonzero), 1;
-    std::printf("ok %d weighted, %d in the tail, %d with matches\n", grouped[1], grouped[2], nonzero);
+    if (grouped[CSM_SEED_WEIGHT] < 50 || grouped[CSM_SEED_TAIL] < 50 || nonzero < 100 ||
+        pendant < 20)
+        return std::printf("too few plans: %d weighted, %d in the tail, %d of them with matches, %d pendant\n", grouped[1],
+                           grouped[2], nonzero, pendant), 1;
+    std::printf("ok %d weighted, %d in the tail, %d of them with matches, %d pendant\n", grouped[1], grouped[2], nonzero,
+                pendant);
     return 0;
 }

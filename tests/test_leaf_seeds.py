@@ -1,6 +1,7 @@
-"""Plans of query edges that end in a leaf start once per data vertex of the inner endpoint: the
-rewritten plans against the ones they stand for (CPU, native), and the engine against the oracle on
-a graph whose hubs own many batch edges each."""
+"""Plans rewritten after the planner — query edges that end in a leaf start once per data vertex of the
+inner endpoint, and counting levels are settled from per-vertex sums although prefix vertices share
+their label: the rewritten plans against the ones they stand for (CPU, native), and the engine
+against the oracle on a graph whose hubs own many batch edges each."""
 import os
 import shutil
 import subprocess
@@ -17,7 +18,7 @@ CSRC = os.path.join(ROOT, "gcsm-bu_b200", "csrc")
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="no C++ compiler")
-def test_grouped_plans_count_what_the_edge_plans_count(tmp_path):
+def test_rewritten_plans_count_what_the_edge_plans_count(tmp_path):
     exe = str(tmp_path / "leaf_group_test")
     subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-o", exe,
                     os.path.join(ROOT, "tests", "native", "leaf_group_test.cpp"), os.path.join(CSRC, "plan.cpp"),
@@ -42,16 +43,19 @@ QUERIES = [
     query([2, 2, 0, 1, 0, 2], PATH6),               # a leaf in the tail next to another
     query([0, 1, 1, 1], STAR),                      # the counting level is the seed level
     query([0, 1, 2], [(0, 1), (1, 2)]),
+    query([2, 2, 0, 1, 0, 3], PATH6),               # settled below vertices of the level's label
+    query([1, 0, 1, 0, 3, 2], [(0, 1), (1, 2), (2, 3), (3, 4), (1, 5)]),  # and above another tail class
+    query([1, 2, 0, 3, 1], [(0, 1), (1, 2), (2, 3), (3, 0), (2, 4)]),     # two pair intersections
 ]
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("strategy", [0, 1, 2, 3])
-def test_grouped_plans_equal_the_oracle(strategy):
+def test_rewritten_plans_equal_the_oracle(strategy):
     rng = np.random.default_rng(23)
     n = 400
     s, d = gen.chung_lu(n, 2400, 2.0, rng)          # uncapped: hubs with many batch edges
-    vl = rng.integers(0, 3, size=n).astype(np.uint32)
+    vl = rng.integers(0, 4, size=n).astype(np.uint32)
     el = np.zeros(len(s), dtype=np.uint32)
     data, batches = gen.make_stream(n, s, d, el, rng, n_ins=240, n_del=240, batch=160)
     data = DataGraph(vl, data.src, data.dst, data.elabels)
@@ -60,6 +64,7 @@ def test_grouped_plans_equal_the_oracle(strategy):
             eng.load_query(q)
         eng.load_graph(data)
         text = [eng.describe(i) for i in range(len(QUERIES))]
+        assert "pendant counting level" in text[6] and "pendant counting level" in text[7]
         assert any("counted per inner vertex" in t for t in text) and any("counted in the tail" in t for t in text)
         oracles = [Oracle(q, data) for q in QUERIES]
         seen = 0

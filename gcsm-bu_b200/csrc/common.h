@@ -48,6 +48,10 @@
 #define CSM_PAIR_SIGS 4095        // signatures fit 12 bits of a table entry's tag, the phase 20
 #define CSM_PAIR_PHASES 0xFFFFFu
 #define CSM_PAIR_MAXMASKS 8       // most masks of a pair_par tail
+#define CSM_NO_SET 0xFFFFu
+#define CSM_SET(slot, a, b, c) ((uint16_t)((slot) | (a) << 3 | (b) << 6 | (c) << 9))  // a, b: the kept keys
+#define CSM_SETS 4                // most sets of a tail
+#define CSM_SET_CAP 256           // entries of a set kept at once (longer ones are counted in pieces)
 
 // One matching-order level (one query vertex) of a plan.
 struct DevLevel {
@@ -91,7 +95,7 @@ struct DevTail {
     uint8_t nmasks;                             // key subsets whose intersection size is used
     uint8_t nclasses;
     uint8_t lane_par;                           // every mask is one key: count 32 prefixes per warp step
-    uint8_t pair_par;                           // every mask is one key or a pair with a memo signature: same
+    uint8_t pair_par;                           // every mask is one key, a pair or a set: same
     uint8_t single;                             // keys that are a mask by themselves
     uint8_t deep;                               // pendant plans: classes whose keys hang off depth c
     uint16_t mask[CSM_TAIL_MAXMASKS];
@@ -99,6 +103,10 @@ struct DevTail {
     // The size of the intersection is a function of it and the two data vertices, kept per phase in a
     // table that all warps share.  Bit 15: the keys stand the other way round in the signature.
     uint16_t mask_pair[CSM_TAIL_MAXMASKS];
+    // A mask of three keys in a pair_par tail: CSM_SET of them, CSM_NO_SET for every other.  Two keys
+    // hang off vertices above the counting level: their intersection is the same for all candidates
+    // of that level and is kept while they are counted.
+    uint16_t mask_set[CSM_TAIL_MAXMASKS];
     uint16_t class_term_begin[CSM_TAIL_MAXCLASSES + 1];  // into the plan's term list
 };
 

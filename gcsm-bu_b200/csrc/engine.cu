@@ -174,7 +174,7 @@ Engine::~Engine() {
                    g_.vlab, d_plans_, d_terms_, d_upd_src_, d_upd_dst_, d_upd_lab_, d_upd_del_, d_keys_raw_, d_keys_,
                    d_sort_temp_, bs_.eff, bs_.heads, bs_.nheads, bs_.seg_nins, bs_.seg_ndel, bs_.seg_end, bs_.scr_y,
                    bs_.scr_lb, bs_.counters, bs_.error, d_ctrl_, d_queue_, d_seq_, d_seed_lo_, d_ticket_prefix_,
-                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_, d_memo_desc_, d_pairs_, d_pair_phase_};
+                   d_counts_, d_frontier_[0], d_frontier_[1], d_rows_, d_rel_delta_, d_touched_, d_memo_, d_memo_desc_, d_pairs_, d_pair_phase_, d_sets_};
     for (void *p : dev)
         if (p) cudaFree(p);
     if (h_pin_) cudaFreeHost(h_pin_);
@@ -629,9 +629,20 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
     bool used = false;
     for (HostPlan &hp : plans) {
         DevTail &t = hp.dev.tail;
-        bool all = hp.dev.tail_start < hp.dev.n && hp.dev.tail_start >= 3 && t.nmasks <= CSM_PAIR_MAXMASKS && !t.lane_par;
+        const int level = hp.dev.tail_start - 1;  // the counting level
+        bool all = hp.dev.tail_start < hp.dev.n && level >= 2 && t.nmasks <= CSM_PAIR_MAXMASKS && !t.lane_par;
+        int sets = 0;
         for (int m = 0; m < t.nmasks; m++) {
             const int bits = __builtin_popcount(t.mask[m]);
+            if (bits == 3) {
+                int k[3], n = 0;
+                for (int x = 0; x < t.nkeys; x++)
+                    if ((t.mask[m] >> x) & 1u) k[n++] = x;
+                std::sort(k, k + 3, [&](int x, int y) { return t.key_parent[x] < t.key_parent[y]; });
+                if (t.key_parent[k[1]] >= level || sets == CSM_SETS) all = false;
+                else t.mask_set[m] = CSM_SET(sets++, k[0], k[1], k[2]);
+                continue;
+            }
             if (bits != 2) {
                 all = all && bits == 1;
                 continue;
@@ -651,11 +662,15 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
         t.pair_par = all ? 1 : 0;
         used = used || all;
     }
+    // One kept-set area per warp: no launch has more than 64 warps on an SM.
+    const size_t set_entries = (size_t)sm_count_ * 64 * CSM_SETS * CSM_SET_CAP;
     if (used && !d_pairs_) {
         size_t free_b = 0, total_b = 0;
-        const size_t want = sizeof(uint4) * (size_t)kPairSlots;
+        const size_t want = sizeof(uint4) * (size_t)kPairSlots + sizeof(uint32_t) * set_entries;
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 4 &&
-            dev_alloc(&d_pair_phase_, 1) == cudaSuccess && dev_alloc(&d_pairs_, kPairSlots) == cudaSuccess) {
+            (d_sets_ || dev_alloc(&d_sets_, set_entries) == cudaSuccess) &&
+            (d_pair_phase_ || dev_alloc(&d_pair_phase_, 1) == cudaSuccess) &&
+            dev_alloc(&d_pairs_, kPairSlots) == cudaSuccess) {
             pair_slots_ = kPairSlots;
             pair_phases_ = CSM_PAIR_PHASES;  // cleared before the first batch
         } else {
@@ -1308,6 +1323,7 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
                        s);
     P.pairs = d_pairs_;
     P.pair_slots = pair_slots_;
+    P.sets = d_sets_;
     stats_.kernel_launches++;
     for (int b = 0; b < 2; b++) P.frontier[b] = expand ? d_frontier_[b] : nullptr;
     P.frontier_cap = expand ? frontier_cap_ : 0;

@@ -285,6 +285,7 @@ class Engine {
     uint4 *d_pairs_ = nullptr;                // pair table, null when no plan uses it
     unsigned int *d_pair_phase_ = nullptr;    // phases it has seen, counted on the device
     uint32_t pair_slots_ = 0;
+    uint32_t *d_sets_ = nullptr;              // kept intersections, CSM_SETS per warp of the largest grid
     uint64_t pair_phases_ = 0;                // the same, an upper bound kept by the host
     int expand_levels_ = 0;                   // most breadth-first levels any plan expands
     LaunchConfig lc_{};                       // configuration in use

@@ -72,7 +72,12 @@ struct __align__(16) WarpState {
     // f[0..n-3], and whether it is being counted (1) or known (2).
     unsigned long long sl_count;
     uint32_t sl_state;
+    // Kept intersections of the counting level (DevTail.mask_set): entries held, or kSetOpen while
+    // there is none for the current prefix.
+    uint32_t set_n[CSM_SETS];
 };
+
+constexpr uint32_t kSetOpen = 0xFFFFFFFFu;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
@@ -272,7 +277,12 @@ __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uin
 // chunk spans, which starts where the last chunk ended and is doubled until it holds the chunk's
 // largest entry.  The window is a power of two and reads past the end count as large, so the search
 // has no data-dependent branch: log2(window) dependent reads, most of them from a few cache lines.
-__device__ uint32_t intersect_lists(const EnumParams &P, uint2 a, uint32_t rule_a, uint2 b, uint32_t rule_b) {
+// KEEP: the vertices found, without the prefix vertices f[j] with bit j of `excl`, go to `out`, and
+// the scan starts at entry `from` of the shorter list and stops (returning where in `from`) before a
+// chunk that might not fit in CSM_SET_CAP entries.
+template <bool KEEP>
+__device__ uint32_t intersect_lists(const EnumParams &P, uint2 a, uint32_t rule_a, uint2 b, uint32_t rule_b,
+                                    const uint32_t *f, uint32_t excl, uint32_t *out, uint32_t &from) {
     const uint32_t lane = lane_id();
     if (b.y < a.y) {
         const uint2 t = a;
@@ -286,8 +296,9 @@ __device__ uint32_t intersect_lists(const EnumParams &P, uint2 a, uint32_t rule_
     // First window: twice what a chunk spans on average.
     const uint32_t per = a.y ? b.y / a.y : 0u;
     const uint32_t w0 = 64u << (per ? 31 - __clz(per) : 0);
-    uint32_t cnt = 0, c0 = 0;
-    for (uint32_t base = 0; base < a.y && c0 < b.y; base += 32) {
+    uint32_t cnt = 0, c0 = 0, base = KEEP ? from : 0u;
+    for (; base < a.y && c0 < b.y; base += 32) {
+        if (KEEP && cnt > CSM_SET_CAP - 32u) break;
         const uint32_t i = base + lane;
         const uint32_t e = i < a.y ? __ldg(A + i) : 0xFFFFFFFFu;
         const uint32_t key = e & ~1u;
@@ -302,9 +313,17 @@ __device__ uint32_t intersect_lists(const EnumParams &P, uint2 a, uint32_t rule_
             if (v < key) pos += s;
         }
         const uint32_t g = pos < b.y ? __ldg(B + pos) : 0xFFFFFFFFu;
-        const bool hit = i < a.y && (g & ~1u) == key && g != 0xFFFFFFFFu && key_counts(rule_a, e) && key_counts(rule_b, g);
-        cnt += __popc(__ballot_sync(0xffffffffu, hit));
+        bool hit = i < a.y && (g & ~1u) == key && g != 0xFFFFFFFFu && key_counts(rule_a, e) && key_counts(rule_b, g);
+        if (KEEP)
+            for (uint32_t em = excl; hit && em; em &= em - 1) hit = f[__ffs(em) - 1] != (e >> 1);
+        const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+        if (KEEP && hit) out[cnt + __popc(hits & ((1u << lane) - 1u))] = e >> 1;
+        cnt += __popc(hits);
         c0 = __shfl_sync(0xffffffffu, pos, last);
+    }
+    if (KEEP) {
+        from = c0 < b.y ? base : a.y;
+        __syncwarp();
     }
     return cnt;
 }
@@ -369,7 +388,9 @@ __device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const Dev
     for (uint32_t need = __ballot_sync(0xffffffffu, miss); need;) {
         const uint32_t l = __ffs(need) - 1;
         const uint32_t va = __shfl_sync(0xffffffffu, a, l), vb = __shfl_sync(0xffffffffu, b, l);
-        const uint32_t c = intersect_lists(P, list_of(P, ra, va, 1000 + d), rule_a, list_of(P, rb, vb, 1000 + d), rule_b);
+        uint32_t from = 0;
+        const uint32_t c = intersect_lists<false>(P, list_of(P, ra, va, 1000 + d), rule_a, list_of(P, rb, vb, 1000 + d), rule_b,
+                                                  nullptr, 0u, nullptr, from);
         const bool same = miss && a == va && b == vb;
         if (same) count = c;
         if (lane == l) store_pair(slot, ta, tb, tag, c);
@@ -389,11 +410,71 @@ __device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const Dev
     return count;
 }
 
+// Size of the three-key mask mi for this lane's prefix f[0..d-1] + cand (where ok).  The intersection
+// of the two keys above the counting level is the same for all of the level's candidates: it is made
+// once and kept (a few dozen vertices as a rule), and the warp then looks up all (candidate, kept
+// vertex) pairs of the chunk, 32 at a time, in the candidates' lists of the third key.
+__device__ uint32_t set_size(WarpState &S, const EnumParams &P, const DevTail *T, uint32_t mi, uint32_t d, bool ok,
+                             uint32_t cand) {
+    const uint32_t lane = lane_id();
+    const uint32_t set = __ldg(&T->mask_set[mi]);
+    const uint32_t slot = set & 7u, ka = (set >> 3) & 7u, kb = (set >> 6) & 7u, kc = (set >> 9) & 7u;
+    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    uint32_t *kept = P.sets + ((size_t)warp * CSM_SETS + slot) * CSM_SET_CAP;
+    const uint32_t pc = __ldg(&T->key_parent[kc]), rule_c = __ldg(&T->key_old[kc]);
+    uint2 list = make_uint2(0u, 0u);
+    if (ok) list = list_of(P, __ldg(&T->key_rel[kc]), pc == d ? cand : S.f[pc], 1200 + d);
+    const uint32_t excl = __ldg(&T->key_excl[kc]);
+    const uint32_t oks = __ballot_sync(0xffffffffu, ok);
+    const uint32_t nok = __popc(oks), rank = __popc(oks & ((1u << lane) - 1u));
+    __syncwarp();
+    if (ok) S.buf[d][rank] = lane;  // the level's buffer is not in use: its candidates are counted here
+    __syncwarp();
+    uint32_t count = 0, from = 0, n = S.set_n[slot];
+    bool more = true;
+    while (more) {
+        if (n == kSetOpen) {
+            const uint2 a = list_of(P, __ldg(&T->key_rel[ka]), S.f[__ldg(&T->key_parent[ka])], 1200 + d);
+            const uint2 b = list_of(P, __ldg(&T->key_rel[kb]), S.f[__ldg(&T->key_parent[kb])], 1200 + d);
+            const uint32_t start = from;
+            n = intersect_lists<true>(P, a, __ldg(&T->key_old[ka]), b, __ldg(&T->key_old[kb]), S.f,
+                                      excl & ((1u << d) - 1u), kept, from);
+            more = from < (a.y < b.y ? a.y : b.y);
+            if (lane == 0 && start == 0 && !more) S.set_n[slot] = n;  // all of it
+        } else {
+            more = false;
+        }
+        const uint32_t total = n * nok;
+        for (uint32_t g0 = 0; g0 < total; g0 += 32) {
+            const uint32_t g = g0 + lane, r = n ? g / n : 0u;
+            const bool in = g < total;
+            const uint32_t src = in ? S.buf[d][r] : 0u;
+            const uint32_t off = __shfl_sync(0xffffffffu, list.x, src), size = __shfl_sync(0xffffffffu, list.y, src);
+            const uint32_t c = __shfl_sync(0xffffffffu, cand, src);
+            bool hit = false;
+            if (in) {
+                const uint32_t w = kept[g - r * n];
+                const uint32_t e = find_entry(P.g.pool + off, size, w);
+                hit = e != 0xFFFFFFFFu && key_counts(rule_c, e) && !(((excl >> d) & 1u) && w == c);
+            }
+            const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+            // This lane's candidate has positions [rank * n, rank * n + n) of the pairs.
+            const uint32_t s0 = rank * n, s1 = s0 + n;
+            const uint32_t lo = s0 > g0 ? s0 - g0 : 0u, hi = s1 > g0 ? s1 - g0 : 0u;
+            if (ok && lo < 32u && hi > lo)
+                count += __popc(hits & (0xFFFFFFFFu << lo) & (hi >= 32u ? 0xFFFFFFFFu : (1u << hi) - 1u));
+        }
+        if (more) n = kSetOpen;
+    }
+    __syncwarp();
+    return count;
+}
+
 // Lane-parallel tail with pair masks (DevTail.pair_par), counting level d >= 2: the tail count of the
 // prefix f[0..d-1] + cand for every lane with ok set (0 for the others).  A pair of data vertices
 // recurs under many prefixes — the lists of two vertices intersect the same whatever was matched
 // between them — so most sizes are one table read instead of a scan of two lists.
-__device__ unsigned long long tail_count_pairs(const WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t d,
+__device__ unsigned long long tail_count_pairs(WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t d,
                                                bool ok, uint32_t cand, uint32_t shared_hit, uint32_t &probes) {
     const DevTail *T = &pl->tail;
     const uint32_t nmasks = __ldg(&T->nmasks);
@@ -403,6 +484,8 @@ __device__ unsigned long long tail_count_pairs(const WarpState &S, const EnumPar
         if (mi >= nmasks) break;
         if (__ldg(&T->mask_pair[mi]) != CSM_NO_PAIR) {
             msize[mi] = pair_size(S, P, T, mi, d, ok, cand);
+        } else if (__ldg(&T->mask_set[mi]) != CSM_NO_SET) {
+            msize[mi] = set_size(S, P, T, mi, d, ok, cand);
         } else {
             msize[mi] = 0;
             if (ok)
@@ -468,6 +551,7 @@ __device__ void enter_level(WarpState &S, const EnumParams &P, const DevPlan *pl
         S.nlf[d] = __ldg(&lv->nlf_bitmap);
         S.exm[d] = __ldg(&lv->excl_mask);
     }
+    if (lane < CSM_SETS && d + 1 == pl->tail_start) S.set_n[lane] = kSetOpen;
     __syncwarp();
     if (d + 1 == pl->tail_start && pl->tail_start < pl->n && (pl->tail.lane_par || pl->tail.pair_par))
         prep_tail_shared(S, P, pl, d);

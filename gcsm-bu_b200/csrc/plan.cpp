@@ -429,7 +429,10 @@ bool build_tail(const Query &q, const HostPlan &hp, int qe, const RelOf &rel_of,
         if (__builtin_popcount(masks[k]) != 1) tail.lane_par = 0;
         else tail.single |= (uint8_t)masks[k];
     }
-    for (size_t k = 0; k < CSM_TAIL_MAXMASKS; k++) tail.mask_pair[k] = CSM_NO_PAIR;
+    for (size_t k = 0; k < CSM_TAIL_MAXMASKS; k++) {
+        tail.mask_pair[k] = CSM_NO_PAIR;
+        tail.mask_set[k] = CSM_NO_SET;
+    }
     return true;
 }
 

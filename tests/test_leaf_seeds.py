@@ -46,6 +46,8 @@ QUERIES = [
     query([2, 2, 0, 1, 0, 3], PATH6),               # settled below vertices of the level's label
     query([1, 0, 1, 0, 3, 2], [(0, 1), (1, 2), (2, 3), (3, 4), (1, 5)]),  # and above another tail class
     query([1, 2, 0, 3, 1], [(0, 1), (1, 2), (2, 3), (3, 0), (2, 4)]),     # two pair intersections
+    query([0, 1, 2, 3, 0], [(0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (2, 3), (0, 4)]),  # three lists of one vertex
+    query([0, 1, 0, 1, 1], [(0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (2, 3), (0, 4)]),  # of the prefix's labels
 ]
 
 

@@ -722,10 +722,15 @@ __device__ bool item_ok(const WarpState &S, const EnumParams &P, uint32_t where,
     return ok;
 }
 
-// Whether some warp waits at the ring for an item.  One 8-byte read of both ring counters.
-__device__ __forceinline__ bool items_wanted(const EnumParams &P) {
-    const unsigned long long w = *(volatile unsigned long long *)&P.ctrl->q_head;
-    return (int32_t)((uint32_t)(w >> 32) - (uint32_t)w) > 0;
+// Warps that wait at the ring for an item (for every lane).  One 8-byte read of both ring counters.
+__device__ __forceinline__ uint32_t items_wanted(const EnumParams &P) {
+    int32_t n = 0;
+    if (lane_id() == 0) {
+        const unsigned long long w = *(volatile unsigned long long *)&P.ctrl->q_head;
+        n = (int32_t)((uint32_t)(w >> 32) - (uint32_t)w);
+    }
+    n = __shfl_sync(0xffffffffu, n, 0);
+    return n > 0 ? (uint32_t)n : 0u;
 }
 
 // Reserves `cnt` (1..32) consecutive ring positions while a warp waits for one; returns the first,
@@ -768,28 +773,32 @@ __device__ __forceinline__ uint2 seed_pair(const EnumParams &P, const DevPlan *p
     return make_uint2(P.kl.src(key), pl->seed_group == CSM_SEED_EDGE ? P.kl.dst(key) : __ldg(P.seg_flagged + c));
 }
 
-// Writes the item of ring position `pos` and publishes it with stamp (epoch, pos + 1).
-__device__ void publish_item(const EnumParams &P, uint32_t pos, uint32_t plan, uint32_t depth, uint32_t lo,
-                             uint32_t hi, const uint32_t *prefix, uint32_t nprefix, bool extra, uint32_t extra_v,
-                             uint32_t extra_pos) {
+// Writes and publishes `cnt` (at most 32) items from ring position `pos` on, one per lane: lane i's
+// item has the range [lo, hi) and the prefix f[0..nf-1], followed by `next` where the depth is nf + 1,
+// or the seed `next`, `next2` where nf is 0 and the depth 2.
+__device__ void publish_items(const EnumParams &P, uint32_t pos, uint32_t cnt, uint32_t plan, uint32_t depth,
+                              const uint32_t *f, uint32_t nf, uint32_t lo, uint32_t hi, uint32_t next, uint32_t next2) {
     const uint32_t lane = lane_id();
-    WorkItem *it = P.queue + (pos & P.qmask);
-    if (lane == 0) {
+    const uint32_t slot = (pos + lane) & P.qmask;
+    if (lane < cnt) {
+        WorkItem *it = P.queue + slot;
         it->plan = plan;
         it->depth = depth;
         it->lo = lo;
         it->hi = hi;
+        for (uint32_t k = 0; k < nf; k++) it->f[k] = f[k];
+        if (depth > nf) it->f[nf] = next;
+        if (depth > nf + 1) it->f[nf + 1] = next2;
     }
-    if (lane < nprefix) it->f[lane] = prefix[lane];
-    if (extra && lane == 0) it->f[extra_pos] = extra_v;
     __threadfence();
-    __syncwarp();
-    if (lane == 0) atomicExch(P.seq + (pos & P.qmask), slot_stamp(P.ctrl->epoch, pos + 1));
+    if (lane < cnt) atomicExch(P.seq + slot, slot_stamp(P.ctrl->epoch, pos + lane + 1));
     __syncwarp();
 }
 
-// Splits pending work of the current item into the queue.  Returns true if it donated.
-__device__ bool try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t L0, uint32_t d) {
+// Splits pending work of the current item into the queue, as many pieces as warps wait for (at most
+// 31 at a time), from the shallowest level that has some.
+__device__ void try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t L0, uint32_t d,
+                           uint32_t waiting) {
     const uint32_t lane = lane_id();
     const uint32_t E = pl->tail_start;
     // A shared last level is counted once per prefix at depth n - 3: the two deepest levels of
@@ -805,44 +814,43 @@ __device__ bool try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl,
         const uint32_t lo = S.lo[l], hi = S.hi[l];
         const uint32_t minr = (l == 1) ? 64u : P.steal_min;
         if (hi > lo && hi - lo >= minr) {
-            uint32_t mid = lo + ((hi - lo) >> 1);
-            if (l == 1) mid = (mid + 31u) & ~31u;
-            if (mid >= hi) continue;
-            const uint32_t slot = reserve_slots(P, 1);
-            if (slot == 0xFFFFFFFFu) return false;
-            publish_item(P, slot, S.item_plan, l == 1 ? 0u : l, mid, hi, S.f, l == 1 ? 0u : l, false, 0, 0);
+            // Equal parts of at least minr / 2 candidates (whole chunks of seeds); the first stays.
+            uint32_t cnt = 2u * (hi - lo) / minr - 1u;
+            cnt = cnt < waiting ? cnt : waiting;
+            cnt = cnt < 31u ? cnt : 31u;
+            uint32_t part = (hi - lo + cnt) / (cnt + 1u);
+            if (l == 1) part = (part + 31u) & ~31u;
+            cnt = (hi - lo - 1u) / part;
+            if (cnt == 0) continue;
+            const uint32_t slot = reserve_slots(P, cnt);
+            if (slot == 0xFFFFFFFFu) return;
+            const uint32_t a = lo + (lane + 1u) * part, b = hi - a < part ? hi : a + part;
+            publish_items(P, slot, cnt, S.item_plan, l == 1 ? 0u : l, S.f, l == 1 ? 0u : l, a, b, 0, 0);
             if (lane == 0) {
-                S.hi[l] = mid;
-                atomicAdd(&P.ctrl->donations, 1ull);
+                S.hi[l] = lo + part;
+                atomicAdd(&P.ctrl->donations, (unsigned long long)cnt);
             }
             __syncwarp();
-            return true;
+            return;
         }
         // Buffered siblings; of the current level's own buffer the next one stays.
         const uint32_t nb = S.nbuf[l], ps = S.pos[l] + (l == d ? 1u : 0u);
         if (l + 1 < sib_end && nb > ps) {
             const uint32_t cnt = nb - ps;
             const uint32_t slot = reserve_slots(P, cnt);
-            if (slot == 0xFFFFFFFFu) return false;
-            for (uint32_t j = 0; j < cnt; j++) {
-                const uint32_t c = S.buf[l][ps + j];
-                if (l == 1) {
-                    const uint2 seed = seed_pair(P, pl, c);
-                    uint32_t pre[2] = {seed.x, seed.y};
-                    publish_item(P, slot + j, S.item_plan, 2, 0, 0xFFFFFFFFu, pre, 2, false, 0, 0);
-                } else {
-                    publish_item(P, slot + j, S.item_plan, l + 1, 0, 0xFFFFFFFFu, S.f, l, true, c, l);
-                }
-            }
+            if (slot == 0xFFFFFFFFu) return;
+            uint2 next = make_uint2(0u, 0u);
+            if (lane < cnt) next.x = S.buf[l][ps + lane];
+            if (lane < cnt && l == 1) next = seed_pair(P, pl, next.x);
+            publish_items(P, slot, cnt, S.item_plan, l + 1, S.f, l == 1 ? 0u : l, 0, 0xFFFFFFFFu, next.x, next.y);
             if (lane == 0) {
                 S.nbuf[l] = (uint8_t)ps;
                 atomicAdd(&P.ctrl->donations, (unsigned long long)cnt);
             }
             __syncwarp();
-            return true;
+            return;
         }
     }
-    return false;
 }
 
 // Ends the launch for every waiting warp (the caller found that nothing holds work any more): the
@@ -1184,16 +1192,15 @@ __device__ unsigned long long count_last_level(WarpState &S, const EnumParams &P
                 }
             }
             if (P.donate) {
-                unsigned int wanted = 0;
-                if (lane == 0) wanted = items_wanted(P);
-                if (__shfl_sync(0xffffffffu, wanted, 0)) {
+                const uint32_t waiting = items_wanted(P);
+                if (waiting) {
                     // The remaining range [lo + 32, hi) is this level's pending work.
                     if (lane == 0) {
                         S.lo[d] = lo + 32;
                         S.hi[d] = hi;
                     }
                     __syncwarp();
-                    try_donate(S, P, pl, L0, d);
+                    try_donate(S, P, pl, L0, d, waiting);
                     hi = S.hi[d];
                     __syncwarp();
                 }
@@ -1381,9 +1388,8 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
         }
         if (P.donate && (iter & 7u) == 0) {
             // While a warp waits for work, split off one piece of this warp's pending work.
-            unsigned int wanted = 0;
-            if (lane == 0) wanted = items_wanted(P);
-            if (__shfl_sync(0xffffffffu, wanted, 0)) try_donate(S, P, pl, L0, d);
+            const uint32_t waiting = items_wanted(P);
+            if (waiting) try_donate(S, P, pl, L0, d, waiting);
         }
         if (S.pos[d] < S.nbuf[d]) {
             if (MODE == CSM_ENUM_MODE_COUNT && d + 2 == E && P.memo != nullptr && pl->memo_slot < CSM_MEMO_PENDING) {
@@ -1441,6 +1447,8 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 d++;
                 if (lane == 0 && d + 2 == n) S.sl_state = 0;  // a new prefix f[0..n-3]
                 enter_level(S, P, pl, d, 0, 0xFFFFFFFFu);
+                // A chunk of a counting level with list intersections is a long step: look before it.
+                if (PAIRS && d + 1 == E && pl->tail.pair_par && S.hi[d] >= 64u) iter |= 7u;
             }
             continue;
         }
@@ -1916,8 +1924,8 @@ __global__ void k_expand_decide(EnumParams P, uint32_t last, unsigned long long 
             const WorkItem *it = P.frontier[out] + i;
             const DevPlan *pl = P.plans + it->plan;
             const uint32_t d = it->depth;
-            if (d >= pl->expand_stop) {
-                if (lane == 0) acc += 1;  // passes through unchanged
+            if (d == 0 || d >= pl->expand_stop) {
+                if (lane == 0) acc += 1;  // passes through unchanged (seed chunks of plans that expand nothing too)
                 continue;
             }
             const DevLevel *lv = &pl->lv[d];

@@ -97,6 +97,7 @@ struct DevTail {
     uint8_t lane_par;                           // every mask is one key: count 32 prefixes per warp step
     uint8_t pair_par;                           // every mask is one key, a pair or a set: same
     uint8_t single;                             // keys that are a mask by themselves
+    uint8_t product;                            // one vertex per class: the tail is the masks' product
     uint8_t deep;                               // pendant plans: classes whose keys hang off depth c
     uint16_t mask[CSM_TAIL_MAXMASKS];
     // Signature of a mask of two keys, CSM_NO_PAIR for every other: the two (relation, rule) pairs.

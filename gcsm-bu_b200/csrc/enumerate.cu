@@ -231,6 +231,13 @@ __device__ __forceinline__ unsigned long long tail_product(const EnumParams &P, 
                                                            const uint32_t (&ksize)[CSM_TAIL_MAXKEYS], uint32_t classes) {
     const DevTail *T = &pl->tail;
     unsigned long long total = 1;
+    if (classes == 0xFFu && __ldg(&T->product)) {
+        const uint32_t nkeys = __ldg(&T->nkeys);
+#pragma unroll
+        for (uint32_t k = 0; k < CSM_TAIL_MAXKEYS; k++)
+            if (k < nkeys) total *= ksize[k];
+        return total;
+    }
     const DevTailTerm *terms = P.terms + pl->term_begin;
     const uint32_t nclasses = __ldg(&T->nclasses);
     for (uint32_t c = 0; c < nclasses; c++) {
@@ -385,16 +392,68 @@ __device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const Dev
         miss = e.x != ta || e.y != tb || e.z != tag;
         count = e.w;
     }
-    for (uint32_t need = __ballot_sync(0xffffffffu, miss); need;) {
-        const uint32_t l = __ffs(need) - 1;
-        const uint32_t va = __shfl_sync(0xffffffffu, a, l), vb = __shfl_sync(0xffffffffu, b, l);
-        uint32_t from = 0;
-        const uint32_t c = intersect_lists<false>(P, list_of(P, ra, va, 1000 + d), rule_a, list_of(P, rb, vb, 1000 + d), rule_b,
-                                                  nullptr, 0u, nullptr, from);
-        const bool same = miss && a == va && b == vb;
-        if (same) count = c;
-        if (lane == l) store_pair(slot, ta, tb, tag, c);
-        need &= ~__ballot_sync(0xffffffffu, same);
+    uint32_t need = __ballot_sync(0xffffffffu, miss);
+    if (need) {
+        uint2 la = make_uint2(0u, 0u), lb = la;
+        if (miss) {
+            la = list_of(P, ra, a, 1000 + d);
+            lb = list_of(P, rb, b, 1000 + d);
+        }
+        // The shorter list of every missing pair; all of them end to end where they are short (64
+        // entries on average), so that pairs over short lists share the warp's lanes instead of taking
+        // a pass each.  Pairs that do not depend on the candidate are one pair for all lanes.
+        const bool swap = lb.y < la.y;
+        const uint2 sh = swap ? lb : la, lg = swap ? la : lb;
+        uint32_t incl = sh.y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += t;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        if ((pa == d || pb == d) && total <= 64u * __popc(need)) {
+            const uint32_t start = incl - sh.y;
+            uint32_t mine = 0;
+            for (uint32_t g0 = 0; g0 < total; g0 += 32) {
+                const uint32_t g = g0 + lane;
+                // The pair of position g: the first lane whose inclusive prefix exceeds g.
+                uint32_t j = 0;
+#pragma unroll
+                for (uint32_t step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= g) j += step;
+                const uint32_t first = __shfl_sync(0xffffffffu, start, j), off = __shfl_sync(0xffffffffu, sh.x, j);
+                const uint32_t loff = __shfl_sync(0xffffffffu, lg.x, j), size = __shfl_sync(0xffffffffu, lg.y, j);
+                const bool sw = __shfl_sync(0xffffffffu, swap, j);
+                bool hit = false;
+                if (g < total) {
+                    const uint32_t e = __ldg(P.g.pool + off + (g - first));
+                    if (key_counts(sw ? rule_b : rule_a, e)) {
+                        const uint32_t x = find_entry(P.g.pool + loff, size, e >> 1);
+                        hit = x != 0xFFFFFFFFu && key_counts(sw ? rule_a : rule_b, x);
+                    }
+                }
+                const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                const uint32_t lo = start > g0 ? start - g0 : 0u, hi = incl > g0 ? incl - g0 : 0u;
+                if (lo < 32u && hi > lo)
+                    mine += __popc(hits & (0xFFFFFFFFu << lo) & (hi >= 32u ? 0xFFFFFFFFu : (1u << hi) - 1u));
+            }
+            if (miss) {
+                count = mine;
+                store_pair(slot, ta, tb, tag, mine);
+            }
+            need = 0;
+        }
+        while (need) {
+            const uint32_t l = __ffs(need) - 1;
+            const uint32_t va = __shfl_sync(0xffffffffu, a, l), vb = __shfl_sync(0xffffffffu, b, l);
+            const uint2 xa = make_uint2(__shfl_sync(0xffffffffu, la.x, l), __shfl_sync(0xffffffffu, la.y, l));
+            const uint2 xb = make_uint2(__shfl_sync(0xffffffffu, lb.x, l), __shfl_sync(0xffffffffu, lb.y, l));
+            uint32_t from = 0;
+            const uint32_t c = intersect_lists<false>(P, xa, rule_a, xb, rule_b, nullptr, 0u, nullptr, from);
+            const bool same = miss && a == va && b == vb;
+            if (same) count = c;
+            if (lane == l) store_pair(slot, ta, tb, tag, c);
+            need &= ~__ballot_sync(0xffffffffu, same);
+        }
     }
     uint32_t excl = __ldg(&T->key_excl[ka]) & ((2u << d) - 1u) & ~(1u << pa) & ~(1u << pb);
     if (excl && ok) {
@@ -493,6 +552,12 @@ __device__ unsigned long long tail_count_pairs(WarpState &S, const EnumParams &P
         }
     }
     unsigned long long total = ok ? 1 : 0;
+    if (__ldg(&T->product)) {
+#pragma unroll
+        for (uint32_t k = 0; k < CSM_PAIR_MAXMASKS; k++)
+            if (k < nmasks) total *= msize[k];
+        return total;
+    }
     const DevTailTerm *terms = P.terms + pl->term_begin;
     const uint32_t nclasses = __ldg(&T->nclasses);
     for (uint32_t c = 0; c < nclasses; c++) {

@@ -420,6 +420,7 @@ bool build_tail(const Query &q, const HostPlan &hp, int qe, const RelOf &rel_of,
         c++;
     }
     tail.nclasses = (uint8_t)c;
+    tail.product = c == n - hp.tail_start ? 1 : 0;
     tail.class_term_begin[c] = (uint16_t)terms.size();
     if (masks.size() > CSM_TAIL_MAXMASKS) return false;
     tail.nmasks = (uint8_t)masks.size();

@@ -144,9 +144,16 @@ struct DevPlan {
     // c's label (they are a factor of the prefix), and where prefix vertices share c's label (depths of
     // lv[c].excl_mask): each such vertex that is a candidate of c takes its own tail value off the
     // sum.  Table memo_tail holds those values, the tail count below c for every data vertex at c.
+    // And where c has one tail vertex below it and prefix vertices share that one's label (depths in
+    // memo_cut): the sum then counts each of them once for every candidate of c adjacent to it, which
+    // is the size of a pair intersection, c's list and the cut vertex's list of relation cut_rel.
     uint8_t memo_slot;
     uint8_t memo_depth;
     uint8_t memo_tail;
+    uint8_t cut_key;      // the tail key
+    uint16_t memo_cut;
+    uint16_t cut_rel;     // relation of (tail vertex -> c)
+    uint16_t cut_pair;    // signature in the pair table (DevTail.mask_pair)
     // CSM_SEED_*: where the updated query edge ends in a leaf (a query vertex of degree one), all
     // batch edges at one data vertex share everything but the leaf, so the search starts once per
     // data vertex f[0] of the inner endpoint that owns batch edges, and the leaf is counted.  Depth

@@ -508,8 +508,16 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
         auto ps = build_plans(q, (uint16_t)qi, nlf_base_[qi], stats[qi], po, rel_of);
         if (po.cartesian)
             for (HostPlan &hp : ps) {
-                group_leaf_seeds(q, nlf_base_[qi], rel_of, hp);
-                extend_pendant(hp);
+                HostPlan grouped = hp;
+                const bool g = group_leaf_seeds(q, nlf_base_[qi], rel_of, grouped);
+                if (g) extend_pendant(q, rel_of, grouped);
+                if (!g || (grouped.dev.seed_group == CSM_SEED_TAIL && grouped.dev.memo_slot == CSM_NO_MEMO)) {
+                    // A pendant plan per batch edge scans two levels less than one per inner vertex
+                    // that has to walk its counting level.
+                    extend_pendant(q, rel_of, hp);
+                    if (!g || hp.dev.memo_slot != CSM_NO_MEMO) continue;
+                }
+                hp = grouped;
             }
         begin.push_back((uint32_t)plans.size());
         plans.insert(plans.end(), ps.begin(), ps.end());
@@ -632,6 +640,22 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
         const int level = hp.dev.tail_start - 1;  // the counting level
         bool all = hp.dev.tail_start < hp.dev.n && level >= 2 && t.nmasks <= CSM_PAIR_MAXMASKS && !t.lane_par;
         int sets = 0;
+        // Signature of the lists (rel << 2 | rule) x and y, CSM_NO_PAIR when there are too many.
+        auto signature = [&](uint32_t x, uint32_t y) -> uint16_t {
+            const bool swap = y < x;
+            if (swap) std::swap(x, y);
+            const size_t id = std::find(sigs.begin(), sigs.end(), std::make_pair(x, y)) - sigs.begin();
+            if (id >= CSM_PAIR_SIGS) return CSM_NO_PAIR;
+            if (id == sigs.size()) sigs.push_back({x, y});
+            return (uint16_t)(id | (swap ? CSM_PAIR_SWAP : 0u));
+        };
+        if (hp.dev.memo_cut && hp.dev.memo_slot < CSM_MEMO_PENDING) {
+            const DevLevel &lv = hp.dev.lv[level];
+            hp.dev.cut_pair = signature((uint32_t)lv.bn_rel[0] << 2 | ((lv.old_mask & 1u) ? CSM_KEY_OLD : CSM_KEY_ANY),
+                                        (uint32_t)hp.dev.cut_rel << 2 | t.key_old[hp.dev.cut_key]);
+            if (hp.dev.cut_pair == CSM_NO_PAIR) hp.dev.memo_slot = CSM_MEMO_PENDING;
+            else used = true;
+        }
         for (int m = 0; m < t.nmasks; m++) {
             const int bits = __builtin_popcount(t.mask[m]);
             if (bits == 3) {
@@ -648,16 +672,8 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
                 continue;
             }
             const int ka = __builtin_ctz(t.mask[m]), kb = 31 - __builtin_clz(t.mask[m]);
-            uint32_t a = (uint32_t)t.key_rel[ka] << 2 | t.key_old[ka], b = (uint32_t)t.key_rel[kb] << 2 | t.key_old[kb];
-            const bool swap = b < a;
-            if (swap) std::swap(a, b);
-            const size_t id = std::find(sigs.begin(), sigs.end(), std::make_pair(a, b)) - sigs.begin();
-            if (id >= CSM_PAIR_SIGS) {
-                all = false;
-                continue;
-            }
-            if (id == sigs.size()) sigs.push_back({a, b});
-            t.mask_pair[m] = (uint16_t)(id | (swap ? CSM_PAIR_SWAP : 0u));
+            t.mask_pair[m] = signature((uint32_t)t.key_rel[ka] << 2 | t.key_old[ka], (uint32_t)t.key_rel[kb] << 2 | t.key_old[kb]);
+            if (t.mask_pair[m] == CSM_NO_PAIR) all = false;
         }
         t.pair_par = all ? 1 : 0;
         used = used || all;
@@ -679,7 +695,10 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
         }
     }
     if (!d_pairs_)
-        for (HostPlan &hp : plans) hp.dev.tail.pair_par = 0;
+        for (HostPlan &hp : plans) {
+            hp.dev.tail.pair_par = 0;
+            if (hp.dev.memo_cut && hp.dev.memo_slot < CSM_MEMO_PENDING) hp.dev.memo_slot = CSM_MEMO_PENDING;
+        }
     return CSM_OK;
 }
 

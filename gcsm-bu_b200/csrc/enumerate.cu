@@ -360,25 +360,13 @@ __device__ __forceinline__ void store_pair(uint4 *slot, uint32_t a, uint32_t b, 
                  : "memory");
 }
 
-// Size of the pair mask mi for this lane's prefix f[0..d-1] + cand (where ok): from the pair table, or
-// counted by the whole warp, one missing pair after the other, and put there.  The table holds the
-// intersection of the two lists under their rules; the prefix vertices of the mask's label that sit in
-// both are taken off here.
-__device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const DevTail *T, uint32_t mi, uint32_t d, bool ok,
-                              uint32_t cand) {
+// Size of the intersection of lists (ra, a) and (rb, b) under their rules, for every lane with ok set:
+// from the pair table under signature `sig`, or counted by the warp and put there.  `uniform`: a and b
+// are the same for all lanes.
+__device__ uint32_t pair_lookup(const EnumParams &P, uint32_t sig, uint32_t ra, uint32_t rule_a, uint32_t a, uint32_t rb,
+                                uint32_t rule_b, uint32_t b, bool ok, bool uniform, uint32_t where) {
     const uint32_t lane = lane_id();
-    const uint32_t mask = __ldg(&T->mask[mi]), sig = __ldg(&T->mask_pair[mi]);
-    uint32_t ka = __ffs(mask) - 1, kb = 31 - __clz(mask);
-    if (sig & CSM_PAIR_SWAP) {
-        const uint32_t t = ka;
-        ka = kb;
-        kb = t;
-    }
-    const uint32_t pa = __ldg(&T->key_parent[ka]), pb = __ldg(&T->key_parent[kb]);
-    const uint32_t ra = __ldg(&T->key_rel[ka]), rb = __ldg(&T->key_rel[kb]);
-    const uint32_t rule_a = __ldg(&T->key_old[ka]), rule_b = __ldg(&T->key_old[kb]);
     const uint32_t tag = P.ctrl->pair_phase << 12 | (sig & 0xFFFu);
-    const uint32_t a = pa == d ? cand : S.f[pa], b = pb == d ? cand : S.f[pb];
     uint32_t ta = a, tb = b;  // lists of one relation and rule: either order is the same pair
     if (ra == rb && rule_a == rule_b && b < a) {
         ta = b;
@@ -396,8 +384,8 @@ __device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const Dev
     if (need) {
         uint2 la = make_uint2(0u, 0u), lb = la;
         if (miss) {
-            la = list_of(P, ra, a, 1000 + d);
-            lb = list_of(P, rb, b, 1000 + d);
+            la = list_of(P, ra, a, where);
+            lb = list_of(P, rb, b, where);
         }
         // The shorter list of every missing pair; all of them end to end where they are short (64
         // entries on average), so that pairs over short lists share the warp's lanes instead of taking
@@ -410,7 +398,7 @@ __device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const Dev
             if (lane >= (uint32_t)o) incl += t;
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        if ((pa == d || pb == d) && total <= 64u * __popc(need)) {
+        if (!uniform && total <= 64u * __popc(need)) {
             const uint32_t start = incl - sh.y;
             uint32_t mine = 0;
             for (uint32_t g0 = 0; g0 < total; g0 += 32) {
@@ -455,6 +443,26 @@ __device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const Dev
             need &= ~__ballot_sync(0xffffffffu, same);
         }
     }
+    return count;
+}
+
+// Size of the pair mask mi for this lane's prefix f[0..d-1] + cand (where ok).  The table holds the
+// intersection of the two lists under their rules; the prefix vertices of the mask's label that sit in
+// both are taken off here.
+__device__ uint32_t pair_size(const WarpState &S, const EnumParams &P, const DevTail *T, uint32_t mi, uint32_t d, bool ok,
+                              uint32_t cand) {
+    const uint32_t mask = __ldg(&T->mask[mi]), sig = __ldg(&T->mask_pair[mi]);
+    uint32_t ka = __ffs(mask) - 1, kb = 31 - __clz(mask);
+    if (sig & CSM_PAIR_SWAP) {
+        const uint32_t t = ka;
+        ka = kb;
+        kb = t;
+    }
+    const uint32_t pa = __ldg(&T->key_parent[ka]), pb = __ldg(&T->key_parent[kb]);
+    const uint32_t ra = __ldg(&T->key_rel[ka]), rb = __ldg(&T->key_rel[kb]);
+    const uint32_t rule_a = __ldg(&T->key_old[ka]), rule_b = __ldg(&T->key_old[kb]);
+    const uint32_t a = pa == d ? cand : S.f[pa], b = pb == d ? cand : S.f[pb];
+    uint32_t count = pair_lookup(P, sig, ra, rule_a, a, rb, rule_b, b, ok, pa != d && pb != d, 1000 + d);
     uint32_t excl = __ldg(&T->key_excl[ka]) & ((2u << d) - 1u) & ~(1u << pa) & ~(1u << pb);
     if (excl && ok) {
         const uint2 la = list_of(P, ra, a, 1100 + d), lb = list_of(P, rb, b, 1100 + d);
@@ -1316,7 +1324,10 @@ __device__ unsigned long long count_shared_last(WarpState &S, const EnumParams &
 // Pendant counting level c = d + 1 (DevPlan.memo_slot): every buffered candidate of level d
 // contributes the table entry of the data vertex y at memo_depth (the candidate itself when that
 // depth is d), less the tail values of the prefix vertices of c's label that are candidates of c below
-// y, times the tail classes that hang off the prefix.  Consumes the buffer.
+// y, times the tail classes that hang off the prefix.  Where prefix vertices share the label of the one
+// tail vertex below c (memo_cut), each is taken off once per candidate of c next to it: a pair
+// intersection.  Consumes the buffer.
+template <bool PAIRS>
 __device__ unsigned long long settle_pendant(WarpState &S, const EnumParams &P, const DevPlan *pl, uint32_t d,
                                              uint32_t &tails) {
     const uint32_t lane = lane_id();
@@ -1325,12 +1336,26 @@ __device__ unsigned long long settle_pendant(WarpState &S, const EnumParams &P, 
     const DevTail *T = &pl->tail;
     const DevLevel *lv = &pl->lv[d + 1];
     unsigned long long v = 0;
+    const uint32_t cut = PAIRS ? __ldg(&pl->memo_cut) : 0u;
+    const uint32_t x = lane < k ? S.buf[d][ps + lane] : 0u;
+    const uint32_t y = md == d ? x : S.f[md];
+    unsigned long long cuts = 0;
+    if (PAIRS && cut) {
+        const uint32_t sig = __ldg(&pl->cut_pair);
+        const uint32_t rc = __ldg(&lv->bn_rel[0]), rule_c = (__ldg(&lv->old_mask) & 1u) ? CSM_KEY_OLD : CSM_KEY_ANY;
+        const uint32_t rl = __ldg(&pl->cut_rel), rule_l = __ldg(&T->key_old[__ldg(&pl->cut_key)]);
+        for (uint32_t em = cut; em; em &= em - 1) {
+            const uint32_t j = __ffs(em) - 1, z = j == d ? x : S.f[j];
+            const bool uniform = md != d && j != d;
+            cuts += (sig & CSM_PAIR_SWAP)
+                        ? pair_lookup(P, sig, rl, rule_l, z, rc, rule_c, y, lane < k, uniform, 970 + d)
+                        : pair_lookup(P, sig, rc, rule_c, y, rl, rule_l, z, lane < k, uniform, 970 + d);
+        }
+    }
     if (lane < k) {
-        const uint32_t x = S.buf[d][ps + lane];
-        const uint32_t y = md == d ? x : S.f[md];
-        v = __ldg(P.memo + (size_t)pl->memo_slot * P.g.V + y);
+        v = __ldg(P.memo + (size_t)pl->memo_slot * P.g.V + y) - cuts;
         uint32_t excl = __ldg(&lv->excl_mask) & ~(1u << md);
-        if (excl && v) {
+        if (excl) {
             const uint2 ms = list_of(P, __ldg(&lv->bn_rel[0]), y, 950 + d);
             const bool old = (__ldg(&lv->old_mask) & 1u) != 0;
             const uint32_t nlf_id = __ldg(&lv->nlf_bitmap);
@@ -1340,6 +1365,15 @@ __device__ unsigned long long settle_pendant(WarpState &S, const EnumParams &P, 
                 if (e == 0xFFFFFFFFu || (old && (e & 1u))) continue;
                 if (nlf_id != CSM_NO_BITMAP && !test_bit(bitmap(P, nlf_id), z)) continue;
                 v -= __ldg(P.memo + (size_t)pl->memo_tail * P.g.V + z);
+                if (!PAIRS || !cut) continue;
+                // z is no candidate: what the cut vertices took off for it comes back.
+                const uint32_t key = __ldg(&pl->cut_key), rule = __ldg(&T->key_old[key]);
+                const uint2 zs = list_of(P, __ldg(&T->key_rel[key]), z, 980 + d);
+                for (uint32_t cm = cut; cm; cm &= cm - 1) {
+                    const uint32_t i = __ffs(cm) - 1;
+                    const uint32_t en = find_entry(P.g.pool + zs.x, zs.y, i == d ? x : S.f[i]);
+                    v += en != 0xFFFFFFFFu && key_counts(rule, en);
+                }
             }
         }
         const uint32_t rest = ((1u << __ldg(&T->nclasses)) - 1u) & ~__ldg(&T->deep);
@@ -1457,9 +1491,10 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             if (waiting) try_donate(S, P, pl, L0, d, waiting);
         }
         if (S.pos[d] < S.nbuf[d]) {
-            if (MODE == CSM_ENUM_MODE_COUNT && d + 2 == E && P.memo != nullptr && pl->memo_slot < CSM_MEMO_PENDING) {
+            if (MODE == CSM_ENUM_MODE_COUNT && d + 2 == E && P.memo != nullptr && pl->memo_slot < CSM_MEMO_PENDING &&
+                (PAIRS || !pl->memo_cut)) {
                 // Pendant counting level below: each buffered candidate's count is a table entry.
-                cnt += settle_pendant(S, P, pl, d, tails);
+                cnt += settle_pendant<PAIRS>(S, P, pl, d, tails);
                 continue;
             }
             if (MODE == CSM_ENUM_MODE_COUNT && d + 2 == n && pl->shared_last) {

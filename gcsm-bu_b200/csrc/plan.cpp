@@ -657,12 +657,14 @@ bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, Ho
     return true;
 }
 
-bool extend_pendant(HostPlan &hp) {
+bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp) {
     DevPlan &dp = hp.dev;
     const DevTail &t = dp.tail;
     const int c = dp.tail_start - 1;
     if (dp.memo_slot != CSM_NO_MEMO || dp.tail_start >= dp.n || !t.lane_par || c < 3 || dp.lv[c].nbn != 1) return false;
+    const uint16_t prefix = (uint16_t)((1u << c) - 1u);
     uint8_t deep = 0;
+    int cut_key = -1, deep_keys = 0;
     for (int cl = 0; cl < t.nclasses; cl++) {
         bool below = false, above = false;
         for (int i = t.class_term_begin[cl]; i < t.class_term_begin[cl + 1]; i++)
@@ -670,7 +672,8 @@ bool extend_pendant(HostPlan &hp) {
                 const int k = __builtin_ctz(t.mask[hp.terms[i].f[j]]);
                 if (t.key_parent[k] == c) {
                     below = true;
-                    if (t.key_excl[k] & ((1u << c) - 1u)) return false;  // a prefix vertex could sit in the list
+                    deep_keys++;
+                    if (t.key_excl[k] & prefix) cut_key = k;  // a prefix vertex could sit in the list
                 } else {
                     above = true;
                     if ((t.key_excl[k] >> c) & 1u) return false;  // c's vertex could sit in the list
@@ -680,9 +683,22 @@ bool extend_pendant(HostPlan &hp) {
         if (below) deep |= (uint8_t)(1u << cl);
     }
     if (!deep) return false;
+    const uint8_t md = dp.lv[c].bn_depth[0];
+    if (cut_key >= 0) {
+        // One tail vertex below c, which has no other query neighbours; a candidate of c next to a cut
+        // vertex then passes c's NLF rule, since that vertex does not share its group with f[md].
+        const uint8_t uc = dp.order[c];
+        int leaf = -1;
+        for (int d = dp.tail_start; d < dp.n; d++)
+            if (q.adjacent(uc, dp.order[d])) leaf = dp.order[d];
+        if (deep_keys != 1 || q.degree(uc) != 2 || leaf < 0 || q.vlabel[leaf] == q.vlabel[dp.order[md]]) return false;
+        dp.memo_cut = t.key_excl[cut_key] & prefix;
+        dp.cut_key = (uint8_t)cut_key;
+        dp.cut_rel = rel_of((uint32_t)leaf, uc);
+    }
     dp.tail.deep = deep;
     dp.memo_slot = CSM_MEMO_PENDING;
-    dp.memo_depth = dp.lv[c].bn_depth[0];
+    dp.memo_depth = md;
     dp.expand_stop = (uint8_t)(c - 1);
     return true;
 }

@@ -56,7 +56,7 @@ bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, Ho
 
 // Marks the device form of a plan as pendant (DevPlan.memo_slot) where it is not already and its
 // counting level allows it.  Returns whether it did.
-bool extend_pendant(HostPlan &hp);
+bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp);
 
 // Text description, one block per query edge, in the spirit of PlanManager::PrintOrders.
 std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans);

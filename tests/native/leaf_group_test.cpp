@@ -81,6 +81,16 @@ long long tail_value(const Graph &g, const DevPlan &p, const std::vector<DevTail
     return tail(g, p, terms, f, p.tail.deep, p.tail_start);
 }
 
+// Vertices in list (ra, a) and in list (rb, b), each under its rule.
+long long common(const Graph &g, int ra, uint32_t a, int rule_a, int rb, uint32_t b, int rule_b) {
+    long long n = 0;
+    for (const Entry &e : g.list(ra, a)) {
+        const int x = g.entry(rb, b, e.v);
+        n += counts(rule_a, e.batch) && x && counts(rule_b, x == 2);
+    }
+    return n;
+}
+
 // A pendant counting level below the prefix f[0..c-1]: the sum over its list, without exclusions, less
 // the prefix vertices that the sum should not hold, times what hangs off the prefix.
 long long settle(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, const uint32_t *f) {
@@ -93,8 +103,17 @@ long long settle(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm
     for (int j = 0; j < c; j++) {
         if (!((lv.excl_mask >> j) & 1u) || j == md) continue;
         const int x = g.entry(lv.bn_rel[0], f[md], f[j]);
-        if (x && !(old && x == 2)) sum -= tail_value(g, p, terms, f[j]);
+        if (!x || (old && x == 2)) continue;
+        sum -= tail_value(g, p, terms, f[j]);
+        for (int i = 0; i < c; i++) {
+            if (!((p.memo_cut >> i) & 1u)) continue;
+            const int y = g.entry(p.tail.key_rel[p.cut_key], f[j], f[i]);
+            sum += y && counts(p.tail.key_old[p.cut_key], y == 2);
+        }
     }
+    for (int i = 0; i < c; i++)
+        if ((p.memo_cut >> i) & 1u)
+            sum -= common(g, lv.bn_rel[0], f[md], old ? CSM_KEY_OLD : CSM_KEY_ANY, p.cut_rel, f[i], p.tail.key_old[p.cut_key]);
     return sum * tail(g, p, terms, f, ~(unsigned)p.tail.deep, c);
 }
 
@@ -143,7 +162,7 @@ long long count(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm>
 
 int main() {
     std::mt19937 rng(77);
-    int grouped[3] = {0, 0, 0}, nonzero = 0, pendant = 0;
+    int grouped[3] = {0, 0, 0}, nonzero = 0, pendant = 0, cut = 0;
     for (int qn = 0; qn < 600; qn++) {
         const uint32_t nv = 2 + rng() % 6, nlab = 1 + rng() % 4;
         std::vector<uint32_t> vl(nv), src, dst, el;
@@ -167,6 +186,7 @@ int main() {
             auto k = std::make_tuple(q.vlabel[u], q.edge_label(u, uu), q.vlabel[uu]);
             return rels.emplace(k, (uint16_t)rels.size()).first->second;
         };
+        for (auto &e : q.qe_list) rel_of(e.first, e.second), rel_of(e.second, e.first);
         EdgeStats st;
         st.card.assign(nv * nv, 1);
         st.avg.assign(nv * nv, 1.f);
@@ -202,9 +222,10 @@ int main() {
             const long long got = count(g, hp.dev, hp.terms);
             nonzero += did && want > 0;
             for (HostPlan ep : {plans[i], hp}) {
-                if (!extend_pendant(ep)) continue;
+                if (!extend_pendant(q, rel_of, ep)) continue;
                 const long long settled = count(g, ep.dev, ep.terms);
                 pendant += want > 0;
+                cut += want > 0 && ep.dev.memo_cut;
                 if (settled != want) {
                     std::printf("FAIL query %d plan %zu: %lld settled, %lld counted\n", qn, i, settled, want);
                     return 1;
@@ -217,10 +238,10 @@ int main() {
         }
     }
     if (grouped[CSM_SEED_WEIGHT] < 50 || grouped[CSM_SEED_TAIL] < 50 || nonzero < 100 ||
-        pendant < 20)
-        return std::printf("too few plans: %d weighted, %d in the tail, %d of them with matches, %d pendant\n", grouped[1],
-                           grouped[2], nonzero, pendant), 1;
-    std::printf("ok %d weighted, %d in the tail, %d of them with matches, %d pendant\n", grouped[1], grouped[2], nonzero,
-                pendant);
+        pendant < 50 || cut < 20)
+        return std::printf("too few plans: %d weighted, %d in the tail, %d of them with matches, %d pendant, %d cut\n",
+                           grouped[1], grouped[2], nonzero, pendant, cut), 1;
+    std::printf("ok %d weighted, %d in the tail, %d of them with matches, %d pendant, %d of them cut\n", grouped[1], grouped[2],
+                nonzero, pendant, cut);
     return 0;
 }

@@ -47,6 +47,7 @@ QUERIES = [
     query([1, 0, 1, 0, 3, 2], [(0, 1), (1, 2), (2, 3), (3, 4), (1, 5)]),  # and above another tail class
     query([1, 2, 0, 3, 1], [(0, 1), (1, 2), (2, 3), (3, 0), (2, 4)]),     # two pair intersections
     query([0, 1, 2, 3, 0], [(0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (2, 3), (0, 4)]),  # three lists of one vertex
+    query([3, 3, 0, 1, 3, 0], [(0, 1), (0, 2), (2, 3), (3, 4), (4, 5)]),  # cut by a vertex of the tail's label
     query([0, 1, 0, 1, 1], [(0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (2, 3), (0, 4)]),  # of the prefix's labels
 ]
 
@@ -67,6 +68,7 @@ def test_rewritten_plans_equal_the_oracle(strategy):
         eng.load_graph(data)
         text = [eng.describe(i) for i in range(len(QUERIES))]
         assert "pendant counting level" in text[6] and "pendant counting level" in text[7]
+        assert "pendant counting level" in text[10]
         assert any("counted per inner vertex" in t for t in text) and any("counted in the tail" in t for t in text)
         oracles = [Oracle(q, data) for q in QUERIES]
         seen = 0

@@ -587,6 +587,11 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
                 const uint32_t a = order[n - 2], b = order[n - 1];
                 if ((int)n - tail_start != 2 || q.vlabel[a] == q.vlabel[b] || q.degree(a) != 2 || q.degree(b) != 2)
                     tail_start = (int)n;
+                // A last vertex with two or three lists, one of them the vertex's before it, is one such
+                // intersection per candidate of the level above (without that neighbour the shared
+                // last level counts it once for all of them).
+                if (tail_start == (int)n && n >= 4 && q.adjacent(a, b) && (q.degree(b) == 2 || q.degree(b) == 3))
+                    tail_start = (int)n - 1;
             }
         }
         hp.order = order;

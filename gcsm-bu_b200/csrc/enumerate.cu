@@ -139,6 +139,34 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t *L, uint32_t
     return lo + __popc(__ballot_sync(0xffffffffu, v < key2));
 }
 
+// First window of a search below: about twice what 32 consecutive entries of a list of `short_size` span
+// in one of `size`, a power of two of at least 64.
+__device__ __forceinline__ uint32_t first_window(uint32_t size, uint32_t short_size) {
+    const uint32_t per = short_size ? size / short_size : 0u;
+    return 64u << (per ? 31 - __clz(per) : 0);
+}
+
+// Entry of the sorted list L that names this lane's vertex (key = vertex << 1), or 0xFFFFFFFF.  The
+// lanes' keys ascend, `top` is the one of lane `last` and the largest; c0 is a position no lane's
+// entry lies before, and moves on to where the next keys start.  All lanes search a window from c0 on,
+// w0 entries wide and doubled until it holds `top`.  The window is a power of two and reads past the
+// end count as large, so the search has no data-dependent branch: log2(window) dependent reads, most
+// of them from a few cache lines.
+__device__ __forceinline__ uint32_t window_find(const uint32_t *L, uint32_t size, uint32_t &c0, uint32_t w0, uint32_t key,
+                                                uint32_t top, uint32_t last) {
+    uint32_t w = w0;
+    while (c0 + w < size && __ldg(L + c0 + w - 1u) < top) w <<= 1;
+    uint32_t pos = c0;
+    for (uint32_t s = w >> 1; s; s >>= 1) {
+        const uint32_t p = pos + s - 1u;
+        const uint32_t v = p < size ? __ldg(L + p) : 0xFFFFFFFFu;
+        if (v < key) pos += s;
+    }
+    const uint32_t e = pos < size ? __ldg(L + pos) : 0xFFFFFFFFu;
+    c0 = __shfl_sync(0xffffffffu, pos, last);
+    return (e & ~1u) == key ? e : 0xFFFFFFFFu;
+}
+
 // Lower bound of key2 among the 32 register-held window entries (sorted, padded with ~0).
 __device__ __forceinline__ uint32_t shfl_lower_bound(uint32_t win, uint32_t key2) {
     uint32_t pos = 0;
@@ -280,10 +308,7 @@ __device__ unsigned long long tail_count_lane(const uint32_t *ts_base, const uin
 }
 
 // Entries that two sorted lists share, each under its rule (CSM_KEY_*).  The warp scans the shorter
-// list 32 entries at a time; every lane searches its entry in the window of the longer list that the
-// chunk spans, which starts where the last chunk ended and is doubled until it holds the chunk's
-// largest entry.  The window is a power of two and reads past the end count as large, so the search
-// has no data-dependent branch: log2(window) dependent reads, most of them from a few cache lines.
+// list 32 entries at a time; every lane searches its entry in the longer one (window_find).
 // KEEP: the vertices found, without the prefix vertices f[j] with bit j of `excl`, go to `out`, and
 // the scan starts at entry `from` of the shorter list and stops (returning where in `from`) before a
 // chunk that might not fit in CSM_SET_CAP entries.
@@ -300,33 +325,20 @@ __device__ uint32_t intersect_lists(const EnumParams &P, uint2 a, uint32_t rule_
         rule_b = r;
     }
     const uint32_t *A = P.g.pool + a.x, *B = P.g.pool + b.x;
-    // First window: twice what a chunk spans on average.
-    const uint32_t per = a.y ? b.y / a.y : 0u;
-    const uint32_t w0 = 64u << (per ? 31 - __clz(per) : 0);
+    const uint32_t w0 = first_window(b.y, a.y);
     uint32_t cnt = 0, c0 = 0, base = KEEP ? from : 0u;
     for (; base < a.y && c0 < b.y; base += 32) {
         if (KEEP && cnt > CSM_SET_CAP - 32u) break;
         const uint32_t i = base + lane;
         const uint32_t e = i < a.y ? __ldg(A + i) : 0xFFFFFFFFu;
-        const uint32_t key = e & ~1u;
         const uint32_t last = a.y - base < 32u ? a.y - base - 1u : 31u;
-        const uint32_t top = __shfl_sync(0xffffffffu, key, last);
-        uint32_t w = w0;
-        while (w < b.y - c0 && __ldg(B + c0 + w - 1u) < top) w <<= 1;
-        uint32_t pos = c0;
-        for (uint32_t s = w >> 1; s; s >>= 1) {
-            const uint32_t p = pos + s - 1u;
-            const uint32_t v = p < b.y ? __ldg(B + p) : 0xFFFFFFFFu;
-            if (v < key) pos += s;
-        }
-        const uint32_t g = pos < b.y ? __ldg(B + pos) : 0xFFFFFFFFu;
-        bool hit = i < a.y && (g & ~1u) == key && g != 0xFFFFFFFFu && key_counts(rule_a, e) && key_counts(rule_b, g);
+        const uint32_t g = window_find(B, b.y, c0, w0, e & ~1u, __shfl_sync(0xffffffffu, e & ~1u, last), last);
+        bool hit = i < a.y && g != 0xFFFFFFFFu && key_counts(rule_a, e) && key_counts(rule_b, g);
         if (KEEP)
             for (uint32_t em = excl; hit && em; em &= em - 1) hit = f[__ffs(em) - 1] != (e >> 1);
         const uint32_t hits = __ballot_sync(0xffffffffu, hit);
         if (KEEP && hit) out[cnt + __popc(hits & ((1u << lane) - 1u))] = e >> 1;
         cnt += __popc(hits);
-        c0 = __shfl_sync(0xffffffffu, pos, last);
     }
     if (KEEP) {
         from = c0 < b.y ? base : a.y;
@@ -1605,57 +1617,25 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             const uint32_t nlf_id = S.nlf[d];
             const uint32_t nlf_word =
                 !ok ? 0u : (nlf_id == CSM_NO_BITMAP ? 0xFFFFFFFFu : __ldg(bitmap(P, nlf_id) + (cand >> 5)));
-            // Membership in the other backward lists.  The chunk's candidates ascend, so each
-            // list keeps a cursor.  The 32 entries at the cursor are read first: when they
-            // reach past the chunk's largest candidate, the window is in registers and
-            // shuffles find each candidate (one dependent read).  Otherwise a 32-ary warp search
-            // brackets the window and lanes search inside it.
-            const uint32_t nbn = S.nbn[d];
-            const uint32_t vmask = __ballot_sync(0xffffffffu, idx < S.hi[d]);
-            const uint32_t target = __shfl_sync(0xffffffffu, cand, 31 - __clz(vmask));
-            const uint32_t key_hi = (target + 1) << 1;
-            // The windows of up to four lists are read together (independent loads in flight
-            // at once), then each list is resolved in turn.
-            for (uint32_t k0 = 0; k0 < nbn; k0 += 4) {
+            // Membership in the other backward lists.  The chunk's candidates ascend, so each list
+            // keeps a cursor and is searched in the window from there on that the chunk spans.
+            const uint32_t nbn = S.nbn[d], bb = S.bnb[d];
+            const uint32_t last = 31 - __clz(__ballot_sync(0xffffffffu, idx < S.hi[d]));
+            const uint32_t key = cand << 1, top = __shfl_sync(0xffffffffu, key, last);
+            const uint32_t psize = S.psz[bb + piv];
+            for (uint32_t k = 0; k < nbn; k++) {
+                if (k == piv) continue;
                 if (!__any_sync(0xffffffffu, ok)) break;
-                uint32_t win[4];
-#pragma unroll
-                for (uint32_t j = 0; j < 4; j++) {
-                    const uint32_t k = k0 + j;
-                    win[j] = 0xFFFFFFFFu;
-                    if (k < nbn && k != piv) {
-                        const uint32_t slot = S.bnb[d] + k;
-                        const uint32_t c0 = S.cur[slot];
-                        if (c0 + lane < S.psz[slot]) win[j] = __ldg(P.g.pool + S.poff[slot] + c0 + lane);
-                    }
+                const uint32_t slot = bb + k, size = S.psz[slot];
+                uint32_t c0 = S.cur[slot];
+                const uint32_t e = window_find(P.g.pool + S.poff[slot], size, c0, first_window(size, psize), key, top, last);
+                if (ok) {
+                    probes++;
+                    ok = e != 0xFFFFFFFFu && !(((oldm >> k) & 1u) && (e & 1u));
                 }
-#pragma unroll
-                for (uint32_t j = 0; j < 4; j++) {
-                    const uint32_t k = k0 + j;
-                    if (k >= nbn || k == piv) continue;
-                    if (!__any_sync(0xffffffffu, ok)) break;
-                    const uint32_t slot = S.bnb[d] + k;
-                    const uint32_t *L = P.g.pool + S.poff[slot];
-                    const uint32_t c0 = S.cur[slot];
-                    const uint32_t size = S.psz[slot];
-                    const uint32_t below = __ballot_sync(0xffffffffu, win[j] < key_hi);
-                    uint32_t e = 0xFFFFFFFFu, hi;
-                    if (below != 0xffffffffu) {
-                        // The window [c0, hi) fits in the 32 entries just read.
-                        hi = c0 + __popc(below);
-                        const uint32_t pos = shfl_lower_bound(win[j], cand << 1);
-                        const uint32_t got = __shfl_sync(0xffffffffu, win[j], pos);
-                        if ((got >> 1) == cand && got != 0xFFFFFFFFu) e = got;
-                    } else {
-                        hi = warp_lower_bound(L, c0 + 32, size, key_hi, lane);
-                        if (ok) e = find_entry(L + c0, hi - c0, cand);
-                    }
-                    if (ok) {
-                        probes++;
-                        ok = e != 0xFFFFFFFFu && !(((oldm >> k) & 1u) && (e & 1u));
-                    }
-                    if (lane == 0) S.cur[slot] = hi;
-                }
+                __syncwarp();
+                if (lane == 0) S.cur[slot] = c0;
+                __syncwarp();
             }
             if (ok) ok = (nlf_word >> (cand & 31)) & 1u;
         }
@@ -1695,30 +1675,20 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
             if (d >= 2) {
                 const DevTail *T = &pl->tail;
                 const uint32_t nkeys = __ldg(&T->nkeys);
-                const uint32_t vm = __ballot_sync(0xffffffffu, idx < S.hi[d]);
-                const uint32_t tgt = __shfl_sync(0xffffffffu, cand, 31 - __clz(vm));
-                const uint32_t key_hi = (tgt + 1) << 1;
+                const uint32_t last = 31 - __clz(__ballot_sync(0xffffffffu, idx < S.hi[d]));
+                const uint32_t key = cand << 1, top = __shfl_sync(0xffffffffu, key, last);
+                const uint32_t psize = S.psz[S.bnb[d] + S.piv[d]];
                 for (uint32_t k = 0; k < nkeys; k++) {
                     if (__ldg(&T->key_parent[k]) >= d || !((__ldg(&T->single) >> k) & 1u)) continue;
                     if (!((__ldg(&T->key_excl[k]) >> d) & 1u)) continue;  // candidates never in this list
                     if (!__any_sync(0xffffffffu, ok)) break;
-                    const uint32_t *L = P.g.pool + S.ts_off[k];
                     const uint32_t size = S.ts_size[k];
-                    const uint32_t c0 = S.ts_cur[k];
-                    const uint32_t win = c0 + lane < size ? __ldg(L + c0 + lane) : 0xFFFFFFFFu;
-                    const uint32_t below = __ballot_sync(0xffffffffu, win < key_hi);
-                    uint32_t e = 0xFFFFFFFFu, hi;
-                    if (below != 0xffffffffu) {
-                        hi = c0 + __popc(below);
-                        const uint32_t pos = shfl_lower_bound(win, cand << 1);
-                        const uint32_t got = __shfl_sync(0xffffffffu, win, pos);
-                        if ((got >> 1) == cand && got != 0xFFFFFFFFu) e = got;
-                    } else {
-                        hi = warp_lower_bound(L, c0 + 32, size, key_hi, lane);
-                        if (ok) e = find_entry(L + c0, hi - c0, cand);
-                    }
+                    uint32_t c0 = S.ts_cur[k];
+                    const uint32_t e =
+                        window_find(P.g.pool + S.ts_off[k], size, c0, first_window(size, psize), key, top, last);
                     __syncwarp();
-                    if (lane == 0) S.ts_cur[k] = hi;
+                    if (lane == 0) S.ts_cur[k] = c0;
+                    __syncwarp();
                     if (ok) {
                         probes++;
                         if (e != 0xFFFFFFFFu && key_counts(__ldg(&T->key_old[k]), e)) shared_hit |= 1u << k;

@@ -343,7 +343,7 @@ csm_status Engine::build_lists(uint64_t ne, const uint32_t *src, const uint32_t 
             cudaMemcpy(d_src, src, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice);
             cudaMemcpy(d_dst, dst, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice);
             cudaMemcpy(d_lab, elabel, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice);
-            store_build_keys(ne, d_src, d_dst, d_lab, nullptr, lt, g_, kl_, k_raw, stream_);
+            store_build_keys(ne, d_src, d_dst, d_lab, nullptr, lt, g_, kl_, k_raw, BatchReset{}, stream_);
         }
         store_sort_keys(nullptr, temp_bytes, k_raw, k_sorted, m, kl_, stream_);
         if ((e = dev_alloc_bytes(&temp, temp_bytes + 16))) {
@@ -1026,21 +1026,30 @@ csm_status Engine::enqueue_batch(uint64_t n, const uint32_t *src, const uint32_t
                                  const uint8_t *is_delete, bool has_delete, bool tuning, cudaStream_t s) {
     const uint32_t m = (uint32_t)(2 * n);
     const uint32_t np = (uint32_t)plans_.size();
-    CSM_CUDA(cudaMemsetAsync(bs_.nheads, 0, sizeof(unsigned int), s));
-    CSM_CUDA(cudaMemsetAsync(bs_.counters, 0, 2 * sizeof(unsigned long long), s));
-    CSM_CUDA(cudaMemsetAsync(bs_.error, 0, sizeof(unsigned int), s));
-    CSM_CUDA(cudaMemsetAsync(d_counts_, 0, 2 * sizeof(unsigned long long) * np, s));
+    if (!m) {
+        CSM_CUDA(cudaMemsetAsync(bs_.nheads, 0, sizeof(unsigned int), s));
+        CSM_CUDA(cudaMemsetAsync(bs_.counters, 0, 2 * sizeof(unsigned long long), s));
+        CSM_CUDA(cudaMemsetAsync(bs_.error, 0, sizeof(unsigned int), s));
+        CSM_CUDA(cudaMemsetAsync(d_counts_, 0, 2 * sizeof(unsigned long long) * np, s));
+    }
     NlfTables nt{d_spec_begin_, d_specs_, d_bits_, words_};
     if (m) {
         LabelTables lt{d_elab_raw_, (uint32_t)elab_raw_.size(), d_rel_table_, (uint32_t)vlab_raw_.size()};
-        store_build_keys(n, src, dst, elabel, is_delete, lt, g_, kl_, d_keys_raw_, s);
+        BatchReset reset;
+        reset.nheads = bs_.nheads;
+        reset.error = bs_.error;
+        reset.counters = bs_.counters;
+        reset.counts = d_counts_;
+        reset.ncounts = 2 * np;
+        reset.touched = d_touched_;
+        reset.words = words_;
+        store_build_keys(n, src, dst, elabel, is_delete, lt, g_, kl_, d_keys_raw_, reset, s);
         size_t tb = sort_temp_bytes_;
         CSM_CUDA(store_sort_keys(d_sort_temp_, tb, d_keys_raw_, d_keys_, m, kl_, s));
-        store_classify(m, d_keys_, kl_, g_, bs_, s);
-        store_touched(m, d_keys_, kl_, d_touched_, words_, s);
+        store_classify(m, d_keys_, kl_, g_, bs_, d_touched_, words_, s);
         // Both phases start from the same seeds: the batch's keys by relation.
         launch_seed_tickets(d_plans_, np, d_keys_, m, kl_, sc_.seed_lo, sc_.ticket_prefix, s);
-        stats_.kernel_launches += 6;
+        stats_.kernel_launches += 5;
         if (d_rel_delta_) {
             CSM_CUDA(cudaMemsetAsync(d_rel_delta_, 0, sizeof(long long) * g_.R, s));
             store_rel_delta(m, d_keys_, kl_, bs_, d_rel_delta_, s);
@@ -1086,14 +1095,20 @@ csm_status Engine::enqueue_batch(uint64_t n, const uint32_t *src, const uint32_t
 // batch's single synchronisation (counts, edge counters, pool top, error bits).
 csm_status Engine::enqueue_readback(cudaStream_t s) {
     const uint32_t np = (uint32_t)plans_.size();
-    unsigned int *h_err = reinterpret_cast<unsigned int *>(h_counts_ + 2 * np + 3);
     CSM_CUDA(record_event(ev_[1], s));
-    CSM_CUDA(cudaMemcpyAsync(h_counts_, d_counts_, 2 * sizeof(unsigned long long) * np, cudaMemcpyDeviceToHost, s));
-    CSM_CUDA(cudaMemcpyAsync(h_counts_ + 2 * np, bs_.counters, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                             s));
-    CSM_CUDA(cudaMemcpyAsync(h_counts_ + 2 * np + 2, g_.pool_top, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                             s));
-    CSM_CUDA(cudaMemcpyAsync(h_err, bs_.error, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+    BatchResult r;
+    r.counts = d_counts_;
+    r.ncounts = 2 * np;
+    r.counters = bs_.counters;
+    r.pool_top = g_.pool_top;
+    r.error = bs_.error;
+    r.h_counts = h_counts_;
+    if (phase_ran_[1] && cfg_.materialize_rows == 0) {
+        r.ctrl = sc_.ctrl;
+        r.h_ctrl = &h_ctrl_[1];
+    }
+    store_read_back(r, s);
+    stats_.kernel_launches++;
     if (d_rel_delta_)
         CSM_CUDA(cudaMemcpyAsync(h_rel_delta_, d_rel_delta_, sizeof(long long) * g_.R, cudaMemcpyDeviceToHost, s));
     return CSM_OK;
@@ -1371,8 +1386,10 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
     stats_.enum_launches++;
     stats_.kernel_launches++;
     CSM_CUDA(record_event(ev_[3 + 2 * ph], s));
-    // Statistics and error bits are read after the batch's final synchronisation.
-    CSM_CUDA(cudaMemcpyAsync(&h_ctrl_[ph], sc_.ctrl, sizeof(EnumControl), cudaMemcpyDeviceToHost, s));
+    // Statistics and error bits are read after the batch's final synchronisation, those of the
+    // insertion phase with the batch's results.
+    if (ph == 0 || rows)
+        CSM_CUDA(cudaMemcpyAsync(&h_ctrl_[ph], sc_.ctrl, sizeof(EnumControl), cudaMemcpyDeviceToHost, s));
     if (rows) {
         // Collect rows per query for csm_get_embeddings (a validation path: synchronous).
         CSM_CUDA(cudaStreamSynchronize(s));

@@ -1820,13 +1820,11 @@ __global__ void __launch_bounds__(256, MINB) k_enumerate(EnumParams P) {
     }
 }
 
-// Per plan: the key range of its seed relation, and the number of 32-key seed chunks.  One warp per
-// plan and a 32-ary search: about log32(m) dependent reads for each end.
-__global__ void k_seed_ranges(const DevPlan *plans, uint32_t nplans, const unsigned long long *keys, uint32_t m,
-                              KeyLayout kl, uint32_t *seed_lo, uint32_t *chunks) {
+// Plan p: the key range of its seed relation, and the number of 32-key seed chunks.  A warp and a
+// 32-ary search: about log32(m) dependent reads for each end.
+__device__ void seed_range(const DevPlan *plans, uint32_t nplans, uint32_t p, const unsigned long long *keys, uint32_t m,
+                           KeyLayout kl, uint32_t *seed_lo, uint32_t *chunks) {
     const uint32_t lane = lane_id();
-    const uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (p >= nplans) return;
     const uint32_t rel = plans[p].seed_rel;
     uint32_t end[2];
 #pragma unroll
@@ -1852,8 +1850,8 @@ __global__ void k_seed_ranges(const DevPlan *plans, uint32_t nplans, const unsig
     }
 }
 
-// Exclusive prefix of chunk counts (one block; plans are few).
-__global__ void __launch_bounds__(1024) k_ticket_prefix(const uint32_t *chunks, uint32_t nplans, uint32_t *prefix) {
+// Exclusive prefix of chunk counts, by one block of 1024 threads.
+__device__ void ticket_prefix(const uint32_t *chunks, uint32_t nplans, uint32_t *prefix) {
     __shared__ uint32_t part[32];
     const uint32_t t = threadIdx.x, lane = lane_id();
     const uint32_t per = (nplans + blockDim.x - 1) / blockDim.x;
@@ -1881,6 +1879,29 @@ __global__ void __launch_bounds__(1024) k_ticket_prefix(const uint32_t *chunks, 
         acc += chunks[i];
     }
     if (t == blockDim.x - 1) prefix[nplans] = acc;
+}
+
+// One block finds the ranges of few plans and their prefix in one launch; more plans (32 warps take
+// more than four turns) get a grid for the ranges and a launch for the prefix.
+constexpr uint32_t kOneBlockPlans = 128;
+
+__global__ void __launch_bounds__(1024) k_seed_tickets(const DevPlan *plans, uint32_t nplans, const unsigned long long *keys,
+                                                       uint32_t m, KeyLayout kl, uint32_t *seed_lo, uint32_t *chunks,
+                                                       uint32_t *prefix) {
+    for (uint32_t p = threadIdx.x >> 5; p < nplans; p += blockDim.x >> 5)
+        seed_range(plans, nplans, p, keys, m, kl, seed_lo, chunks);
+    __syncthreads();
+    ticket_prefix(chunks, nplans, prefix);
+}
+
+__global__ void k_seed_ranges(const DevPlan *plans, uint32_t nplans, const unsigned long long *keys, uint32_t m,
+                              KeyLayout kl, uint32_t *seed_lo, uint32_t *chunks) {
+    const uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (p < nplans) seed_range(plans, nplans, p, keys, m, kl, seed_lo, chunks);
+}
+
+__global__ void __launch_bounds__(1024) k_ticket_prefix(const uint32_t *chunks, uint32_t nplans, uint32_t *prefix) {
+    ticket_prefix(chunks, nplans, prefix);
 }
 
 // Resets the control block for one phase.  The phase epoch (which marks queue slots ready) is the
@@ -2076,6 +2097,10 @@ void launch_seed_tickets(const DevPlan *plans, uint32_t nplans, const unsigned l
                          KeyLayout kl, uint32_t *seed_lo, uint32_t *ticket_prefix, cudaStream_t s) {
     // seed_lo holds three arrays of nplans: first key, end key, chunk count.
     uint32_t *chunks = seed_lo + 2 * nplans;
+    if (nplans <= kOneBlockPlans) {
+        k_seed_tickets<<<1, 1024, 0, s>>>(plans, nplans, keys, m, kl, seed_lo, chunks, ticket_prefix);
+        return;
+    }
     k_seed_ranges<<<(nplans + 3) / 4, 128, 0, s>>>(plans, nplans, keys, m, kl, seed_lo, chunks);
     k_ticket_prefix<<<1, 1024, 0, s>>>(chunks, nplans, ticket_prefix);
 }

@@ -33,7 +33,16 @@ __device__ __forceinline__ uint32_t slack_capacity(uint32_t size) {
 __global__ void k_build_keys(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elab,
                              const uint8_t *isdel, uint32_t V, const uint8_t *vlab, const uint32_t *elab_raw,
                              uint32_t nel, const uint16_t *rel_table, uint32_t nvl, KeyLayout kl,
-                             unsigned long long *keys) {
+                             unsigned long long *keys, BatchReset r) {
+    // The batch's counters, instead of a memset each in front of this kernel.
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    if (t == 0 && r.nheads) {
+        *r.nheads = 0;
+        *r.error = 0;
+        r.counters[0] = r.counters[1] = 0;
+    }
+    for (uint32_t i = t; i < r.ncounts; i += nt) r.counts[i] = 0;
+    for (uint32_t i = t; i < r.words; i += nt) r.touched[i] = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t x = src[i], y = dst[i];
         unsigned long long k0 = CSM_INVALID_KEY, k1 = CSM_INVALID_KEY;
@@ -62,16 +71,22 @@ __global__ void k_build_keys(uint64_t n, const uint32_t *src, const uint32_t *ds
 }
 
 // Deduplicates and classifies sorted keys; marks the entries of effective deletions and
-// collects the first key of every adjacency-list segment.
+// collects the first key of every adjacency-list segment.  `touched` gets the bit of every vertex that
+// owns a list some key belongs to (the key's source): keys are sorted, so one lane per distinct source
+// sets it.  Updates that match no relation carry CSM_INVALID_KEY (sorted to the end): they own no
+// list, and their all-ones source field is no vertex, so they are skipped.
 __global__ void k_classify(uint32_t m, const unsigned long long *keys, KeyLayout kl, const uint2 *meta,
                            uint32_t *pool, uint32_t V, uint8_t *eff, uint32_t *heads, unsigned int *nheads,
-                           unsigned long long *counters) {
+                           unsigned long long *counters, uint32_t *touched, uint32_t words) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x) {
         const unsigned long long k = keys[p];
         uint8_t e = CSM_EFF_NONE;
         if (k != CSM_INVALID_KEY) {
             const unsigned long long prev = p ? keys[p - 1] : CSM_INVALID_KEY;
             if (p == 0 || kl.list_of(prev) != kl.list_of(k)) heads[atomicAdd(nheads, 1u)] = p;
+            const uint32_t owner = kl.src(k);
+            if ((p == 0 || kl.src(prev) != owner) && (owner >> 5) < words)
+                atomicOr(touched + (owner >> 5), 1u << (owner & 31));
             if (p == 0 || (prev >> 1) != (k >> 1)) {
                 const uint32_t r = kl.rel(k), x = kl.src(k), y = kl.dst(k);
                 const uint2 ms = meta[(size_t)r * V + x];
@@ -426,18 +441,15 @@ __global__ void k_rel_delta(uint32_t m, const unsigned long long *keys, KeyLayou
         atomicAdd(reinterpret_cast<unsigned long long *>(delta + rel), (unsigned long long)(long long)sum);  // two's complement
 }
 
-// Bit per vertex that owns a list some batch key belongs to (the key's source).  Keys are
-// sorted, so neighbouring lanes mostly share a word; one lane per distinct source sets it.
-// Updates that match no relation carry CSM_INVALID_KEY (sorted to the end): they own no list,
-// and their all-ones source field is no vertex, so they are skipped.
-__global__ void k_touched(uint32_t m, const unsigned long long *keys, KeyLayout kl, uint32_t *bits, uint32_t words) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const unsigned long long k = keys[i];
-    if (k == CSM_INVALID_KEY) return;
-    const uint32_t x = kl.src(k);
-    if (i > 0 && kl.src(keys[i - 1]) == x) return;
-    if ((x >> 5) < words) atomicOr(bits + (x >> 5), 1u << (x & 31));
+// The batch's results, straight to the host's memory: one launch instead of a copy each.
+__global__ void k_read_back(BatchResult r) {
+    for (uint32_t i = threadIdx.x; i < r.ncounts; i += blockDim.x) r.h_counts[i] = r.counts[i];
+    if (threadIdx.x < 2) r.h_counts[r.ncounts + threadIdx.x] = r.counters[threadIdx.x];
+    if (threadIdx.x == 2) r.h_counts[r.ncounts + 2] = *r.pool_top;
+    if (threadIdx.x == 3) *reinterpret_cast<unsigned int *>(r.h_counts + r.ncounts + 3) = *r.error;
+    if (r.ctrl)
+        for (uint32_t i = threadIdx.x; i < sizeof(EnumControl) / 4; i += blockDim.x)
+            reinterpret_cast<uint32_t *>(r.h_ctrl)[i] = reinterpret_cast<const uint32_t *>(r.ctrl)[i];
 }
 
 // Entry count of every relation (sum of its list sizes).  The loop is warp-uniform so that all
@@ -469,9 +481,9 @@ inline int grid_for(size_t n, int block) {
 
 void store_build_keys(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elab, const uint8_t *isdel,
                       const LabelTables &lt, const DeviceGraph &g, KeyLayout kl, unsigned long long *keys,
-                      cudaStream_t s) {
+                      const BatchReset &reset, cudaStream_t s) {
     k_build_keys<<<grid_for(n, 256), 256, 0, s>>>(n, src, dst, elab, isdel, g.V, g.vlab, lt.elab_raw, lt.nel,
-                                                  lt.rel_table, lt.nvl, kl, keys);
+                                                  lt.rel_table, lt.nvl, kl, keys, reset);
 }
 
 cudaError_t store_sort_keys(void *temp, size_t &temp_bytes, const unsigned long long *in, unsigned long long *out,
@@ -480,9 +492,9 @@ cudaError_t store_sort_keys(void *temp, size_t &temp_bytes, const unsigned long 
 }
 
 void store_classify(uint32_t m, const unsigned long long *keys, KeyLayout kl, DeviceGraph &g, BatchScratch &b,
-                    cudaStream_t s) {
+                    uint32_t *touched, uint32_t words, cudaStream_t s) {
     k_classify<<<grid_for(m, 256), 256, 0, s>>>(m, keys, kl, g.meta, g.pool, g.V, b.eff, b.heads, b.nheads,
-                                                b.counters);
+                                                b.counters, touched, words);
     k_seg_info<<<grid_for((size_t)m * 32, 256), 256, 0, s>>>(b.heads, b.nheads, keys, m, kl, b.eff, b.seg_nins,
                                                              b.seg_ndel, b.seg_end);
 }
@@ -521,11 +533,7 @@ void store_rel_delta(uint32_t m, const unsigned long long *keys, KeyLayout kl, c
     if (m) k_rel_delta<<<(m + 255) / 256, 256, 0, s>>>(m, keys, kl, b.eff, delta);
 }
 
-void store_touched(uint32_t m, const unsigned long long *keys, KeyLayout kl, uint32_t *bits, uint32_t words,
-                   cudaStream_t s) {
-    cudaMemsetAsync(bits, 0, sizeof(uint32_t) * words, s);
-    if (m) k_touched<<<(m + 255) / 256, 256, 0, s>>>(m, keys, kl, bits, words);
-}
+void store_read_back(const BatchResult &r, cudaStream_t s) { k_read_back<<<1, 256, 0, s>>>(r); }
 
 void store_rel_sizes(const DeviceGraph &g, unsigned long long *out, cudaStream_t s) {
     k_rel_sizes<<<grid_for((size_t)g.V * g.R, 256), 256, 0, s>>>(g.V, g.R, g.meta, out);

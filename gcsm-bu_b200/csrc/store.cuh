@@ -60,13 +60,36 @@ struct BatchScratch {
     unsigned int *error = nullptr;    // [1]
 };
 
+// What a batch starts from zero: cleared by the kernel that builds its keys.
+struct BatchReset {
+    unsigned int *nheads = nullptr, *error = nullptr;
+    unsigned long long *counters = nullptr;  // [2]
+    unsigned long long *counts = nullptr;    // [ncounts] matches per plan and phase
+    uint32_t ncounts = 0;
+    uint32_t *touched = nullptr;             // [words] bit per vertex owning a list that a batch key belongs to
+    uint32_t words = 0;
+};
+
+// What the host reads of a batch, written to its (pinned) memory by one kernel.
+struct BatchResult {
+    const unsigned long long *counts = nullptr;  // [ncounts]
+    uint32_t ncounts = 0;
+    const unsigned long long *counters = nullptr, *pool_top = nullptr;
+    const unsigned int *error = nullptr;
+    const EnumControl *ctrl = nullptr;           // of the last phase, or nullptr
+    unsigned long long *h_counts = nullptr;      // counts, counters, pool top, error
+    EnumControl *h_ctrl = nullptr;
+};
+void store_read_back(const BatchResult &r, cudaStream_t s);
+
 void store_build_keys(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elab, const uint8_t *isdel,
                       const LabelTables &lt, const DeviceGraph &g, KeyLayout kl, unsigned long long *keys,
-                      cudaStream_t s);
+                      const BatchReset &reset, cudaStream_t s);
 cudaError_t store_sort_keys(void *temp, size_t &temp_bytes, const unsigned long long *in, unsigned long long *out,
                             uint32_t m, KeyLayout kl, cudaStream_t s);
+// Also sets the bits of `touched` (cleared with the keys).
 void store_classify(uint32_t m, const unsigned long long *keys, KeyLayout kl, DeviceGraph &g, BatchScratch &b,
-                    cudaStream_t s);
+                    uint32_t *touched, uint32_t words, cudaStream_t s);
 void store_delete(uint32_t m, const unsigned long long *keys, KeyLayout kl, DeviceGraph &g, BatchScratch &b,
                   cudaStream_t s);
 void store_insert(uint32_t m, const unsigned long long *keys, KeyLayout kl, DeviceGraph &g, BatchScratch &b,
@@ -79,9 +102,6 @@ void store_nlf_all(DeviceGraph &g, const NlfTables &nt, cudaStream_t s);
 // Per-relation net entry change of a classified batch (delta[R], accumulated).
 void store_rel_delta(uint32_t m, const unsigned long long *keys, KeyLayout kl, const BatchScratch &b, long long *delta,
                      cudaStream_t s);
-// Bit per vertex owning a list that a batch key belongs to (bits[words], cleared first).
-void store_touched(uint32_t m, const unsigned long long *keys, KeyLayout kl, uint32_t *bits, uint32_t words,
-                   cudaStream_t s);
 // Per-relation entry counts (out[R], accumulated).
 void store_rel_sizes(const DeviceGraph &g, unsigned long long *out, cudaStream_t s);
 void store_edge_stats(DeviceGraph &g, uint32_t rel, const uint32_t *bits_u, const uint32_t *bits_uu,

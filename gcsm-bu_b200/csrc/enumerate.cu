@@ -1051,7 +1051,7 @@ __device__ int take_ticket(WarpState &S, const EnumParams &P, const WorkItem *fr
 
 __device__ void write_row(const EnumParams &P, const DevPlan *pl, const WarpState &S, uint32_t d, uint32_t w,
                           unsigned long long r) {
-    uint32_t *row = P.rows + r * CSM_ROW_WORDS;
+    uint32_t *row = P.rows + r * P.row_words;
     row[0] = pl->query;
     for (uint32_t k = 0; k < d; k++) row[1 + pl->order[k]] = S.f[k];
     row[1 + pl->order[d]] = w;
@@ -1723,7 +1723,7 @@ __device__ unsigned long long run_item(WarpState &S, const EnumParams &P, uint32
                 } else if (ok) {
                     if (d == 1) {
                         const unsigned long long key = __ldg(P.keys + cand);
-                        uint32_t *row = P.rows + (r + rank) * CSM_ROW_WORDS;
+                        uint32_t *row = P.rows + (r + rank) * P.row_words;
                         row[0] = pl->query;
                         row[1 + pl->order[0]] = P.kl.src(key);
                         row[1 + pl->order[1]] = P.kl.dst(key);

@@ -101,7 +101,8 @@ struct EnumParams {
     EnumControl *ctrl;
     unsigned long long *counts;      // per plan
     uint32_t mode;                   // 0 count, 1 materialize, 2 expand one level
-    uint32_t *rows;                  // materialize: rows of 1 + CSM_MAXQV words
+    uint32_t *rows;                  // materialize: rows of row_words words
+    uint32_t row_words;              // query id and a word per vertex of the largest query
     unsigned long long row_cap;
     uint32_t donate;
     uint32_t steal_min;

@@ -589,7 +589,8 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
                     tail_start = (int)n;
                 // A last vertex with two or three lists, one of them the vertex's before it, is one such
                 // intersection per candidate of the level above (without that neighbour the shared
-                // last level counts it once for all of them).
+                // last level counts it once for all of them): four queries at 16,411 updates 56 -> 40 ms,
+                // 1024 updates with a captured graph 0.81 -> 0.60 ms.
                 if (tail_start == (int)n && n >= 4 && q.adjacent(a, b) && (q.degree(b) == 2 || q.degree(b) == 3))
                     tail_start = (int)n - 1;
             }
@@ -614,6 +615,8 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
 // apart.  Another query vertex x of the leaf's label can be matched to the far end of one of those
 // edges unless x hangs off the inner endpoint by an edge of the same relation that must be no batch
 // edge; where some x can, the leaf is counted in the tail, whose polynomial handles the overlap.
+// On hubs the plain form repeats the whole query for dozens of batch edges (65,536 updates: dense query
+// 234 -> 50 ms, tree query 292 -> 113 ms).
 bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp) {
     const int i = hp.dev.qe;
     const uint32_t n = (uint32_t)hp.order.size();

@@ -441,7 +441,8 @@ __global__ void k_rel_delta(uint32_t m, const unsigned long long *keys, KeyLayou
         atomicAdd(reinterpret_cast<unsigned long long *>(delta + rel), (unsigned long long)(long long)sum);  // two's complement
 }
 
-// The batch's results, straight to the host's memory: one launch instead of a copy each.
+// The batch's results, straight to the host's memory: one launch instead of a copy each (with the memsets
+// that k_build_keys took over, 64 updates and their inverse 0.47 -> 0.40 ms).
 __global__ void k_read_back(BatchResult r) {
     for (uint32_t i = threadIdx.x; i < r.ncounts; i += blockDim.x) r.h_counts[i] = r.counts[i];
     if (threadIdx.x < 2) r.h_counts[r.ncounts + threadIdx.x] = r.counters[threadIdx.x];

@@ -1171,6 +1171,9 @@ csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *ds
     const uint32_t m = (uint32_t)(2 * n);
     const uint32_t np = (uint32_t)plans_.size();
     rows_valid_ = false;
+    // A phase that the batch does not run leaves no rows (the vectors keep their memory).
+    for (auto &phase : last_rows_)
+        for (auto &rows : phase) rows.clear();
     phase_ran_[0] = phase_ran_[1] = false;
     last_frontier_rows_ = 0;
     deferred_ = CSM_OK;

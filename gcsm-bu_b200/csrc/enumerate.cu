@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "window.h"
 
 namespace csm {
 
@@ -139,12 +140,11 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t *L, uint32_t
     return lo + __popc(__ballot_sync(0xffffffffu, v < key2));
 }
 
-// First window of a search below: about twice what 32 consecutive entries of a list of `short_size` span
-// in one of `size`, a power of two of at least 64.
-__device__ __forceinline__ uint32_t first_window(uint32_t size, uint32_t short_size) {
-    const uint32_t per = short_size ? size / short_size : 0u;
-    return 64u << (per ? 31 - __clz(per) : 0);
-}
+// Entries of a list in device memory (window.h).
+struct ListReader {
+    const uint32_t *L;
+    __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return __ldg(L + i); }
+};
 
 // Entry of the sorted list L that names this lane's vertex (key = vertex << 1), or 0xFFFFFFFF.  The
 // lanes' keys ascend, `top` is the one of lane `last` and the largest; c0 is a position no lane's
@@ -155,14 +155,8 @@ __device__ __forceinline__ uint32_t first_window(uint32_t size, uint32_t short_s
 // and a warp search (four queries at 16,411 updates 39.6 -> 34.1 ms, 1M on 43M edges 55.8 -> 52.1 ms).
 __device__ __forceinline__ uint32_t window_find(const uint32_t *L, uint32_t size, uint32_t &c0, uint32_t w0, uint32_t key,
                                                 uint32_t top, uint32_t last) {
-    uint32_t w = w0;
-    while (c0 + w < size && __ldg(L + c0 + w - 1u) < top) w <<= 1;
-    uint32_t pos = c0;
-    for (uint32_t s = w >> 1; s; s >>= 1) {
-        const uint32_t p = pos + s - 1u;
-        const uint32_t v = p < size ? __ldg(L + p) : 0xFFFFFFFFu;
-        if (v < key) pos += s;
-    }
+    const ListReader r{L};
+    const uint32_t pos = window_lower_bound(r, size, c0, window_for(r, size, c0, w0, top), key);
     const uint32_t e = pos < size ? __ldg(L + pos) : 0xFFFFFFFFu;
     c0 = __shfl_sync(0xffffffffu, pos, last);
     return (e & ~1u) == key ? e : 0xFFFFFFFFu;

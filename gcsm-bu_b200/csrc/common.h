@@ -15,6 +15,13 @@
 
 #include <stdint.h>
 
+// Small functions that the kernels and the CPU tests share.
+#ifdef __CUDACC__
+#define CSM_HD __host__ __device__ __forceinline__
+#else
+#define CSM_HD inline
+#endif
+
 #define CSM_MAXQV 16
 #define CSM_MAXQE 42
 #define CSM_MAXBN 15
@@ -193,7 +200,8 @@ struct WorkItem {
 // of position p may write the slot once its word reads (epoch, p) — or, in the first lap, any
 // older epoch — and publishes with (epoch, p + 1); the consumer of p releases the slot with
 // (epoch, p + qcap).  (epoch, CSM_QUEUE_OVER) tells the waiting warps that nothing is left.
-// Slots are reused for the whole launch and no position is ever skipped.
+// Slots are reused for the whole launch and no position is ever skipped.  A waiting warp that runs
+// out of patience closes the ring (ring.h): no position is given an item any more, and it leaves.
 //
 // The counters that many warps touch at once lie in 128-byte lines of their own, so that traffic
 // on one does not queue behind the others.
@@ -211,7 +219,7 @@ struct alignas(128) EnumControl {
     unsigned int blocks_done;         // blocks of the deciding launch that have finished
     unsigned int pair_phase;          // phase number of the engine's pair table (1 .. CSM_PAIR_PHASES)
     unsigned long long max_front;     // largest frontier of the phase
-    alignas(128) unsigned int q_head; // donation positions reserved (8-byte aligned pair with q_tail)
+    alignas(128) unsigned int q_head; // donation positions reserved, CSM_QUEUE_CLOSED (8-byte aligned pair with q_tail)
     unsigned int q_tail;              // donation positions taken by warps out of work
     alignas(128) unsigned int active; // warps holding work, and items in the ring
     alignas(128)
@@ -238,10 +246,11 @@ struct alignas(128) EnumControl {
 #define CSM_QUEUE_POS_LIMIT 0x7FFFFFFFu
 #define CSM_QUEUE_MIN_SLOTS 32u
 #define CSM_QUEUE_OVER 0xFFFFFFFFu
+#define CSM_QUEUE_CLOSED 0x80000000u  // bit of q_head: no further position is reserved
 
 #define CSM_ERRBIT_TIMEOUT 1u  // the launch ran past its time limit and stopped early
 #define CSM_ERRBIT_OUTPUT 2u
 #define CSM_ERRBIT_POOL 8u
-#define CSM_ERRBIT_IDLE 4u     // a warp out of work waited past its bound (with CSM_ERRBIT_TIMEOUT)
+#define CSM_ERRBIT_IDLE 4u     // an item reserved for a waiting warp never came (with CSM_ERRBIT_TIMEOUT)
 #define CSM_ERRBIT_FRONTIER 32u  // a semi-BFS level outgrew its frontier buffer
 #define CSM_ERRBIT_CORRUPT 16u  // a consistency check failed (see EnumControl.bad_*)

@@ -1271,7 +1271,7 @@ csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *ds
         // batch (the update kernels do not depend on the counts), so only the counts are short.
         if ((c.error & CSM_ERRBIT_TIMEOUT) && deferred_ == CSM_OK)
             deferred_ = fail(CSM_ERR_TIMEOUT, c.error & CSM_ERRBIT_IDLE
-                                                  ? "a warp of the enumeration waited for work past its bound: this "
+                                                  ? "a work item handed to a warp of the enumeration never came: this "
                                                     "batch's counts are incomplete; the graph holds the whole batch"
                                                   : "the enumeration ran past its time limit (time_limit_us): this batch's "
                                                     "counts are incomplete; the graph holds the whole batch");
@@ -1337,7 +1337,7 @@ csm_status Engine::enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s) {
     P.counts = d_counts_ + (phase == CSM_PHASE_INS ? np : 0);
     P.steal_min = lc_.steal_chunk;
     // A warp out of work is told when nothing is left; the bound (minutes of polling about once a
-    // microsecond) only ends the wait if that never happens, and the launch then reports it.
+    // microsecond without an item being handed out) lets it go before that.
     P.idle_limit = 1u << 28;
     P.time_limit_ns = time_limit_us_ * 1000ull;
     P.abort_flag = phase == CSM_PHASE_INS ? bs_.error : nullptr;

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "ring.h"
 #include "window.h"
 
 namespace csm {
@@ -794,13 +795,12 @@ __device__ bool item_ok(const WarpState &S, const EnumParams &P, uint32_t where,
 
 // Warps that wait at the ring for an item (for every lane).  One 8-byte read of both ring counters.
 __device__ __forceinline__ uint32_t items_wanted(const EnumParams &P) {
-    int32_t n = 0;
+    uint32_t n = 0;
     if (lane_id() == 0) {
         const unsigned long long w = *(volatile unsigned long long *)&P.ctrl->q_head;
-        n = (int32_t)((uint32_t)(w >> 32) - (uint32_t)w);
+        n = ring_wanted((uint32_t)w, (uint32_t)(w >> 32));
     }
-    n = __shfl_sync(0xffffffffu, n, 0);
-    return n > 0 ? (uint32_t)n : 0u;
+    return __shfl_sync(0xffffffffu, n, 0);
 }
 
 // Reserves `cnt` (1..32) consecutive ring positions while a warp waits for one; returns the first,
@@ -815,7 +815,7 @@ __device__ uint32_t reserve_slots(const EnumParams &P, uint32_t cnt) {
     if (lane == 0) w = *(volatile unsigned long long *)&P.ctrl->q_head;
     w = __shfl_sync(0xffffffffu, w, 0);
     const uint32_t pos = (uint32_t)w;
-    if ((int32_t)((uint32_t)(w >> 32) - pos) <= 0) return 0xFFFFFFFFu;
+    if (!ring_wanted(pos, (uint32_t)(w >> 32))) return 0xFFFFFFFFu;
     const uint32_t p = pos + lane;
     bool free_slot = pos <= CSM_QUEUE_POS_LIMIT - cnt;
     if (free_slot && lane < cnt && p > P.qmask)
@@ -928,15 +928,15 @@ __device__ void try_donate(WarpState &S, const EnumParams &P, const DevPlan *pl,
 // slots of all waiting positions get the stamp that says so.
 __device__ void release_waiting(const EnumParams &P) {
     const unsigned long long w = *(volatile unsigned long long *)&P.ctrl->q_head;
-    const uint32_t head = (uint32_t)w, waiting = (uint32_t)(w >> 32) - head;
+    const uint32_t head = (uint32_t)w & ~CSM_QUEUE_CLOSED, waiting = ring_unserved(head, (uint32_t)(w >> 32));
     const uint32_t n = waiting < P.qmask + 1u ? waiting : P.qmask + 1u;
     const unsigned long long over = slot_stamp(P.ctrl->epoch, CSM_QUEUE_OVER);
     for (uint32_t i = lane_id(); i < n; i += 32) *(volatile unsigned long long *)(P.seq + ((head + i) & P.qmask)) = over;
 }
 
 // An idle warp takes the next ring position as its own and waits for that position's item: 1 = item
-// copied into S, 0 = the launch is over (or its time limit has passed, err), -1 = an item that
-// failed its check.  Every waiting warp polls a word of its own slot, so thousands of waiting warps
+// copied into S, 0 = the launch is over for this warp (or its time limit has passed, err), -1 = an item
+// that failed its check.  Every waiting warp polls a word of its own slot, so thousands of waiting warps
 // do not crowd the counters the working ones need.  With all of them polling the shared counters, and
 // taking back a shared request count by compare-and-swap on leaving, a launch over a handful of items
 // took 270 us (4,736 warps queueing on one address); it takes 13-22 us now, and the launches where
@@ -959,18 +959,25 @@ __device__ int await_item(WarpState &S, const EnumParams &P, unsigned int &err, 
     if (lane == 0) {
         volatile unsigned long long *seq = P.seq + (pos & P.qmask);
         uint32_t ns = 64, polls = 0, head = 0;
+        bool closed = false;
         while (got == 0) {
             const unsigned long long w = *seq;
             if (w == slot_stamp(ep, pos + 1)) got = 1;
             else if (w == slot_stamp(ep, CSM_QUEUE_OVER)) got = 2;
             else if (deadline && device_ns() > deadline) got = 3;
-            else if (++polls >= P.idle_limit) got = 4;
-            else __nanosleep(ns);
+            else if (++polls >= P.idle_limit) {
+                // Nothing was handed out for the whole bound (some warp has a long piece of work that
+                // cannot be split).  No position gets an item from here on, so this warp can go.
+                if (ring_may_leave(atomicOr(&P.ctrl->q_head, CSM_QUEUE_CLOSED), pos)) got = 2;
+                else if (closed) got = 4;
+                closed = true;
+                polls = 0;
+            } else __nanosleep(ns);
             if (ns < 1024) ns <<= 1;
             if (got == 0 && (polls & 255u) == 0) {
                 // Seldom: whether anything holds work, and whether it is still being handed out (the
                 // bound is on waiting without a sign of progress).
-                const uint32_t h = *(volatile unsigned int *)&P.ctrl->q_head;
+                const uint32_t h = *(volatile unsigned int *)&P.ctrl->q_head & ~CSM_QUEUE_CLOSED;
                 if (*(volatile unsigned int *)&P.ctrl->active == 0) got = 2;
                 if (h != head) polls = 0;
                 head = h;

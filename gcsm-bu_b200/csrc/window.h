@@ -6,11 +6,7 @@
 
 #include <stdint.h>
 
-#ifdef __CUDACC__
-#define CSM_HD __host__ __device__ __forceinline__
-#else
-#define CSM_HD inline
-#endif
+#include "common.h"
 
 namespace csm {
 

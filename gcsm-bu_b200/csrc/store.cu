@@ -483,7 +483,10 @@ inline int grid_for(size_t n, int block) {
 void store_build_keys(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elab, const uint8_t *isdel,
                       const LabelTables &lt, const DeviceGraph &g, KeyLayout kl, unsigned long long *keys,
                       const BatchReset &reset, cudaStream_t s) {
-    k_build_keys<<<grid_for(n, 256), 256, 0, s>>>(n, src, dst, elab, isdel, g.V, g.vlab, lt.elab_raw, lt.nel,
+    // Threads for the updates or for the words to clear, whichever are more: with one block for both, 64
+    // updates and their inverse on 100M vertices took 0.74 ms instead of 0.28.
+    const size_t threads = n > reset.words ? n : reset.words;
+    k_build_keys<<<grid_for(threads, 256), 256, 0, s>>>(n, src, dst, elab, isdel, g.V, g.vlab, lt.elab_raw, lt.nel,
                                                   lt.rel_table, lt.nvl, kl, keys, reset);
 }
 

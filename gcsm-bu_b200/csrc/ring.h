@@ -5,15 +5,14 @@
 
 namespace csm {
 
-// Positions taken by waiting warps that no item has been reserved for.
-CSM_HD uint32_t ring_unserved(uint32_t head, uint32_t tail) {
-    const int32_t n = (int32_t)(tail - (head & ~CSM_QUEUE_CLOSED));
-    return n > 0 ? (uint32_t)n : 0u;
-}
+// Warps that an item may be handed to, as a signed number: not above zero when none waits.  The closing bit
+// of the head takes 2^31 off, so a closed ring needs no test of its own.
+CSM_HD int32_t ring_wanted(uint32_t head, uint32_t tail) { return (int32_t)(tail - head); }
 
-// Warps that an item may be handed to.
-CSM_HD uint32_t ring_wanted(uint32_t head, uint32_t tail) {
-    return head & CSM_QUEUE_CLOSED ? 0u : ring_unserved(head, tail);
+// Positions taken by waiting warps that no item has been reserved for, in a closed ring too.
+CSM_HD uint32_t ring_unserved(uint32_t head, uint32_t tail) {
+    const int32_t n = ring_wanted(head & ~CSM_QUEUE_CLOSED, tail);
+    return n > 0 ? (uint32_t)n : 0u;
 }
 
 // Whether a warp that waits at `pos` may leave without an item, having closed the ring when its head was

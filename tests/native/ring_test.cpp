@@ -28,7 +28,7 @@ struct Launch {
 
 bool hand_out(Launch &L, uint32_t pieces) {
     const uint32_t pos = L.head.load(), tail = L.tail.load();
-    if (!csm::ring_wanted(pos, tail)) return false;
+    if (csm::ring_wanted(pos, tail) <= 0) return false;
     if (pos >= kSlots && L.seq[pos % kSlots].load() != pos) return false;
     uint32_t expect = pos;
     if (!L.head.compare_exchange_strong(expect, pos + 1)) return false;
@@ -104,7 +104,7 @@ int main() {
     for (uint32_t h : {0u, 1u, 1000u, 0x7FFFFFFFu})
         for (uint32_t n : {0u, 1u, 5000u}) {
             const uint32_t t = h + n;
-            if (csm::ring_wanted(h, t) != n || csm::ring_wanted(h | CSM_QUEUE_CLOSED, t) != 0 ||
+            if (csm::ring_wanted(h, t) != (int32_t)n || csm::ring_wanted(h | CSM_QUEUE_CLOSED, t) > 0 ||
                 csm::ring_unserved(h | CSM_QUEUE_CLOSED, t) != n || !csm::ring_may_leave(h, h) ||
                 csm::ring_may_leave(h | CSM_QUEUE_CLOSED, h - 1)) {
                 std::printf("FAIL counters %u %u\n", h, n);

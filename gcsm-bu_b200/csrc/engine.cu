@@ -1120,12 +1120,15 @@ csm_status Engine::enqueue_readback(cudaStream_t s) {
 // Replays the batch's device work from a CUDA graph captured for this batch size and launch
 // configuration (captured on first use; any reallocation of engine buffers starts a new one).
 csm_status Engine::launch_graph(uint64_t n, bool has_delete, cudaStream_t s) {
-    GraphKey key{n, has_delete, graph_gen_, lc_.strategy, lc_.steal_chunk, lc_.warps_per_block, lc_.occupancy, blocks_};
+    const GraphKey key{n,   has_delete,    graph_gen_, lc_.strategy, lc_.steal_chunk, lc_.warps_per_block, lc_.occupancy, blocks_,
+                       sc_};
     GraphEntry *hit = nullptr;
     for (auto &g : graphs_)
         if (g.key == key) hit = &g;
     if (!hit) {
-        if (graphs_.size() >= 8) clear_graphs();
+        size_t same = 0;
+        for (auto &g : graphs_) same += g.key.scratch == key.scratch;
+        if (same >= kGraphsPerScratch || graphs_.size() >= kGraphs) clear_graphs();
         const Stats0 before{stats_.kernel_launches, stats_.enum_launches};
         CSM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
         capturing_ = true;

@@ -27,6 +27,10 @@ struct EnumScratch {
     uint32_t qcap = 0;                  // ring slots (a power of two, >= CSM_QUEUE_MIN_SLOTS)
     uint32_t *seed_lo = nullptr;
     uint32_t *ticket_prefix = nullptr;
+    bool operator==(const EnumScratch &o) const {
+        return ctrl == o.ctrl && queue == o.queue && seq == o.seq && qcap == o.qcap && seed_lo == o.seed_lo &&
+               ticket_prefix == o.ticket_prefix;
+    }
 };
 
 // Resources lent to the engine for one batch: enumeration scratch, two semi-BFS frontier
@@ -211,7 +215,8 @@ class Engine {
     uint32_t *d_memo_desc_ = nullptr;         // per table: representative plan, slot, tail values' slot
     uint32_t memo_tables_ = 0;                // pendant tables filled each phase
     unsigned long long last_frontier_rows_ = 0;
-    // CUDA graphs of whole batches (depth-first strategies), keyed by what the capture bakes in.
+    // CUDA graphs of whole batches (depth-first strategies), keyed by what the capture bakes in: a tenant
+    // of the serving loop runs on the scratch of whichever slot takes its request.
     struct GraphKey {
         uint64_t n;
         bool del;
@@ -219,11 +224,13 @@ class Engine {
         int strategy;
         uint32_t steal;
         int wpb, occ, blocks;
+        EnumScratch scratch;
         bool operator==(const GraphKey &o) const {
             return n == o.n && del == o.del && gen == o.gen && strategy == o.strategy && steal == o.steal &&
-                   wpb == o.wpb && occ == o.occ && blocks == o.blocks;
+                   wpb == o.wpb && occ == o.occ && blocks == o.blocks && scratch == o.scratch;
         }
     };
+    static constexpr size_t kGraphsPerScratch = 8, kGraphs = 64;
     struct GraphEntry {
         GraphKey key{};
         cudaGraphExec_t exec = nullptr;

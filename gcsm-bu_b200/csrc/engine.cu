@@ -1121,7 +1121,7 @@ csm_status Engine::enqueue_readback(cudaStream_t s) {
 // configuration (captured on first use; any reallocation of engine buffers starts a new one).
 csm_status Engine::launch_graph(uint64_t n, bool has_delete, cudaStream_t s) {
     const GraphKey key{n,   has_delete,    graph_gen_, lc_.strategy, lc_.steal_chunk, lc_.warps_per_block, lc_.occupancy, blocks_,
-                       sc_};
+                       sc_, time_limit_us_};
     GraphEntry *hit = nullptr;
     for (auto &g : graphs_)
         if (g.key == key) hit = &g;

@@ -225,9 +225,10 @@ class Engine {
         uint32_t steal;
         int wpb, occ, blocks;
         EnumScratch scratch;
+        uint64_t limit_us;
         bool operator==(const GraphKey &o) const {
             return n == o.n && del == o.del && gen == o.gen && strategy == o.strategy && steal == o.steal &&
-                   wpb == o.wpb && occ == o.occ && blocks == o.blocks && scratch == o.scratch;
+                   wpb == o.wpb && occ == o.occ && blocks == o.blocks && scratch == o.scratch && limit_us == o.limit_us;
         }
     };
     static constexpr size_t kGraphsPerScratch = 8, kGraphs = 64;

@@ -1,4 +1,4 @@
-"""GPU tests of what a captured graph bakes in: the scratch of the slot it was captured on."""
+"""GPU tests of what a captured graph bakes in: the scratch of the slot it was captured on, and the time limit."""
 import numpy as np
 import pytest
 
@@ -8,6 +8,30 @@ from helpers import small_workload
 from oracle import Oracle
 
 pytestmark = pytest.mark.gpu
+
+
+def test_time_limit_set_after_the_capture():
+    w = small_workload("c2", scale=0.05, nqueries=2)
+    eng = csm.Engine(search_strategy=0, cuda_graphs=1)
+    oracles = []
+    for q in w.queries:
+        eng.load_query(q)
+        oracles.append(Oracle(q, w.data))
+    eng.load_graph(w.data)
+    a, b = w.batches[0], w.batches[1]
+    n = min(len(a.src), len(b.src))
+    cut = [Batch(x.src[:n], x.dst[:n], x.elabels[:n], x.is_delete[:n]) for x in (a, b, a, b)]
+    for i, x in enumerate(cut):
+        eng.set_time_limit(1 if i in (1, 2) else 0)
+        rc, res = eng.apply_partial(x)
+        full = [o.apply(x) for o in oracles]
+        if i in (1, 2):
+            assert rc == -4, "a 1-microsecond limit must stop the replayed launch"
+        else:
+            assert rc == 0
+            assert [(r.positive, r.negative) for r in res] == [(f["pos"], f["neg"]) for f in full]
+    assert eng.stats().graph_launches == len(cut)
+    eng.close()
 
 
 def test_tenants_with_graphs_move_between_slots():

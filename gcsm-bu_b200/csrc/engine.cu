@@ -76,16 +76,19 @@ csm_status Engine::cuda_fail(cudaError_t e, const char *where) {
         if (e__ != cudaSuccess) return cuda_fail(e__, #call); \
     } while (0)
 
+// Persistent launch: never more blocks than can be resident at once.  Warps that run out of work
+// wait for the others while any warp holds work, so a block that could only start after resident
+// blocks exit would stall the launch until the idle bound runs out.
+int Engine::grid_blocks(const LaunchConfig &c) const {
+    const int resident = enum_blocks_per_sm(c.warps_per_block, c.occupancy);
+    return sm_count_ * (cfg_.blocks_per_sm > 0 && cfg_.blocks_per_sm < resident ? cfg_.blocks_per_sm : resident);
+}
+
 void Engine::set_launch_config(const LaunchConfig &c) {
-    // Persistent launch: never more blocks than can be resident at once.  Warps that run out
-    // of work wait for the others while any warp holds work, so a block that could only start
-    // after resident blocks exit would stall the launch until the idle bound runs out.
     lc_ = c;
     warps_per_block_ = c.warps_per_block;
     occupancy_ = c.occupancy;
-    const int resident = enum_blocks_per_sm(warps_per_block_, occupancy_);
-    const int bps = cfg_.blocks_per_sm > 0 && cfg_.blocks_per_sm < resident ? cfg_.blocks_per_sm : resident;
-    blocks_ = sm_count_ * bps;
+    blocks_ = grid_blocks(c);
     stats_.tuned_strategy = (uint64_t)c.strategy;
     stats_.tuned_steal_chunk = c.steal_chunk;
     stats_.tuned_warps_per_block = (uint64_t)c.warps_per_block;
@@ -633,11 +636,9 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
 
 // Signatures of the tails' pair masks, shared by all plans, and the table of their counts.
 csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
-    // 4M entries (64 MB) stay in the L2 cache; like the pendant tables they take a quarter of the
-    // free memory at most.
-    constexpr uint32_t kPairSlots = 1u << 22;
     std::vector<std::pair<uint32_t, uint32_t>> sigs;
     bool used = false;
+    uint32_t nsets = 0;  // most kept sets of a plan
     for (HostPlan &hp : plans) {
         DevTail &t = hp.dev.tail;
         const int level = hp.dev.tail_start - 1;  // the counting level
@@ -680,20 +681,37 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
         }
         t.pair_par = all ? 1 : 0;
         used = used || all;
+        if (all) nsets = std::max(nsets, (uint32_t)sets);
     }
-    // One kept-set area per warp: no launch has more than 64 warps on an SM.
-    const size_t set_entries = (size_t)sm_count_ * 64 * CSM_SETS * CSM_SET_CAP;
-    if (used && !d_pairs_) {
+    // A kept-set area per set and warp of the largest grid that any launch configuration has.  Like the
+    // pendant tables these take a quarter of the free memory at most.
+    uint64_t warps = enum_warps();
+    for (const LaunchConfig &c : tune_cands_)
+        warps = std::max<uint64_t>(warps, (uint64_t)grid_blocks(c) * (uint64_t)c.warps_per_block);
+    const size_t set_entries = (size_t)warps * nsets * CSM_SET_CAP;
+    if (used && (!d_pairs_ || set_entries > set_entries_)) {
         size_t free_b = 0, total_b = 0;
-        const size_t want = sizeof(uint4) * (size_t)kPairSlots + sizeof(uint32_t) * set_entries;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 4 &&
-            (d_sets_ || dev_alloc(&d_sets_, set_entries) == cudaSuccess) &&
-            (d_pair_phase_ || dev_alloc(&d_pair_phase_, 1) == cudaSuccess) &&
-            dev_alloc(&d_pairs_, kPairSlots) == cudaSuccess) {
-            pair_slots_ = kPairSlots;
-            pair_phases_ = CSM_PAIR_PHASES;  // cleared before the first batch
-        } else {
+        const uint32_t slots = d_pairs_ ? 0u : pair_slots_wanted();
+        const size_t want = sizeof(uint4) * (size_t)slots + sizeof(uint32_t) * set_entries;
+        bool ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 4;
+        if (ok && set_entries > set_entries_) {
+            if (d_sets_) cudaFree(d_sets_);
+            d_sets_ = nullptr;
+            set_entries_ = 0;
+            ok = dev_alloc(&d_sets_, set_entries) == cudaSuccess;
+            if (ok) set_entries_ = set_entries;
+        }
+        ok = ok && (d_pair_phase_ || dev_alloc(&d_pair_phase_, 1) == cudaSuccess);
+        if (ok && !d_pairs_) {
+            ok = dev_alloc(&d_pairs_, slots) == cudaSuccess;
+            if (ok) {
+                pair_slots_ = slots;
+                pair_phases_ = CSM_PAIR_PHASES;  // cleared before the first batch
+            }
+        }
+        if (!ok) {
             (void)cudaGetLastError();
+            if (d_pairs_) cudaFree(d_pairs_);
             d_pairs_ = nullptr;
         }
     }
@@ -702,6 +720,24 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
             hp.dev.tail.pair_par = 0;
             if (hp.dev.memo_cut && hp.dev.memo_slot < CSM_MEMO_PENDING) hp.dev.memo_slot = CSM_MEMO_PENDING;
         }
+    return CSM_OK;
+}
+
+// A slot of the pair table for 16 to 8 entries of the adjacency pool, so the table of an engine over a
+// small graph stays small (a thousand tenants have one each), and at most 4M slots: 64 MB stay in the
+// L2 cache.  With 2M pool entries (10,000 vertices, 50,000 edges) 2 MB instead of 64: 1024 updates with a
+// captured graph 0.46 ms with either.
+uint32_t Engine::pair_slots_wanted() const {
+    uint32_t slots = 1u << 14;
+    while (slots < (1u << 22) && 16ull * slots < g_.pool_cap) slots <<= 1;
+    return slots;
+}
+
+// Starts the pair table over: entries carry the number of their phase, counted from here.
+csm_status Engine::clear_pairs(cudaStream_t s) {
+    CSM_CUDA(cudaMemsetAsync(d_pairs_, 0, sizeof(uint4) * (size_t)pair_slots_, s));
+    CSM_CUDA(cudaMemsetAsync(d_pair_phase_, 0, sizeof(unsigned int), s));
+    pair_phases_ = 0;
     return CSM_OK;
 }
 
@@ -1182,10 +1218,9 @@ csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *ds
     deferred_ = CSM_OK;
     NlfTables nt{d_spec_begin_, d_specs_, d_bits_, words_};
     if (d_pairs_ && pair_phases_ + 64 > CSM_PAIR_PHASES) {
-        // Entries carry the number of their phase; before the numbers run out the table starts over.
-        CSM_CUDA(cudaMemsetAsync(d_pairs_, 0, sizeof(uint4) * (size_t)pair_slots_, s));
-        CSM_CUDA(cudaMemsetAsync(d_pair_phase_, 0, sizeof(unsigned int), s));
-        pair_phases_ = 0;
+        // Before the phase numbers run out the table starts over.
+        const csm_status pst = clear_pairs(s);
+        if (pst != CSM_OK) return pst;
     }
     pair_phases_ += 2 * (tune_left_ > 0 ? tune_cands_.size() + 1 : 2);  // the batch's phases, a rerun's too
     const bool tuning = tune_left_ > 0 && !no_alloc_ && cfg_.materialize_rows == 0;
@@ -1472,6 +1507,20 @@ csm_status Engine::maybe_compact(cudaStream_t s) {
     stats_.pool_used = total;
     stats_.pool_capacity = want;
     stats_.compactions++;
+    if (d_pairs_ && pair_slots_wanted() > pair_slots_) {
+        // The pair table grows with the pool; without memory for that it stays as it is.
+        const uint32_t slots = pair_slots_wanted();
+        uint4 *pairs = nullptr;
+        if (dev_alloc(&pairs, slots) == cudaSuccess) {
+            cudaFree(d_pairs_);
+            d_pairs_ = pairs;
+            pair_slots_ = slots;
+            const csm_status st = clear_pairs(s);
+            if (st != CSM_OK) poisoned_ = true;
+            return st;
+        }
+        cudaGetLastError();
+    }
     return CSM_OK;
 }
 

@@ -264,6 +264,8 @@ class Engine {
     csm_status compute_edge_stats(std::vector<EdgeStats> &stats);
     csm_status install_plans(const std::vector<EdgeStats> &stats);
     csm_status install_pairs(std::vector<HostPlan> &plans);
+    uint32_t pair_slots_wanted() const;
+    csm_status clear_pairs(cudaStream_t s);
     csm_status maybe_replan();
     size_t terms_cap_ = 0;
     long long *d_rel_delta_ = nullptr;      // [R] net entry change of the current batch
@@ -293,7 +295,8 @@ class Engine {
     uint4 *d_pairs_ = nullptr;                // pair table, null when no plan uses it
     unsigned int *d_pair_phase_ = nullptr;    // phases it has seen, counted on the device
     uint32_t pair_slots_ = 0;
-    uint32_t *d_sets_ = nullptr;              // kept intersections, CSM_SETS per warp of the largest grid
+    uint32_t *d_sets_ = nullptr;              // kept intersections: sets of the plans * warps of the largest grid
+    size_t set_entries_ = 0;
     uint64_t pair_phases_ = 0;                // the same, an upper bound kept by the host
     int expand_levels_ = 0;                   // most breadth-first levels any plan expands
     LaunchConfig lc_{};                       // configuration in use
@@ -303,6 +306,7 @@ class Engine {
     bool tuned_this_batch_ = false;
     cudaEvent_t tune_ev_[32] = {};
     void set_launch_config(const LaunchConfig &c);
+    int grid_blocks(const LaunchConfig &c) const;
 
     // Results of the last batch.
     std::vector<uint64_t> last_counts_;   // 2 * nplans

@@ -489,7 +489,7 @@ __device__ uint32_t set_size(WarpState &S, const EnumParams &P, const DevTail *T
     const uint32_t set = __ldg(&T->mask_set[mi]);
     const uint32_t slot = set & 7u, ka = (set >> 3) & 7u, kb = (set >> 6) & 7u, kc = (set >> 9) & 7u;
     const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    uint32_t *kept = P.sets + ((size_t)warp * CSM_SETS + slot) * CSM_SET_CAP;
+    uint32_t *kept = P.sets + ((size_t)slot * gridDim.x * (blockDim.x >> 5) + warp) * CSM_SET_CAP;
     const uint32_t pc = __ldg(&T->key_parent[kc]), rule_c = __ldg(&T->key_old[kc]);
     uint2 list = make_uint2(0u, 0u);
     if (ok) list = list_of(P, __ldg(&T->key_rel[kc]), pc == d ? cand : S.f[pc], 1200 + d);

@@ -121,7 +121,7 @@ struct EnumParams {
     // signature, count}, a power of two of them, or nullptr.
     uint4 *pairs;
     uint32_t pair_slots;
-    uint32_t *sets;                  // CSM_SETS * CSM_SET_CAP entries per warp of the grid
+    uint32_t *sets;                  // CSM_SET_CAP entries per kept set of a plan and warp of the grid
 };
 
 #define CSM_ROW_WORDS (1 + CSM_MAXQV)

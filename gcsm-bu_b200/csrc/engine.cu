@@ -501,6 +501,7 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
     };
     std::vector<HostPlan> plans;
     std::vector<uint32_t> begin;
+    std::vector<char> own_table;  // per plan: pendant without extend_pendant
     for (size_t qi = 0; qi < queries_.size(); qi++) {
         const Query &q = queries_[qi];
         PlanOptions po;
@@ -511,69 +512,32 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
             return rel_table_[((size_t)vl(q.vlabel[u]) * nel + el(q.edge_label(u, uu))) * nvl + vl(q.vlabel[uu])];
         };
         auto ps = build_plans(q, (uint16_t)qi, nlf_base_[qi], stats[qi], po, rel_of);
-        if (po.cartesian)
-            for (HostPlan &hp : ps) {
-                HostPlan grouped = hp;
-                const bool g = group_leaf_seeds(q, nlf_base_[qi], rel_of, grouped);
-                if (g) extend_pendant(q, rel_of, grouped);
-                if (!g || (grouped.dev.seed_group == CSM_SEED_TAIL && grouped.dev.memo_slot == CSM_NO_MEMO)) {
-                    // A pendant plan per batch edge scans two levels less than one per inner vertex
-                    // that has to walk its counting level (a path of six at 16,411 updates: two
-                    // thirds of the four-query batch, 98 -> 56 ms with both rules).
-                    extend_pendant(q, rel_of, hp);
-                    if (!g || hp.dev.memo_slot != CSM_NO_MEMO) continue;
-                }
-                hp = grouped;
+        for (HostPlan &hp : ps) {
+            own_table.push_back(hp.dev.memo_slot == CSM_MEMO_PENDING);
+            if (!po.cartesian) continue;
+            HostPlan grouped = hp;
+            const bool g = group_leaf_seeds(q, nlf_base_[qi], rel_of, grouped);
+            if (g && grouped.dev.memo_slot == CSM_MEMO_PENDING) own_table.back() = true;
+            if (g) extend_pendant(q, rel_of, grouped);
+            if (!g || (grouped.dev.seed_group == CSM_SEED_TAIL && grouped.dev.memo_slot == CSM_NO_MEMO)) {
+                // A pendant plan per batch edge scans two levels less than one per inner vertex
+                // that has to walk its counting level (a path of six at 16,411 updates: two
+                // thirds of the four-query batch, 98 -> 56 ms with both rules).
+                extend_pendant(q, rel_of, hp);
+                if (!g || hp.dev.memo_slot != CSM_NO_MEMO) continue;
             }
+            hp = grouped;
+        }
         begin.push_back((uint32_t)plans.size());
         plans.insert(plans.end(), ps.begin(), ps.end());
     }
     begin.push_back((uint32_t)plans.size());
     if (!plans_.empty() && plans.size() != plans_.size()) return fail(CSM_ERR_STATE, "re-planning changed the plan count");
-    // Pendant plans with the same counting level and deep tail classes read one table: its entries do
-    // not depend on the depths or on the query.  The tail values it sums are a table too, shared by
-    // what hangs off the counting vertex alone.  At most kMaxPendantTables of each (V entries);
-    // further pendant plans, or all of them when the tables do not fit, count normally.
+    // At most kMaxPendantTables tables of sums; further pendant plans, or all of them when the tables do not
+    // fit, count normally.
     constexpr size_t kMaxPendantTables = 16;
-    std::vector<std::vector<int64_t>> sigs, tail_sigs;
-    std::vector<uint32_t> tables;  // per table: representative plan, slot, tail values' slot
-    for (uint32_t i = 0; i < plans.size(); i++) {
-        DevPlan &dp = plans[i].dev;
-        if (dp.memo_slot != CSM_MEMO_PENDING) continue;
-        const DevLevel &lv = dp.lv[dp.tail_start - 1];
-        const DevTail &t = dp.tail;
-        std::vector<int64_t> tail_sig;
-        for (int c = 0; c < t.nclasses; c++) {
-            if (!((t.deep >> c) & 1u)) continue;
-            tail_sig.push_back(-1);
-            for (int x = t.class_term_begin[c]; x < t.class_term_begin[c + 1]; x++) {
-                const DevTailTerm &term = plans[i].terms[x];
-                tail_sig.insert(tail_sig.end(), {term.coef, term.nf});
-                for (int j = 0; j < term.nf; j++) {
-                    const int k = __builtin_ctz(t.mask[term.f[j]]);
-                    tail_sig.insert(tail_sig.end(), {t.key_rel[k], t.key_old[k]});
-                }
-            }
-        }
-        std::vector<int64_t> sig{lv.bn_rel[0], lv.old_mask & 1, lv.nlf_bitmap};
-        sig.insert(sig.end(), tail_sig.begin(), tail_sig.end());
-        size_t slot = std::find(sigs.begin(), sigs.end(), sig) - sigs.begin();
-        const size_t ts = std::find(tail_sigs.begin(), tail_sigs.end(), tail_sig) - tail_sigs.begin();
-        if (slot == sigs.size()) {
-            if (sigs.size() == kMaxPendantTables) continue;
-            sigs.push_back(sig);
-            if (ts == tail_sigs.size()) tail_sigs.push_back(tail_sig);
-            tables.insert(tables.end(), {i, (uint32_t)slot, (uint32_t)ts});
-        }
-        dp.memo_slot = (uint8_t)slot;
-        dp.memo_tail = (uint8_t)ts;
-    }
-    // Tail value tables come first.
-    const uint32_t ntail = (uint32_t)tail_sigs.size();
-    for (size_t t = 0; t < tables.size(); t += 3) tables[t + 1] += ntail;
-    for (auto &hp : plans)
-        if (hp.dev.memo_slot < CSM_MEMO_PENDING) hp.dev.memo_slot = (uint8_t)(hp.dev.memo_slot + ntail);
-    const size_t ntables = ntail + sigs.size();
+    size_t ntables = 0;
+    std::vector<uint32_t> tables = assign_pendant_tables(plans, own_table, kMaxPendantTables, ntables);
     if (ntables > memo_cap_) {
         if (d_memo_) cudaFree(d_memo_);
         d_memo_ = nullptr;

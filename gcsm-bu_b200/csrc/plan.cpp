@@ -711,6 +711,54 @@ bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp) {
     return true;
 }
 
+std::vector<uint32_t> assign_pendant_tables(std::vector<HostPlan> &plans, const std::vector<char> &first, size_t max_sums,
+                                            size_t &ntables) {
+    std::vector<std::vector<int64_t>> sigs, tail_sigs;
+    std::vector<uint32_t> tables;
+    std::vector<uint32_t> by_rank;
+    for (bool rank : {true, false})
+        for (uint32_t i = 0; i < plans.size(); i++)
+            if ((first[i] != 0) == rank) by_rank.push_back(i);
+    for (uint32_t i : by_rank) {
+        DevPlan &dp = plans[i].dev;
+        if (dp.memo_slot != CSM_MEMO_PENDING) continue;
+        const DevLevel &lv = dp.lv[dp.tail_start - 1];
+        const DevTail &t = dp.tail;
+        std::vector<int64_t> tail_sig;
+        for (int c = 0; c < t.nclasses; c++) {
+            if (!((t.deep >> c) & 1u)) continue;
+            tail_sig.push_back(-1);
+            for (int x = t.class_term_begin[c]; x < t.class_term_begin[c + 1]; x++) {
+                const DevTailTerm &term = plans[i].terms[x];
+                tail_sig.insert(tail_sig.end(), {term.coef, term.nf});
+                for (int j = 0; j < term.nf; j++) {
+                    const int k = __builtin_ctz(t.mask[term.f[j]]);
+                    tail_sig.insert(tail_sig.end(), {t.key_rel[k], t.key_old[k]});
+                }
+            }
+        }
+        std::vector<int64_t> sig{lv.bn_rel[0], lv.old_mask & 1, lv.nlf_bitmap};
+        sig.insert(sig.end(), tail_sig.begin(), tail_sig.end());
+        const size_t slot = std::find(sigs.begin(), sigs.end(), sig) - sigs.begin();
+        const size_t ts = std::find(tail_sigs.begin(), tail_sigs.end(), tail_sig) - tail_sigs.begin();
+        if (slot == sigs.size()) {
+            if (sigs.size() == max_sums) continue;
+            sigs.push_back(sig);
+            if (ts == tail_sigs.size()) tail_sigs.push_back(tail_sig);
+            tables.insert(tables.end(), {i, (uint32_t)slot, (uint32_t)ts});
+        }
+        dp.memo_slot = (uint8_t)slot;
+        dp.memo_tail = (uint8_t)ts;
+    }
+    // Tail value tables come first.
+    const uint32_t ntail = (uint32_t)tail_sigs.size();
+    for (size_t t = 0; t < tables.size(); t += 3) tables[t + 1] += ntail;
+    for (HostPlan &hp : plans)
+        if (hp.dev.memo_slot < CSM_MEMO_PENDING) hp.dev.memo_slot = (uint8_t)(hp.dev.memo_slot + ntail);
+    ntables = ntail + sigs.size();
+    return tables;
+}
+
 std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans) {
     std::ostringstream os;
     os << "Orders:\n";
@@ -728,7 +776,8 @@ std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans) {
         }
         os << "\n    tail: " << (hp.dev.tail_start < hp.dev.n ? "from depth " + std::to_string(hp.dev.tail_start) : std::string("none"))
            << ", " << hp.terms.size() << " terms" << (hp.dev.shared_last ? ", last level shared by the level above" : "")
-           << (hp.dev.memo_slot != CSM_NO_MEMO ? ", pendant counting level" : "")
+           << (hp.dev.memo_slot == CSM_NO_MEMO ? "" : hp.dev.memo_slot == CSM_MEMO_PENDING
+               ? ", pendant counting level without a table" : ", pendant counting level")
            << (hp.dev.seed_group == CSM_SEED_WEIGHT ? ", leaf of the updated edge counted per inner vertex"
                : hp.dev.seed_group == CSM_SEED_TAIL ? ", leaf of the updated edge counted in the tail" : "")
            << "\n";

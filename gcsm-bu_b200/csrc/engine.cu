@@ -533,21 +533,20 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
     }
     begin.push_back((uint32_t)plans.size());
     if (!plans_.empty() && plans.size() != plans_.size()) return fail(CSM_ERR_STATE, "re-planning changed the plan count");
-    // At most kMaxPendantTables tables of sums; further pendant plans, or all of them when the tables do not
-    // fit, count normally.
+    // At most kMaxPendantTables tables of sums; further pendant plans count normally.  The tables are an
+    // optimisation: they only take memory the adjacency pool is unlikely to need (at most a quarter of what is
+    // free now), and where that is short for all of them the first ones get theirs.
     constexpr size_t kMaxPendantTables = 16;
-    size_t ntables = 0;
-    std::vector<uint32_t> tables = assign_pendant_tables(plans, own_table, kMaxPendantTables, ntables);
+    const size_t table_bytes = (size_t)g_.V * sizeof(unsigned long long);
+    size_t free_b = 0, total_b = 0, ntables = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+    const size_t room = std::max(memo_cap_, (free_b + memo_cap_ * table_bytes) / 4 / table_bytes);
+    std::vector<uint32_t> tables = assign_pendant_tables(plans, own_table, kMaxPendantTables, room, ntables);
     if (ntables > memo_cap_) {
         if (d_memo_) cudaFree(d_memo_);
         d_memo_ = nullptr;
         memo_cap_ = 0;
-        // The tables are an optimisation: they only take memory the adjacency pool is unlikely
-        // to need (at most a quarter of what is free now).
-        size_t free_b = 0, total_b = 0;
-        const size_t want = ntables * (size_t)g_.V * sizeof(unsigned long long);
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 4 &&
-            (d_memo_desc_ || dev_alloc(&d_memo_desc_, 3 * kMaxPendantTables) == cudaSuccess) &&
+        if ((d_memo_desc_ || dev_alloc(&d_memo_desc_, 3 * kMaxPendantTables) == cudaSuccess) &&
             dev_alloc(&d_memo_, ntables * (size_t)g_.V) == cudaSuccess) {
             memo_cap_ = ntables;
         } else {

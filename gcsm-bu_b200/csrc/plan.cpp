@@ -712,7 +712,7 @@ bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp) {
 }
 
 std::vector<uint32_t> assign_pendant_tables(std::vector<HostPlan> &plans, const std::vector<char> &first, size_t max_sums,
-                                            size_t &ntables) {
+                                            size_t max_tables, size_t &ntables) {
     std::vector<std::vector<int64_t>> sigs, tail_sigs;
     std::vector<uint32_t> tables;
     std::vector<uint32_t> by_rank;
@@ -742,7 +742,8 @@ std::vector<uint32_t> assign_pendant_tables(std::vector<HostPlan> &plans, const 
         const size_t slot = std::find(sigs.begin(), sigs.end(), sig) - sigs.begin();
         const size_t ts = std::find(tail_sigs.begin(), tail_sigs.end(), tail_sig) - tail_sigs.begin();
         if (slot == sigs.size()) {
-            if (sigs.size() == max_sums) continue;
+            const size_t more = ts == tail_sigs.size() ? 2 : 1;
+            if (sigs.size() == max_sums || sigs.size() + tail_sigs.size() + more > max_tables) continue;
             sigs.push_back(sig);
             if (ts == tail_sigs.size()) tail_sigs.push_back(tail_sig);
             tables.insert(tables.end(), {i, (uint32_t)slot, (uint32_t)ts});

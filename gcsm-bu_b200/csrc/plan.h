@@ -61,12 +61,12 @@ bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp);
 // Table slots (DevPlan.memo_slot, memo_tail) of the pendant plans of an engine.  Plans with the same
 // counting level and deep tail classes read one table: its entries do not depend on the depths or on the
 // query.  The tail values it sums are a table too, shared by what hangs off the counting vertex alone.
-// At most `max_sums` tables of sums; further plans stay CSM_MEMO_PENDING.  Plans marked in `first` (those
+// At most `max_sums` tables of sums, and `max_tables` with the tail values; further plans stay CSM_MEMO_PENDING.  Plans marked in `first` (those
 // that are pendant without extend_pendant) come first, whatever queries were registered before theirs: such
 // a query after twenty that need extend_pendant took 10.2 ms at 250,007 updates, before them 5.2.
 // Returns, per table of sums: a plan that reads it, its slot, the slot of its tail values.
 std::vector<uint32_t> assign_pendant_tables(std::vector<HostPlan> &plans, const std::vector<char> &first, size_t max_sums,
-                                            size_t &ntables);
+                                            size_t max_tables, size_t &ntables);
 
 // Text description, one block per query edge, in the spirit of PlanManager::PrintOrders.
 std::string describe_plans(const Query &q, const std::vector<HostPlan> &plans);

@@ -4,6 +4,7 @@
 #include <map>
 #include <random>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "plan.h"
@@ -69,19 +70,22 @@ int main() {
         extended += !p.own[i] && p.plans[i].dev.memo_slot == CSM_MEMO_PENDING;
     }
     CHECK(own > 0 && extended > 16);
-    for (size_t max_sums : {(size_t)0, (size_t)1, (size_t)16, (size_t)200}) {
+    for (auto [max_sums, max_tables] : {std::pair<size_t, size_t>{0, 400}, {1, 400}, {16, 400}, {16, 32}, {16, 20}, {16, 7},
+                                        {16, 1}, {16, 0}, {200, 400}}) {
         std::vector<HostPlan> plans = p.plans;
         size_t ntables = 0;
-        const std::vector<uint32_t> tables = assign_pendant_tables(plans, p.own, max_sums, ntables);
+        const std::vector<uint32_t> tables = assign_pendant_tables(plans, p.own, max_sums, max_tables, ntables);
         const size_t sums = tables.size() / 3;
-        CHECK(sums <= max_sums && ntables <= 2 * sums && ntables >= sums);
+        CHECK(sums <= max_sums && ntables <= 2 * sums && ntables >= sums && ntables <= max_tables);
+        CHECK(max_tables > 20 || sums >= max_tables / 2);  // the room there is gets used
         int with = 0, without = 0;
         for (size_t i = 0; i < plans.size(); i++) {
             const DevPlan &dp = plans[i].dev;
             if (dp.memo_slot == CSM_NO_MEMO) continue;
             if (dp.memo_slot == CSM_MEMO_PENDING) {
                 without++;
-                CHECK(sums == max_sums && (max_sums < 16 || !p.own[i]));  // a plan goes without only when none is left
+                // A plan goes without only when no table is left.
+                CHECK((sums == max_sums || ntables + 2 > max_tables) && (max_sums < 16 || max_tables < 20 || !p.own[i]));
                 continue;
             }
             with++;
@@ -96,7 +100,7 @@ int main() {
             }
             CHECK(found && dp.memo_slot < ntables && dp.memo_tail < dp.memo_slot);
         }
-        CHECK(with + without == own + extended || max_sums == 0);
+        CHECK(with + without == own + extended);
         CHECK(max_sums < 200 || without == 0);
     }
     std::printf("ok %d plans pendant as they stand, %d extended\n", own, extended);

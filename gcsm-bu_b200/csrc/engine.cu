@@ -1170,6 +1170,17 @@ void Engine::clear_graphs() {
 
 csm_status Engine::run_batch(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elabel,
                              const uint8_t *is_delete, bool has_delete, cudaStream_t s, csm_batch_result *out) {
+    try {
+        return run_batch_steps(n, src, dst, elabel, is_delete, has_delete, s, out);
+    } catch (...) {
+        // Host memory ran out between two steps: the graph may hold part of the batch.
+        poisoned_ = true;
+        throw;
+    }
+}
+
+csm_status Engine::run_batch_steps(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elabel,
+                                   const uint8_t *is_delete, bool has_delete, cudaStream_t s, csm_batch_result *out) {
     const uint32_t m = (uint32_t)(2 * n);
     const uint32_t np = (uint32_t)plans_.size();
     rows_valid_ = false;

@@ -152,6 +152,8 @@ class Engine {
     int64_t inject_left_ = 0;
     csm_status run_batch(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elabel,
                          const uint8_t *is_delete, bool has_delete, cudaStream_t s, csm_batch_result *out);
+    csm_status run_batch_steps(uint64_t n, const uint32_t *src, const uint32_t *dst, const uint32_t *elabel,
+                               const uint8_t *is_delete, bool has_delete, cudaStream_t s, csm_batch_result *out);
     csm_status enumerate_phase(uint32_t phase, uint32_t m, cudaStream_t s);
     csm_status maybe_compact(cudaStream_t s);
 

@@ -1184,9 +1184,11 @@ csm_status Engine::run_batch_steps(uint64_t n, const uint32_t *src, const uint32
     const uint32_t m = (uint32_t)(2 * n);
     const uint32_t np = (uint32_t)plans_.size();
     rows_valid_ = false;
-    // A phase that the batch does not run leaves no rows (the vectors keep their memory).
-    for (auto &phase : last_rows_)
-        for (auto &rows : phase) rows.clear();
+    // A phase that the batch does not run leaves no rows.  (One that runs resizes them: cleared here, they
+    // would be filled with zeros first, 2% of a pass over 4,001 updates with rows.)
+    for (int deleted : {0, 1})
+        if (!m || (deleted && !has_delete))
+            for (auto &rows : last_rows_[deleted]) rows.clear();
     phase_ran_[0] = phase_ran_[1] = false;
     last_frontier_rows_ = 0;
     deferred_ = CSM_OK;

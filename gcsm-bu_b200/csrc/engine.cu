@@ -1194,9 +1194,13 @@ csm_status Engine::run_batch_steps(uint64_t n, const uint32_t *src, const uint32
     deferred_ = CSM_OK;
     NlfTables nt{d_spec_begin_, d_specs_, d_bits_, words_};
     if (d_pairs_ && pair_phases_ + 64 > CSM_PAIR_PHASES) {
-        // Before the phase numbers run out the table starts over.
+        // Before the phase numbers run out the table starts over; the first time already after
+        // kFirstPairPhases, so that a restart is nothing that only engines of half a million batches meet.
+        const bool first = !pairs_cleared_;
         const csm_status pst = clear_pairs(s);
         if (pst != CSM_OK) return pst;
+        pairs_cleared_ = true;
+        if (first) pair_phases_ = CSM_PAIR_PHASES - 64 - kFirstPairPhases;
     }
     pair_phases_ += 2 * (tune_left_ > 0 ? tune_cands_.size() + 1 : 2);  // the batch's phases, a rerun's too
     const bool tuning = tune_left_ > 0 && !no_alloc_ && cfg_.materialize_rows == 0;

@@ -300,6 +300,8 @@ class Engine {
     uint32_t *d_sets_ = nullptr;              // kept intersections: sets of the plans * warps of the largest grid
     size_t set_entries_ = 0;
     uint64_t pair_phases_ = 0;                // the same, an upper bound kept by the host
+    bool pairs_cleared_ = false;
+    static constexpr uint64_t kFirstPairPhases = 64;
     int expand_levels_ = 0;                   // most breadth-first levels any plan expands
     LaunchConfig lc_{};                       // configuration in use
     std::vector<LaunchConfig> tune_cands_;    // autotuner candidates

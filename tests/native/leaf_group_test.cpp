@@ -2,7 +2,8 @@
 // labelled queries and random data graphs with some edges marked as batch edges, the plan that starts
 // once per data vertex of the inner endpoint, and the plan whose counting level is settled from
 // per-vertex sums, count what the plan that starts at every batch edge counts.  All device forms are
-// evaluated by the same small interpreter (levels, flag rules, exclusions, tail polynomial, tables).
+// evaluated by the same small interpreter (levels, flag rules, exclusions, candidate bitmaps, tail
+// polynomial, tables).
 #include <algorithm>
 #include <cstdio>
 #include <map>
@@ -36,6 +37,15 @@ struct Graph {
         for (const Entry &e : list(rel, v))
             if (e.v == w) return e.batch ? 2 : 1;
         return 0;
+    }
+    // Candidate bitmaps (the NLF rule): per bitmap the groups that a vertex needs, a relation and how many
+    // neighbours in it.
+    std::vector<std::vector<std::pair<int, uint32_t>>> groups;
+    bool candidate(uint32_t bitmap, uint32_t v) const {
+        if (bitmap == CSM_NO_BITMAP) return true;
+        for (auto &g : groups[bitmap])
+            if (list(g.first, v).size() < g.second) return false;
+        return true;
     }
 };
 
@@ -92,18 +102,20 @@ long long common(const Graph &g, int ra, uint32_t a, int rule_a, int rb, uint32_
 }
 
 // A pendant counting level below the prefix f[0..c-1]: the sum over its list, without exclusions, less
-// the prefix vertices that the sum should not hold, times what hangs off the prefix.
+// the prefix vertices that the sum should not hold, times what hangs off the prefix.  As on the device, the
+// cut vertices are taken off without a look at the level's candidate bitmap: where extend_pendant allows a cut,
+// a vertex next to a cut vertex passes it.
 long long settle(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> &terms, const uint32_t *f) {
     const int c = p.tail_start - 1, md = p.memo_depth;
     const DevLevel &lv = p.lv[c];
     const bool old = lv.old_mask & 1u;
     long long sum = 0;
     for (const Entry &e : g.list(lv.bn_rel[0], f[md]))
-        if (!(old && e.batch)) sum += tail_value(g, p, terms, e.v);
+        if (!(old && e.batch) && g.candidate(lv.nlf_bitmap, e.v)) sum += tail_value(g, p, terms, e.v);
     for (int j = 0; j < c; j++) {
         if (!((lv.excl_mask >> j) & 1u) || j == md) continue;
         const int x = g.entry(lv.bn_rel[0], f[md], f[j]);
-        if (!x || (old && x == 2)) continue;
+        if (!x || (old && x == 2) || !g.candidate(lv.nlf_bitmap, f[j])) continue;
         sum -= tail_value(g, p, terms, f[j]);
         for (int i = 0; i < c; i++) {
             if (!((p.memo_cut >> i) & 1u)) continue;
@@ -131,7 +143,7 @@ long long walk(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm> 
         }
         for (int j = 0; ok && j < d; j++)
             if (((lv.excl_mask >> j) & 1u) && f[j] == e.v) ok = false;
-        if (!ok) continue;
+        if (!ok || !g.candidate(lv.nlf_bitmap, e.v)) continue;
         f[d] = e.v;
         total += walk(g, p, terms, f, d + 1);
     }
@@ -145,12 +157,13 @@ long long count(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm>
         for (const Entry &e : g.list(p.seed_rel, v)) batch += e.batch;
         // The position without a query vertex holds a number: it must never be read as a vertex.
         uint32_t f[CSM_MAXQV] = {v, batch};
+        if (!g.candidate(p.nlf0, v)) continue;
         if (p.seed_group != CSM_SEED_EDGE) {
             if (batch) total += (p.seed_group == CSM_SEED_WEIGHT ? batch : 1) * walk(g, p, terms, f, 2);
             continue;
         }
         for (const Entry &e : g.list(p.seed_rel, v)) {
-            if (!e.batch) continue;
+            if (!e.batch || !g.candidate(p.nlf1, e.v)) continue;
             f[1] = e.v;
             total += walk(g, p, terms, f, 2);
         }
@@ -209,6 +222,10 @@ int main() {
                         if (it != rels.end()) g.lists[{it->second, e.first}].push_back({e.second, batch});
                     }
                 }
+        g.groups.resize(nv);
+        for (uint32_t u = 0; u < nv; u++)
+            for (auto &grp : q.nlf[u])
+                g.groups[u].push_back({rels.at(std::make_tuple(q.vlabel[u], grp.elabel, grp.vlabel)), (uint32_t)grp.count});
         for (size_t i = 0; i < plans.size(); i++) {
             HostPlan hp = plans[i];
             const long long want = count(g, plans[i].dev, plans[i].terms);

@@ -512,22 +512,8 @@ csm_status Engine::install_plans(const std::vector<EdgeStats> &stats) {
             return rel_table_[((size_t)vl(q.vlabel[u]) * nel + el(q.edge_label(u, uu))) * nvl + vl(q.vlabel[uu])];
         };
         auto ps = build_plans(q, (uint16_t)qi, nlf_base_[qi], stats[qi], po, rel_of);
-        for (HostPlan &hp : ps) {
-            own_table.push_back(hp.dev.memo_slot == CSM_MEMO_PENDING);
-            if (!po.cartesian) continue;
-            HostPlan grouped = hp;
-            const bool g = group_leaf_seeds(q, nlf_base_[qi], rel_of, grouped);
-            if (g && grouped.dev.memo_slot == CSM_MEMO_PENDING) own_table.back() = true;
-            if (g) extend_pendant(q, rel_of, grouped);
-            if (!g || (grouped.dev.seed_group == CSM_SEED_TAIL && grouped.dev.memo_slot == CSM_NO_MEMO)) {
-                // A pendant plan per batch edge scans two levels less than one per inner vertex
-                // that has to walk its counting level (a path of six at 16,411 updates: two
-                // thirds of the four-query batch, 98 -> 56 ms with both rules).
-                extend_pendant(q, rel_of, hp);
-                if (!g || hp.dev.memo_slot != CSM_NO_MEMO) continue;
-            }
-            hp = grouped;
-        }
+        for (HostPlan &hp : ps)
+            own_table.push_back(po.cartesian ? rewrite_plan(q, nlf_base_[qi], rel_of, hp) : hp.dev.memo_slot == CSM_MEMO_PENDING);
         begin.push_back((uint32_t)plans.size());
         plans.insert(plans.end(), ps.begin(), ps.end());
     }

@@ -665,6 +665,24 @@ bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, Ho
     return true;
 }
 
+bool counted_by_lane(const DevPlan &dp) {
+    const DevTail &t = dp.tail;
+    const int level = dp.tail_start - 1;
+    if (dp.tail_start >= dp.n) return false;
+    if (t.lane_par) return true;
+    if (level < 2 || t.nmasks > CSM_PAIR_MAXMASKS) return false;
+    int sets = 0;
+    for (int m = 0; m < t.nmasks; m++) {
+        const int bits = __builtin_popcount(t.mask[m]);
+        if (bits > 3) return false;
+        if (bits < 3) continue;
+        int above = 0;
+        for (int k = 0; k < t.nkeys; k++) above += ((t.mask[m] >> k) & 1u) && t.key_parent[k] < level;
+        if (above < 2 || ++sets > CSM_SETS) return false;
+    }
+    return true;
+}
+
 bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp) {
     DevPlan &dp = hp.dev;
     const DevTail &t = dp.tail;
@@ -709,6 +727,28 @@ bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp) {
     dp.memo_depth = md;
     dp.expand_stop = (uint8_t)(c - 1);
     return true;
+}
+
+bool rewrite_plan(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp) {
+    bool own = hp.dev.memo_slot == CSM_MEMO_PENDING;
+    HostPlan grouped = hp;
+    const bool g = group_leaf_seeds(q, nlf_base, rel_of, grouped);
+    if (g && grouped.dev.memo_slot == CSM_MEMO_PENDING) own = true;
+    if (g) extend_pendant(q, rel_of, grouped);
+    if (!g || (grouped.dev.seed_group == CSM_SEED_TAIL && grouped.dev.memo_slot == CSM_NO_MEMO)) {
+        // A pendant plan per batch edge scans two levels less than one per inner vertex
+        // that has to walk its counting level (a path of six at 16,411 updates: two
+        // thirds of the four-query batch, 98 -> 56 ms with both rules).
+        extend_pendant(q, rel_of, hp);
+        if (!g || hp.dev.memo_slot != CSM_NO_MEMO) return own;
+        // With the leaf in the tail a vertex of its label can bring a mask of four lists, and the tail is
+        // then counted one prefix at a time.  Where the plan per batch edge is counted for 32 at once that
+        // costs more than the repeats it saves: 262,144 updates on 43M edges 2080 -> 738 ms with the edge
+        // form, 106 -> 53 and 150 -> 74 ms at half the size; 96 -> 104 ms where hubs own most batch edges.
+        if (!counted_by_lane(grouped.dev) && counted_by_lane(hp.dev)) return own;
+    }
+    hp = grouped;
+    return own;
 }
 
 std::vector<uint32_t> assign_pendant_tables(std::vector<HostPlan> &plans, const std::vector<char> &first, size_t max_sums,

@@ -54,9 +54,17 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
 // leaf would need a tail that exceeds the device tables.
 bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp);
 
+// Whether a plan has a tail that is counted for 32 prefixes at once: its masks are single keys, pairs, or
+// triples with two keys above the counting level.
+bool counted_by_lane(const DevPlan &dp);
+
 // Marks the device form of a plan as pendant (DevPlan.memo_slot) where it is not already and its
 // counting level allows it.  Returns whether it did.
 bool extend_pendant(const Query &q, const RelOf &rel_of, HostPlan &hp);
+
+// Rewrites the device form of a plan as group_leaf_seeds and extend_pendant allow, where that is the form
+// that counts faster.  Returns whether the plan was pendant without extend_pendant.
+bool rewrite_plan(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp);
 
 // Table slots (DevPlan.memo_slot, memo_tail) of the pendant plans of an engine.  Plans with the same
 // counting level and deep tail classes read one table: its entries do not depend on the depths or on the

@@ -175,7 +175,7 @@ long long count(const Graph &g, const DevPlan &p, const std::vector<DevTailTerm>
 
 int main() {
     std::mt19937 rng(77);
-    int grouped[3] = {0, 0, 0}, nonzero = 0, pendant = 0, cut = 0;
+    int grouped[3] = {0, 0, 0}, nonzero = 0, pendant = 0, cut = 0, kept = 0;
     for (int qn = 0; qn < 600; qn++) {
         const uint32_t nv = 2 + rng() % 6, nlab = 1 + rng() % 4;
         std::vector<uint32_t> vl(nv), src, dst, el;
@@ -248,6 +248,19 @@ int main() {
                     return 1;
                 }
             }
+            HostPlan rp = plans[i];
+            rewrite_plan(q, 0, rel_of, rp);
+            if (count(g, rp.dev, rp.terms) != want) {
+                std::printf("FAIL query %d plan %zu: its rewritten form counts otherwise than %lld\n", qn, i, want);
+                return 1;
+            }
+            // A leaf in the tail must not cost the plan its counting of 32 prefixes at once.
+            if (rp.dev.seed_group == CSM_SEED_TAIL && rp.dev.memo_slot == CSM_NO_MEMO && counted_by_lane(plans[i].dev) &&
+                !counted_by_lane(rp.dev)) {
+                std::printf("FAIL query %d plan %zu: grouped into a tail that is counted one prefix at a time\n", qn, i);
+                return 1;
+            }
+            kept += did && rp.dev.seed_group == CSM_SEED_EDGE && !counted_by_lane(hp.dev);
             if (got != want) {
                 std::printf("FAIL query %d plan %zu: %lld per inner vertex, %lld per batch edge\n", qn, i, got, want);
                 return 1;
@@ -255,10 +268,10 @@ int main() {
         }
     }
     if (grouped[CSM_SEED_WEIGHT] < 50 || grouped[CSM_SEED_TAIL] < 50 || nonzero < 100 ||
-        pendant < 50 || cut < 20)
-        return std::printf("too few plans: %d weighted, %d in the tail, %d of them with matches, %d pendant, %d cut\n",
-                           grouped[1], grouped[2], nonzero, pendant, cut), 1;
-    std::printf("ok %d weighted, %d in the tail, %d of them with matches, %d pendant, %d of them cut\n", grouped[1], grouped[2],
-                nonzero, pendant, cut);
+        pendant < 50 || cut < 20 || kept < 5)
+        return std::printf("too few plans: %d weighted, %d in the tail, %d of them with matches, %d pendant, %d cut, %d not grouped\n",
+                           grouped[1], grouped[2], nonzero, pendant, cut, kept), 1;
+    std::printf("ok %d weighted, %d in the tail, %d of them with matches, %d pendant, %d of them cut, %d not grouped\n", grouped[1], grouped[2],
+                nonzero, pendant, cut, kept);
     return 0;
 }

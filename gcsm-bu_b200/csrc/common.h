@@ -87,9 +87,11 @@ struct DevTailTerm {
     uint8_t f[7];                  // mask ids
 };
 
-// Cartesian tail of a plan: query vertices at depth >= tail_start are leaves whose only
-// neighbour is matched earlier (plan.cpp:1785-1841 TreeCartesianProduct).  Their number of
-// injective assignments is counted by inclusion-exclusion over the leaves of one label.
+// Cartesian tail of a plan: the query vertices at depth >= tail_start are pairwise non-adjacent and
+// have all their neighbours matched earlier (leaves, as in plan.cpp:1785-1841 TreeCartesianProduct, and
+// vertices with several lists; the leaf of the updated edge, too, see DevPlan.seed_group).  The number of
+// their injective assignments is counted by inclusion-exclusion over the vertices of one label, from the
+// sizes of intersections of their lists.
 struct DevTail {
     uint8_t nkeys;                              // distinct (parent depth, relation, old) lists
     uint8_t key_parent[CSM_TAIL_MAXKEYS];

@@ -76,9 +76,8 @@ csm_status Engine::cuda_fail(cudaError_t e, const char *where) {
         if (e__ != cudaSuccess) return cuda_fail(e__, #call); \
     } while (0)
 
-// Persistent launch: never more blocks than can be resident at once.  Warps that run out of work
-// wait for the others while any warp holds work, so a block that could only start after resident
-// blocks exit would stall the launch until the idle bound runs out.
+// Persistent launch: never more blocks than can be resident at once.  Warps that run out of work stay
+// while any warp holds some, so a block without room would start when nothing is left to take.
 int Engine::grid_blocks(const LaunchConfig &c) const {
     const int resident = enum_blocks_per_sm(c.warps_per_block, c.occupancy);
     return sm_count_ * (cfg_.blocks_per_sm > 0 && cfg_.blocks_per_sm < resident ? cfg_.blocks_per_sm : resident);
@@ -673,8 +672,8 @@ csm_status Engine::install_pairs(std::vector<HostPlan> &plans) {
 }
 
 // A slot of the pair table for 16 to 8 entries of the adjacency pool, so the table of an engine over a
-// small graph stays small (a thousand tenants have one each), and at most 4M slots: 64 MB stay in the
-// L2 cache.  With 2M pool entries (10,000 vertices, 50,000 edges) 2 MB instead of 64: 1024 updates with a
+// small graph stays small (a thousand tenants have one each), and at most 4M slots: the 64 MB of one
+// engine at a time stay in the L2 cache.  With 2M pool entries (10,000 vertices, 50,000 edges) 2 MB instead of 64: 1024 updates with a
 // captured graph 0.46 ms with either.
 uint32_t Engine::pair_slots_wanted() const {
     uint32_t slots = 1u << 14;

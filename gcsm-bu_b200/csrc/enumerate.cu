@@ -19,12 +19,14 @@
 //
 // Load balance: warps first take seed chunks from a ticket counter.  A warp that runs out of
 // work takes the next position of a global ring and waits there; a busy warp that sees waiting
-// positions splits off part of its pending work (the upper half of a candidate range, or buffered
-// sibling candidates) into the ring.  Every wait is bounded, and a launch whose bound runs out
-// reports it; a warp never waits on another warp's progress to finish its own items.
+// positions hands out pending work of its shallowest level that has some: the candidate range in as
+// many parts as warps wait (at most 31), or the buffered sibling candidates, one item each.  Every
+// wait is bounded: a warp whose bound runs out closes the ring and leaves (ring.h).  A warp never
+// waits on another warp's progress to finish its own items.
 //
-// Tail leaves (query vertices of degree one matched after their neighbour) are not enumerated:
-// their number of injective assignments is computed from list sizes by inclusion-exclusion.
+// Tail vertices (the last of the order, pairwise non-adjacent, all their neighbours matched before
+// them) are not enumerated: the number of their injective assignments is computed by
+// inclusion-exclusion from the sizes of their lists and of the lists' intersections.
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
@@ -1933,8 +1935,9 @@ __global__ void k_phase_begin(EnumControl *ctrl, const uint32_t *nticket, uint32
 }
 
 // Tail values of the pendant plans (DevPlan.memo_tail): for every data vertex w at the counting level,
-// the deep tail classes' count below it (no prefix vertex can sit in their lists).  blockIdx.y names
-// the table; the first of those that share tail values fills them.
+// the deep tail classes' count below it, without exclusions.  No prefix vertex can sit in their lists, but
+// for the cut vertices (DevPlan.memo_cut), which settle_pendant takes off.  blockIdx.y names the table;
+// the first of those that share tail values fills them.
 __global__ void k_tail_values(EnumParams P, const uint32_t *desc, unsigned long long *memo) {
     const DevPlan *pl = P.plans + desc[3 * blockIdx.y];
     const uint32_t slot = desc[3 * blockIdx.y + 2];

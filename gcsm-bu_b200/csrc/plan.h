@@ -50,8 +50,8 @@ std::vector<HostPlan> build_plans(const Query &q, uint16_t query_id, uint32_t nl
 // Rewrites the device form of the plan of a query edge with a leaf endpoint so that its seeds are
 // the data vertices of the inner endpoint instead of the batch edges (DevPlan.seed_group); order,
 // bn and tail_start keep describing the plan it stands for.  Returns whether it did: not for edges
-// without a leaf, queries of two vertices or of CSM_MAXQV, or row-materialising plans, nor when the
-// leaf would need a tail that exceeds the device tables.
+// without a leaf, queries of two vertices or row-materialising plans, nor where the leaf has to be counted
+// in the tail and the query has CSM_MAXQV vertices or the tail would exceed the device tables.
 bool group_leaf_seeds(const Query &q, uint32_t nlf_base, const RelOf &rel_of, HostPlan &hp);
 
 // Whether a plan has a tail that is counted for 32 prefixes at once: its masks are single keys, pairs, or

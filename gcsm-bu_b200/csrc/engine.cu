@@ -104,6 +104,8 @@ csm_status Engine::init() {
     CSM_CUDA(cudaGetDeviceProperties(&prop, device_));
     if (prop.major < 10) return fail(CSM_ERR_NO_DEVICE, "this library is built for sm_100a (B200)");
     sm_count_ = prop.multiProcessorCount;
+    // stream_ does not wait for the default stream, and a copy from pageable memory returns before it has
+    // arrived: every fill and copy that a kernel on stream_ reads goes through stream_ as well.
     CSM_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     for (auto &e : ev_) CSM_CUDA(cudaEventCreate(&e));
     if (cfg_.queue_slots != 0) {
@@ -165,7 +167,7 @@ csm_status Engine::init() {
         for (size_t i = 0; i < 2 * tune_cands_.size(); i++) CSM_CUDA(cudaEventCreate(&tune_ev_[i]));
     }
     CSM_CUDA(dev_alloc(&d_ctrl_, 1));
-    CSM_CUDA(cudaMemset(d_ctrl_, 0, sizeof(EnumControl)));
+    CSM_CUDA(cudaMemsetAsync(d_ctrl_, 0, sizeof(EnumControl), stream_));
     CSM_CUDA(cudaMallocHost(&h_counts_, sizeof(unsigned long long) * 64));
     CSM_CUDA(cudaMallocHost(&h_ctrl_, sizeof(EnumControl) * 2));
     return CSM_OK;
@@ -302,23 +304,26 @@ csm_status Engine::prepare_tables(uint32_t nv, const uint32_t *vlabel, const uin
     }
     const size_t nmeta = (size_t)g_.R * nv;
     CSM_CUDA(dev_alloc(&g_.vlab, nv));
-    CSM_CUDA(cudaMemcpy(g_.vlab, vlab.data(), nv, cudaMemcpyHostToDevice));
+    CSM_CUDA(cudaMemcpyAsync(g_.vlab, vlab.data(), nv, cudaMemcpyHostToDevice, stream_));
     CSM_CUDA(dev_alloc(&d_elab_raw_, nel));
-    CSM_CUDA(cudaMemcpy(d_elab_raw_, elab_raw_.data(), sizeof(uint32_t) * nel, cudaMemcpyHostToDevice));
+    CSM_CUDA(cudaMemcpyAsync(d_elab_raw_, elab_raw_.data(), sizeof(uint32_t) * nel, cudaMemcpyHostToDevice, stream_));
     CSM_CUDA(dev_alloc(&d_rel_table_, rel_table_.size()));
-    CSM_CUDA(cudaMemcpy(d_rel_table_, rel_table_.data(), sizeof(uint16_t) * rel_table_.size(), cudaMemcpyHostToDevice));
+    CSM_CUDA(cudaMemcpyAsync(d_rel_table_, rel_table_.data(), sizeof(uint16_t) * rel_table_.size(),
+                             cudaMemcpyHostToDevice, stream_));
     CSM_CUDA(dev_alloc(&d_spec_begin_, nvl + 1));
-    CSM_CUDA(cudaMemcpy(d_spec_begin_, spec_begin.data(), sizeof(uint32_t) * (nvl + 1), cudaMemcpyHostToDevice));
+    CSM_CUDA(cudaMemcpyAsync(d_spec_begin_, spec_begin.data(), sizeof(uint32_t) * (nvl + 1), cudaMemcpyHostToDevice,
+                             stream_));
     CSM_CUDA(dev_alloc(&d_specs_, specs.size()));
     if (!specs.empty())
-        CSM_CUDA(cudaMemcpy(d_specs_, specs.data(), sizeof(NlfSpec) * specs.size(), cudaMemcpyHostToDevice));
+        CSM_CUDA(cudaMemcpyAsync(d_specs_, specs.data(), sizeof(NlfSpec) * specs.size(), cudaMemcpyHostToDevice, stream_));
     CSM_CUDA(dev_alloc(&d_bits_, (size_t)nbitmaps_ * words_));
-    CSM_CUDA(cudaMemset(d_bits_, 0, sizeof(uint32_t) * (size_t)nbitmaps_ * words_));
+    CSM_CUDA(cudaMemsetAsync(d_bits_, 0, sizeof(uint32_t) * (size_t)nbitmaps_ * words_, stream_));
     CSM_CUDA(dev_alloc(&g_.meta, nmeta));
     CSM_CUDA(dev_alloc(&g_.cap, nmeta));
     CSM_CUDA(dev_alloc(&g_.pool_top, 1));
     CSM_CUDA(dev_alloc(&d_touched_, words_));
-    CSM_CUDA(cudaMemset(d_touched_, 0, sizeof(uint32_t) * words_));
+    CSM_CUDA(cudaMemsetAsync(d_touched_, 0, sizeof(uint32_t) * words_, stream_));
+    CSM_CUDA(cudaStreamSynchronize(stream_));  // the host arrays end here
     return CSM_OK;
 }
 
@@ -344,9 +349,12 @@ csm_status Engine::build_lists(uint64_t ne, const uint32_t *src, const uint32_t 
             break;
         }
         if (ne) {
-            cudaMemcpy(d_src, src, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice);
-            cudaMemcpy(d_dst, dst, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice);
-            cudaMemcpy(d_lab, elabel, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice);
+            if ((e = cudaMemcpyAsync(d_src, src, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice, stream_)) ||
+                (e = cudaMemcpyAsync(d_dst, dst, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice, stream_)) ||
+                (e = cudaMemcpyAsync(d_lab, elabel, sizeof(uint32_t) * ne, cudaMemcpyHostToDevice, stream_))) {
+                st = cuda_fail(e, "initial edge copies");
+                break;
+            }
             store_build_keys(ne, d_src, d_dst, d_lab, nullptr, lt, g_, kl_, k_raw, BatchReset{}, stream_);
         }
         store_sort_keys(nullptr, temp_bytes, k_raw, k_sorted, m, kl_, stream_);
@@ -423,7 +431,7 @@ csm_status Engine::finish_load() {
     // launch, so it only needs room for the items in flight at once.
     CSM_CUDA(dev_alloc(&d_queue_, qcap_));
     CSM_CUDA(dev_alloc(&d_seq_, qcap_));
-    CSM_CUDA(cudaMemset(d_seq_, 0, sizeof(unsigned long long) * qcap_));
+    CSM_CUDA(cudaMemsetAsync(d_seq_, 0, sizeof(unsigned long long) * qcap_, stream_));
     sc_.ctrl = d_ctrl_;
     sc_.queue = d_queue_;
     sc_.seq = d_seq_;
@@ -851,11 +859,12 @@ csm_status Engine::upload_snapshot(uint64_t used, uint64_t capacity, const std::
     if (want > 0xFFFFFFF0ull) want = 0xFFFFFFF0ull;
     g_.pool_cap = want;
     CSM_CUDA(dev_alloc(&g_.pool, g_.pool_cap));
-    CSM_CUDA(cudaMemcpy(g_.meta, meta.data(), sizeof(uint2) * nmeta, cudaMemcpyHostToDevice));
-    CSM_CUDA(cudaMemcpy(g_.cap, cap.data(), sizeof(uint32_t) * nmeta, cudaMemcpyHostToDevice));
-    if (used) CSM_CUDA(cudaMemcpy(g_.pool, pool.data(), sizeof(uint32_t) * used, cudaMemcpyHostToDevice));
+    CSM_CUDA(cudaMemcpyAsync(g_.meta, meta.data(), sizeof(uint2) * nmeta, cudaMemcpyHostToDevice, stream_));
+    CSM_CUDA(cudaMemcpyAsync(g_.cap, cap.data(), sizeof(uint32_t) * nmeta, cudaMemcpyHostToDevice, stream_));
+    if (used) CSM_CUDA(cudaMemcpyAsync(g_.pool, pool.data(), sizeof(uint32_t) * used, cudaMemcpyHostToDevice, stream_));
     const unsigned long long top = used;
-    CSM_CUDA(cudaMemcpy(g_.pool_top, &top, sizeof(top), cudaMemcpyHostToDevice));
+    CSM_CUDA(cudaMemcpyAsync(g_.pool_top, &top, sizeof(top), cudaMemcpyHostToDevice, stream_));
+    CSM_CUDA(cudaStreamSynchronize(stream_));  // the host arrays end here
     return finish_load();
 }
 

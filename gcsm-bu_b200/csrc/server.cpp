@@ -119,10 +119,11 @@ class Server {
         for (auto &sl : slots_) {
             e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaMalloc(&sl.sc.ctrl, sizeof(EnumControl));
-            if (e == cudaSuccess) e = cudaMemset(sl.sc.ctrl, 0, sizeof(EnumControl));
+            if (e == cudaSuccess) e = cudaMemsetAsync(sl.sc.ctrl, 0, sizeof(EnumControl), sl.stream);
             if (e == cudaSuccess) e = cudaMalloc(&sl.sc.queue, sizeof(WorkItem) * kSlotQueueItems);
             if (e == cudaSuccess) e = cudaMalloc(&sl.sc.seq, sizeof(unsigned long long) * kSlotQueueItems);
-            if (e == cudaSuccess) e = cudaMemset(sl.sc.seq, 0, sizeof(unsigned long long) * kSlotQueueItems);
+            if (e == cudaSuccess)
+                e = cudaMemsetAsync(sl.sc.seq, 0, sizeof(unsigned long long) * kSlotQueueItems, sl.stream);
             if (e == cudaSuccess) e = cudaMalloc(&sl.sc.seed_lo, sizeof(uint32_t) * 3 * kSlotMaxPlans);
             if (e == cudaSuccess) e = cudaMalloc(&sl.sc.ticket_prefix, sizeof(uint32_t) * (kSlotMaxPlans + 1));
             if (e != cudaSuccess) return cuda_fail(e, "slot scratch");
